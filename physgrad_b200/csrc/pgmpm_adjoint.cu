@@ -32,7 +32,7 @@ __global__ void k_adj_grid(View V, AdjView A) {
          w += gridDim.x * tiles_per_block) {
         const uint32_t nt = V.tile_list[w];
         if (nt >= (uint32_t)V.total_nt) continue;
-        const int s = V.S == 1 ? 0 : scene_of_node_tile(V.scenes, V.S, (int)nt);
+        const int s = scene_of_node_tile(V, (int)nt);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)nt - sc.nt_base;
         const int i = 4 * (lt % sc.nt[0]) + (l & 3);
@@ -73,7 +73,7 @@ __global__ void __launch_bounds__(GATHER_T, 3) k_adj_gather(View V, AdjView A) {
     uint32_t flags = 0;
     // particles in physical order (the order of the state planes)
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += stride) {
-        const int s = V.S == 1 ? 0 : scene_of_particle(V.scenes, V.S, (int)p);
+        const int s = scene_of_particle(V, (int64_t)p);
         const SceneDev& sc = scene_ref(V, s);
         const int mid = MULTI ? V.mat[p] : 0;
         const MatDev mt = V.mats[mid];

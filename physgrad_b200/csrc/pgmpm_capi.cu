@@ -441,12 +441,29 @@ int pgmpm_create_ex(const pgmpm_scene_desc* scenes, int32_t n_scenes, const int6
         sw = (passes - 1) & 1;
     }
     s->sort_which = sw;
+    // first scenes of the particle and tile blocks (scene_of_particle and its
+    // tile counterparts)
+    std::vector<int32_t> tab;
+    if (n_scenes > 1) {
+        tab.reserve((size_t)scene_tab_size(N, s->total_ct, s->total_nt));
+        auto fill = [&](int64_t count, int64_t block, int SceneDev::*begin) {
+            int sc = 0;
+            for (int64_t i = 0; i < count; i += block) {
+                while (sc + 1 < n_scenes && s->scenes[sc + 1].*begin <= i) ++sc;
+                tab.push_back(sc);
+            }
+        };
+        fill(N, SCENE_BLOCK_P, &SceneDev::p_begin);
+        fill(s->total_ct, SCENE_BLOCK_T, &SceneDev::ct_base);
+        fill(s->total_nt, SCENE_BLOCK_T, &SceneDev::nt_base);
+    }
     const size_t n4 = sizeof(uint32_t) * (size_t)std::max<int64_t>(N, 1);
     cudaError_t e = cudaSuccess;
 #define AL(buf, bytes)                                         \
     if (e == cudaSuccess) e = (buf).alloc(bytes);
     AL(s->d_scenes, sizeof(SceneDev) * n_scenes);
     AL(s->d_mats, sizeof(MatDev) * n_materials);
+    if (!tab.empty()) AL(s->scene_tab, sizeof(int32_t) * tab.size());
     AL(s->q, sizeof(float4) * 6 * (size_t)std::max<int64_t>(N, 1));
     if (s->pf.physics == PHYS_MLS) AL(s->pay, sizeof(float4) * 4 * (size_t)std::max<int64_t>(N, 1));
     AL(s->mV, sizeof(float2) * (size_t)std::max<int64_t>(N, 1));
@@ -486,6 +503,8 @@ int pgmpm_create_ex(const pgmpm_scene_desc* scenes, int32_t n_scenes, const int6
     if (e == cudaSuccess && s->tune.step_sort == 0 && alloc_bin_sort(s) != PGMPM_OK) e = cudaErrorMemoryAllocation;
     if (e == cudaSuccess) e = cudaMemcpy(s->d_scenes.p, s->scenes.data(), sizeof(SceneDev) * n_scenes, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(s->d_mats.p, md.data(), sizeof(MatDev) * n_materials, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && !tab.empty())
+        e = cudaMemcpy(s->scene_tab.p, tab.data(), sizeof(int32_t) * tab.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(s->grid_mp.p, 0, s->grid_mp.bytes);
     if (e == cudaSuccess) e = cudaMemset(s->grid_v.p, 0, s->grid_v.bytes);
     if (e == cudaSuccess) e = cudaMemset(s->tile_flags.p, 0, s->tile_flags.bytes);

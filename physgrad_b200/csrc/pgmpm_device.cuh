@@ -274,32 +274,6 @@ __device__ __forceinline__ void sp_load_nbr(const SparseTiles& sp, uint32_t c, u
     nb[4] = b.x; nb[5] = b.y; nb[6] = b.z; nb[7] = b.w;
 }
 
-// ----------------------------------------------------------- scene lookup
-__device__ __forceinline__ int scene_of_cell_tile(const SceneDev* sc, int S, int ct) {
-    int lo = 0, hi = S - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&sc[mid].ct_base) <= ct) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-__device__ __forceinline__ int scene_of_node_tile(const SceneDev* sc, int S, int nt) {
-    int lo = 0, hi = S - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&sc[mid].nt_base) <= nt) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-__device__ __forceinline__ int scene_of_particle(const SceneDev* sc, int S, int p) {
-    int lo = 0, hi = S - 1;
-    while (lo < hi) {
-        int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&sc[mid].p_begin) <= p) lo = mid; else hi = mid - 1;
-    }
-    return lo;
-}
-
 // ------------------------------------------------------ constitutive laws
 // Rotation of the polar decomposition F = R S by the determinant-scaled
 // Newton iteration X <- (zeta X + (zeta X)^{-T}) / 2, zeta = |det X|^{-1/3}

@@ -37,7 +37,7 @@ __global__ void k_keys(View V) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     uint32_t flags = 0;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < V.N; p += stride) {
-        const int s = V.S == 1 ? 0 : scene_of_particle(V.scenes, V.S, (int)p);
+        const int s = scene_of_particle(V, (int64_t)p);
         const SceneDev& sc = scene_ref(V, s);
         const float4 q0 = V.q[p];
         const float x[3] = {q0.x, q0.y, q0.z};
@@ -84,7 +84,7 @@ __global__ void k_payload(View V) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     uint32_t flags = 0;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += stride) {
-        const int s = V.S == 1 ? 0 : scene_of_particle(V.scenes, V.S, (int)p);
+        const int s = scene_of_particle(V, (int64_t)p);
         const SceneDev& sc = scene_ref(V, s);
         float x[3], F[9], v[3], C[9];
         unpack_xF(V.q[p], V.q[N + p], V.q[2 * N + p], x, F);
@@ -124,7 +124,7 @@ __global__ void k_mark(View V) {
             const uint32_t slot = atomicAdd(&V.counters[CNT_CTILES], 1u);
             V.ctile_list[slot] = ct;
         }
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int tx = lt % sc.ct[0], ty = (lt / sc.ct[0]) % sc.ct[1], tz = lt / (sc.ct[0] * sc.ct[1]);
@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(512) k_p2g(View V, int ppt) {
             seg = send;
             continue;
         }
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -342,7 +342,7 @@ __global__ void __launch_bounds__(P2G_T, 3) k_p2g_tiles(View V, AdjView AV) {
         if (w >= ntiles) break;
         const uint32_t ct = V.ptile_list ? V.ptile_list[w] : V.ctile_list[w];  // largest tiles first
         const uint2 rg = V.ctile_range[ct];
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -659,7 +659,7 @@ __global__ void __launch_bounds__(P2GC_T, 6) k_p2g_cells(View V, AdjView AV) {
         const uint32_t wt = w / S, slice = w - wt * S;
         const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];  // largest tiles first
         const uint2 rg = V.ctile_range[ct];
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -834,7 +834,7 @@ __global__ void __launch_bounds__(P2GP_T, 5) k_p2g_pairs(View V) {
         const uint32_t wt = w / S, slice = w - wt * S;
         const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
         const uint2 rg = V.ctile_range[ct];
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -966,7 +966,7 @@ __global__ void __launch_bounds__(P2GR_T, 5) k_p2g_runs(View V) {
         const uint32_t wt = w / S, slice = w - wt * S;
         const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
         const uint2 rg = V.ctile_range[ct];
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         int ox, oy, oz0;
         tile_origin(V, sc, ct, ox, oy, oz0);
@@ -1162,7 +1162,7 @@ __global__ void __launch_bounds__(ADJR_T, 6) k_adj_runs(View V, AdjView AV) {
         const uint32_t wt = w / S, slice = w - wt * S;
         const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
         const uint2 rg = V.ctile_range[ct];
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -1317,7 +1317,7 @@ __global__ void k_grid(View V) {
          w += gridDim.x * tiles_per_block) {
         const uint32_t nt = V.tile_list[w];
         if (nt >= (uint32_t)V.total_nt) continue;
-        const int s = V.S == 1 ? 0 : scene_of_node_tile(V.scenes, V.S, (int)nt);
+        const int s = scene_of_node_tile(V, (int)nt);
         const SceneDev& sc = scene_ref(V, s);
         int i, j, k;
         if (V.sp.cap) {  // sparse: the slot's coordinates
@@ -1630,7 +1630,7 @@ __device__ __forceinline__ void k_g2p_impl(const View& V) {
             flags |= FLAG_TILE_RANGE;
             continue;
         }
-        const int s = V.S == 1 ? 0 : scene_of_particle(V.scenes, V.S, (int)p);
+        const int s = scene_of_particle(V, (int64_t)p);
         const SceneDev& sc = scene_ref(V, s);
         const float4* gv = V.grid_v;
         auto fetch = [&](int, int, int, int idx) { return __ldg(&gv[idx]); };
@@ -1683,7 +1683,7 @@ __global__ void __launch_bounds__(256) k_g2p_tiles(View V) {
         if (w >= ntiles) break;
         const uint32_t ct = V.ctile_list[w];
         const uint2 rg = V.ctile_range[ct];
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -1812,7 +1812,7 @@ __global__ void __launch_bounds__(G2_T, MINB) k_g2p2g(View V) {
         const uint32_t wt = w / S, slice = w - wt * S;
         const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
         const uint2 rg = V.ctile_range[ct];
-        const int s = V.S == 1 ? 0 : scene_of_cell_tile(V.scenes, V.S, (int)ct);
+        const int s = scene_of_cell_tile(V, (int)ct);
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),

@@ -121,6 +121,7 @@ struct pgmpm_solver_s {
     bool uploaded = false;
 
     // device buffers
+    pgmpm::DevBuf scene_tab;  // more than one scene: see scene_of_particle
     pgmpm::DevBuf d_scenes, d_mats, q, pay, mV, mat, user_of_phys, phys_of_user, keys, ka, va, kb, vb, sort_scratch;
     pgmpm::DevBuf grid_mp, grid_v, grid_vpre, tile_flags, tile_list, ctile_list, ctile_range, counters, staging;
     pgmpm::DevBuf bs_ccount, bs_coff, bs_tcount, bs_toff, bs_bsum, bs_slot, cell_range;  // per-step bin sort
@@ -221,6 +222,7 @@ struct pgmpm_solver_s {
         V.S = S;
         V.M = M;
         V.scenes = d_scenes.as<pgmpm::SceneDev>();
+        V.scene_tab = scene_tab.as<int32_t>();
         V.mats = d_mats.as<pgmpm::MatDev>();
         V.q = b.q;
         V.q_out = b.q_out;

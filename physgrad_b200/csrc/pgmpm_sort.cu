@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(BS_T) bs_finish(View V, uint32_t* __restrict__
     const int64_t nt = (int64_t)(blockIdx.x - cell_blocks) * BS_T + threadIdx.x;
     bool act = false;
     if (nt < V.total_nt) {
-        const int s = V.S == 1 ? 0 : scene_of_node_tile(V.scenes, V.S, (int)nt);
+        const int s = scene_of_node_tile(V, (int)nt);
         const SceneDev& sc = V.scenes[s];
         const int l = (int)nt - sc.nt_base;
         const int x = l % sc.nt[0], y = (l / sc.nt[0]) % sc.nt[1], z = l / (sc.nt[0] * sc.nt[1]);
