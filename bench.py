@@ -106,15 +106,17 @@ FP32_NOMINAL_TFLOPS = 148 * 128 * 2 * 1.965e9 / 1e12
 
 def kernel_launches_per_step(scenes, n_particles, fused=False):
     """Our kernels per step: the sort, then P2G, the grid update and G2P.
-    The solver sorts with the bin sort (5 kernels: count, 2-kernel scan of
-    the tile counts, cell offsets + node tiles, scatter) when the grids hold
-    at most about 8 cells per particle, else with the radix sort (3 kernels
-    per 8-bit pass + the tile marking).  With the fused kernel (bin sort
-    only) a chained step is the sort, the grid update and G2P2G."""
+    The solver sorts with the bin sort (tiles and scatter; a counting kernel
+    above 2^20 particles, where G2P does not count the next step's keys, and
+    a group sum above 65,536 cell tiles) when the grids hold at most about 8
+    cells per particle, else with the radix sort (3 kernels per 8-bit pass +
+    the tile marking).  With the fused kernel (bin sort only) a chained step
+    is the counting sort, the grid update and G2P2G."""
     cells = sum(((int(s.n[0]) - 3) // 4 + 1) * ((int(s.n[1]) - 3) // 4 + 1) * ((int(s.n[2]) - 3) // 4 + 1)
                 for s in scenes) * 64
     if cells <= 8 * max(n_particles, 1) + (1 << 20):
-        return 5 + (2 if fused else 3)
+        count = 1 if fused or n_particles > (1 << 20) else 0
+        return 2 + count + (1 if cells > 64 * 65536 else 0) + (2 if fused else 3)
     bits = max(1, int(np.ceil(np.log2(max(2, cells)))))
     passes = (bits + 7) // 8
     return 3 * passes + 1 + 3

@@ -85,17 +85,17 @@ int alloc_bin_sort(pgmpm_solver s) {
     if (s->bs_ccount.p) return PGMPM_OK;
     const size_t ct = (size_t)s->total_ct;
     CK(s->bs_ccount.alloc(sizeof(uint32_t) * (ct * 64 + 1)));
-    CK(s->bs_coff.alloc(sizeof(uint32_t) * ct * 64));
-    CK(s->bs_tcount.alloc(sizeof(uint32_t) * (ct + 1)));
-    CK(s->bs_toff.alloc(sizeof(uint32_t) * (ct + 1)));
-    CK(s->bs_bsum.alloc(sizeof(uint32_t) * (size_t)bin_sort_scan_blocks((int)ct)));
+    CK(s->bs_tcount.alloc(sizeof(uint32_t) * ((ct + 4) & ~(size_t)3)));
+    CK(s->bs_gsum.alloc(sizeof(uint32_t) * (size_t)bin_sort_groups((int64_t)ct)));
+    CK(s->bs_work.alloc(sizeof(uint32_t) * SW_WORDS));
     CK(s->bs_slot.alloc(sizeof(uint32_t) * (size_t)std::max<int64_t>(s->N, 1)));
     CK(s->cell_range.alloc(sizeof(uint2) * 64 * std::max<size_t>(ct, 1)));
-    CK(s->ptile_list.alloc(sizeof(uint32_t) * std::max<size_t>(ct, 1)));
-    CK(s->tile_rank.alloc(sizeof(uint32_t) * std::max<size_t>(ct, 1)));
+    CK(s->ptile.alloc(sizeof(uint4) * std::max<size_t>(ct, 1)));
+    CK(s->tile_info.alloc(sizeof(uint4) * std::max<size_t>(ct, 1)));
     // the counters start at zero and every sort leaves them zero
     CK(cudaMemset(s->bs_ccount.p, 0, s->bs_ccount.bytes));
     CK(cudaMemset(s->bs_tcount.p, 0, s->bs_tcount.bytes));
+    CK(cudaMemset(s->bs_work.p, 0, s->bs_work.bytes));
     return PGMPM_OK;
 }
 
@@ -142,7 +142,7 @@ int conditional_sort(pgmpm_solver s, const View& V, const BinSortBufs& B, uint32
     CK(cudaStreamUpdateCaptureDependencies(st, &cn, 1, cudaStreamSetCaptureDependencies));
     cudaGraph_t body = np.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(s->body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t e = bin_sort_step(V, B, s->num_sms, s->body_stream);
+    const cudaError_t e = bin_sort_step(V, B, s->num_sms, false, s->body_stream);
     cudaGraph_t out = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(s->body_stream, &out);
     CK(e);
@@ -150,7 +150,8 @@ int conditional_sort(pgmpm_solver s, const View& V, const BinSortBufs& B, uint32
     return PGMPM_OK;
 }
 
-int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, bool write_vc, StepKind kind) {
+int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, bool write_vc, StepKind kind,
+                bool counted, bool count_next) {
     if (s->N == 0) {  // nothing to move; keep the timing events consistent
         if (timed)
             for (int i = 0; i < 5; ++i) CK(cudaEventRecord(s->ev[i], st));
@@ -160,13 +161,15 @@ int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, 
         return fail(PGMPM_ERR_STATE, "internal: fused step without the bin sort");
     if (b.sort_mode != 0 && (s->tune.step_sort != 0 || kind != STEP_SPLIT || (b.sort_mode == 2 && !b.resort)))
         return fail(PGMPM_ERR_STATE, "internal: a recorded sort needs the bin sort and split steps");
+    if ((counted || count_next) && (!s->counts_ahead() || kind != STEP_SPLIT || b.sort_mode != 0))
+        return fail(PGMPM_ERR_STATE, "internal: keys counted ahead need the bin sort and the physical-order G2P");
     View V = s->view_for(b);
+    if (count_next) V.cnt = s->sort_counts();
     // P2G variant 1 builds its payload from the state's v and C
     V.write_vc = write_vc || s->pf.physics != PHYS_MLS || s->tune.p2g_variant == 1 ? 1 : 0;
     // per-step resets: tile counts, active node count, work cursors, and the
-    // active node tile flags.  The bin sort's first kernel clears the
-    // counters and the sort writes every flag itself, so a bin-sorted step
-    // has no memset node.
+    // active node tile flags.  The bin sort writes the counters and every
+    // flag itself, so a bin-sorted step has no memset node.
     if (s->tune.step_sort != 0) {
         CK(cudaMemsetAsync(b.tile_flags, 0, sizeof(uint32_t) * (size_t)s->total_nt, st));
         CK(cudaMemsetAsync(b.counters, 0, sizeof(uint32_t) * CNT_RESET, st));
@@ -175,19 +178,15 @@ int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, 
     if (s->tune.step_sort == 0) {
         BinSortBufs B;
         B.keys_in = b.keys_in;
-        B.ccount = s->bs_ccount.as<uint32_t>();
-        B.coff = s->bs_coff.as<uint32_t>();
-        B.tcount = s->bs_tcount.as<uint32_t>();
-        B.toff = s->bs_toff.as<uint32_t>();
-        B.bsum = s->bs_bsum.as<uint32_t>();
-        B.slot = s->bs_slot.as<uint32_t>();
+        B.cnt = s->sort_counts();
         B.out_k = b.which ? b.kb : b.ka;  // where the step's readers look (View::skeys / order)
         B.out_v = b.which ? b.vb : b.va;
         B.cell_range = b.cell_range;
-        B.ptile_list = b.ptile_list;
-        B.tile_rank = s->tile_rank.as<uint32_t>();
+        B.ptile = b.ptile;
+        B.tile_info = s->tile_info.as<uint4>();
+        B.gsum = s->bs_gsum.as<uint32_t>();
         if (b.sort_mode == 0) {
-            CK(bin_sort_step(V, B, s->num_sms, st));
+            CK(bin_sort_step(V, B, s->num_sms, counted, st));
         } else if (b.sort_mode == 2) {
             int rc = conditional_sort(s, V, B, b.resort, st);
             if (rc) return rc;
@@ -233,17 +232,17 @@ int unprime(pgmpm_solver s, cudaStream_t st) {
 
 namespace {
 
-// The step graph of one kind (mid = false: the call's last step; mid = true:
-// a step that another step of the same call follows, v and C not stored).
-int build_graph(pgmpm_solver s, StepKind kind, bool mid) {
-    cudaGraph_t& graph = s->step_graph[kind][mid ? 1 : 0];
-    cudaGraphExec_t& exec = s->step_exec[kind][mid ? 1 : 0];
+// The step graph of one kind and place in its call (see step_exec).
+int build_graph(pgmpm_solver s, StepKind kind, int place) {
+    cudaGraph_t& graph = s->step_graph[kind][place];
+    cudaGraphExec_t& exec = s->step_exec[kind][place];
+    const bool mid = (place & 1) != 0, ahead = s->counts_ahead() && kind == STEP_SPLIT;
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     exec = nullptr;
     graph = nullptr;
     CK(cudaStreamBeginCapture(s->cap_stream, cudaStreamCaptureModeThreadLocal));
-    int rc = record_step(s, s->live_bufs(), s->cap_stream, false, !mid, kind);
+    int rc = record_step(s, s->live_bufs(), s->cap_stream, false, !mid, kind, ahead && (place & 2), ahead && mid);
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->cap_stream, &g);
     if (rc != PGMPM_OK) {
@@ -288,14 +287,16 @@ int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
                 (s->met.average_step_ms * s->met.total_steps + s->met.last_step_ms) / (s->met.total_steps + 1);
             s->met.particle_steps_per_s = s->met.average_step_ms > 0 ? s->N / (s->met.average_step_ms * 1e-3) : 0;
         } else if (s->use_graph) {
-            const bool mid = k + 1 < n_steps;
-            if (!s->step_exec[kind][mid ? 1 : 0]) {
-                int rc = build_graph(s, kind, mid);
+            const int place = (k + 1 < n_steps ? 1 : 0) | (k > 0 && s->counts_ahead() ? 2 : 0);
+            if (!s->step_exec[kind][place]) {
+                int rc = build_graph(s, kind, place);
                 if (rc) return rc;
             }
-            CK(cudaGraphLaunch(s->step_exec[kind][mid ? 1 : 0], st));
+            CK(cudaGraphLaunch(s->step_exec[kind][place], st));
         } else {
-            int rc = record_step(s, s->live_bufs(), st, false, k + 1 == n_steps, kind);
+            const bool ahead = s->counts_ahead() && kind == STEP_SPLIT;
+            int rc = record_step(s, s->live_bufs(), st, false, k + 1 == n_steps, kind, ahead && k > 0,
+                                 ahead && k + 1 < n_steps);
             if (rc) return rc;
         }
         if (kind == STEP_FUSED_FIRST || kind == STEP_FUSED) s->primed = true;

@@ -40,12 +40,12 @@ namespace {
 size_t nodes_of(pgmpm_solver s) { return (size_t)s->total_nt * 64; }
 
 // Bytes one forward step adds to the record: sorted keys, order and the next
-// keys per particle, node-tile flags and list, cell-tile list and ranges,
-// cell ranges and the largest-first list, counters.
+// keys per particle, node-tile flags and list, cell ranges and the
+// largest-first list of occupied tiles, counters.
 size_t rec_step_bytes(pgmpm_solver s) {
     const size_t N = (size_t)std::max<int64_t>(s->N, 1);
     const size_t ct = std::max<size_t>((size_t)s->total_ct, 1);
-    return 12 * N + 8 * (size_t)s->total_nt + ct * (4 + 8 + 8 * 64 + 4) + 4 * CNT_WORDS;
+    return 12 * N + 8 * (size_t)s->total_nt + ct * (8 * 64 + 16) + 4 * CNT_WORDS;
 }
 
 // The tape: `slots` steps per set (states, keys, grid), and per-step sort
@@ -74,13 +74,14 @@ int ensure_tape(pgmpm_solver s, int slots, int rec = 0) {
     CK(s->tape_gvpre.alloc(sizeof(float4) * nodes * gs));
     CK(s->tape_flags.alloc(sizeof(uint32_t) * (size_t)s->total_nt * ss));
     CK(s->tape_tiles.alloc(sizeof(uint32_t) * (size_t)s->total_nt * ss));
-    CK(s->tape_ctiles.alloc(sizeof(uint32_t) * (size_t)s->total_ct * ss));
-    CK(s->tape_crange.alloc(sizeof(uint2) * (size_t)s->total_ct * ss));
+    // read after the radix sort only, which the record's steps do not run
+    CK(s->tape_ctiles.alloc(sizeof(uint32_t) * (size_t)s->total_ct * gs));
+    CK(s->tape_crange.alloc(sizeof(uint2) * (size_t)s->total_ct * gs));
     CK(s->tape_counters.alloc(sizeof(uint32_t) * CNT_WORDS * ss));
     CK(cudaMemset(s->tape_counters.p, 0, s->tape_counters.bytes));
     if (s->bs_ccount.p) {  // the bin sort is available: per-slot cell tables
         CK(s->tape_cells.alloc(sizeof(uint2) * 64 * std::max<size_t>((size_t)s->total_ct, 1) * ss));
-        CK(s->tape_ptile.alloc(sizeof(uint32_t) * std::max<size_t>((size_t)s->total_ct, 1) * ss));
+        CK(s->tape_ptile.alloc(sizeof(uint4) * std::max<size_t>((size_t)s->total_ct, 1) * ss));
     }
     if (rec) {
         CK(s->rec_keys.alloc(sizeof(uint32_t) * N * ((size_t)rec + 1)));
@@ -120,11 +121,12 @@ void set_sort_slot(pgmpm_solver s, StepBufs& b, size_t js) {
     }
     b.tile_flags = s->tape_flags.as<uint32_t>() + (size_t)s->total_nt * js;
     b.tile_list = s->tape_tiles.as<uint32_t>() + (size_t)s->total_nt * js;
-    b.ctile_list = s->tape_ctiles.as<uint32_t>() + (size_t)s->total_ct * js;
-    b.ctile_range = s->tape_crange.as<uint2>() + (size_t)s->total_ct * js;
+    const bool slot = js < (size_t)s->tape_slots * s->tape_sets;  // else a step of the record
+    b.ctile_list = slot ? s->tape_ctiles.as<uint32_t>() + (size_t)s->total_ct * js : nullptr;
+    b.ctile_range = slot ? s->tape_crange.as<uint2>() + (size_t)s->total_ct * js : nullptr;
     const size_t ct = std::max<size_t>((size_t)s->total_ct, 1);
     b.cell_range = s->tape_cells.p ? s->tape_cells.as<uint2>() + ct * 64 * js : nullptr;
-    b.ptile_list = s->tape_ptile.p ? s->tape_ptile.as<uint32_t>() + ct * js : nullptr;
+    b.ptile = s->tape_ptile.p ? s->tape_ptile.as<uint4>() + ct * js : nullptr;
     b.counters = s->tape_counters.as<uint32_t>() + CNT_WORDS * js;
 }
 
@@ -206,7 +208,9 @@ int record_tape_forward(pgmpm_solver s, int len, cudaStream_t st, int t = 0, int
             b.resort = s->rec_resort.as<uint32_t>() + t;
             b.sort_mode = j == 0 ? 1 : 2;
         }
-        int rc = record_step(s, b, st, false, true, step_kind(s, j, len, false, true));
+        const bool ahead = s->counts_ahead() && b.sort_mode == 0;  // each G2P counts for the next slot's sort
+        int rc = record_step(s, b, st, false, true, step_kind(s, j, len, false, true), ahead && j > 0,
+                             ahead && j + 1 < len);
         if (rc) return rc;
     }
     return PGMPM_OK;
@@ -243,7 +247,8 @@ int run_recorded(pgmpm_solver s, int g0, int len, cudaStream_t st) {
             b.keys_in = s->rec_keys.as<uint32_t>() + N * (size_t)(g0 + j);
             b.keys_out = s->rec_keys.as<uint32_t>() + N * (size_t)(g0 + j + 1);
             set_sort_slot(s, b, (size_t)(g0 + j));
-            int r = record_step(s, b, c, false, j + 1 == len, STEP_SPLIT);
+            const bool ahead = s->counts_ahead();
+            int r = record_step(s, b, c, false, j + 1 == len, STEP_SPLIT, ahead && j > 0, ahead && j + 1 < len);
             if (r) return r;
         }
         CK(launch_merge_flags(s->tape_counters.as<uint32_t>() + (size_t)CNT_WORDS * g0, len,

@@ -28,6 +28,20 @@ enum {
 };
 static_assert(CNT_STAMP < CNT_WORDS, "counter layout");
 
+// The bin sort's counters (pgmpm_sort.cu): particles per cell and per cell
+// tile, and each particle's slot in its cell.  A G2P that another step of the same call follows counts its new keys there
+// itself (View::cnt), and that step's sort starts from the counts.
+struct SortCounts {
+    uint32_t* ccount;      // total_ct * 64 + 1 words (cells + overflow bin)
+    uint32_t* tcount;      // total_ct + 1 words
+    uint32_t* slot;        // N words
+    uint32_t ncells;       // total_ct * 64: keys from here on are out of range
+};
+// words of the sort's list counters (View::sort_work): occupied cell tiles,
+// active node tiles, particles with a key in range, occupied tiles per size
+// class.  Zero between steps: the grid update clears them.
+enum { SW_CTILES = 0, SW_TILES = 1, SW_VALID = 2, SW_BUCKET = 3, SW_WORDS = 16 };
+
 // Everything a step kernel needs, passed by value.
 struct View {
     int64_t N;
@@ -55,10 +69,13 @@ struct View {
     uint32_t* tile_flags;      // node tile active flags (per global node tile)
     uint32_t* tile_list;       // active node tiles
     uint32_t* ctile_list;      // occupied cell tiles (global cell tile ids)
-    const uint32_t* ptile_list;  // the same tiles, largest first (null: use ctile_list)
+    const uint4* ptile;        // bin sort: the occupied cell tiles, largest first, as (tile, first
+                               // sorted position, end, scene); null (radix sort): use ctile_list
     uint2* ctile_range;        // per global cell tile: [begin, end) in sorted order
     const uint2* cell_range;   // per global cell: [begin, end) in sorted order (null: search skeys)
     uint32_t* counters;        // see CNT_*
+    uint32_t* sort_work;       // see SW_* (null without the bin sort)
+    SortCounts cnt;            // counters a G2P counts its new keys into (ccount null: it does not)
     int total_ct, total_nt;
     SparseTiles sp;            // sparse grid (sp.cap == 0: dense; tile ids are then slots)
 };
@@ -97,6 +114,55 @@ __device__ __forceinline__ int scene_of_node_tile(const View& V, int nt) {
     int s = __ldg(&V.scene_tab[scene_tab_nt(V.N, V.total_ct) + nt / SCENE_BLOCK_T]);
     while (s + 1 < V.S && __ldg(&V.scenes[s + 1].nt_base) <= nt) ++s;
     return s;
+}
+
+// One occupied cell tile of the step: its index, its particles' range in the
+// sorted order, its scene.
+struct TileWork {
+    uint32_t ct;
+    uint2 rg;
+    int s;
+};
+__device__ __forceinline__ TileWork tile_work(const View& V, uint32_t w) {
+    if (V.ptile) {
+        const uint4 t = __ldg(&V.ptile[w]);
+        return {t.x, make_uint2(t.y, t.z), (int)t.w};
+    }
+    const uint32_t ct = V.ctile_list[w];
+    return {ct, V.ctile_range[ct], scene_of_cell_tile(V, (int)ct)};
+}
+
+// Counts key k into the sort's counters: adds each run of equal keys among
+// the active lanes with one atomic.  Returns the run's first slot in its
+// first lane (in flight until used); run_slot() gives each lane its own.
+struct KeyRun {
+    uint32_t mask;  // lanes that count together
+    int start;      // first lane of this lane's run
+    uint32_t base;  // the run's first slot, in lane `start`
+};
+__device__ __forceinline__ KeyRun count_key(const SortCounts& c, uint32_t k) {
+    const uint32_t m = __activemask();
+    const int lane = threadIdx.x & 31;
+    const uint32_t upto = lane == 31 ? 0xFFFFFFFFu : ((2u << lane) - 1u);  // lanes <= this one
+    const uint32_t prev = __shfl_up_sync(m, k, 1);
+    const bool first = lane == 0 || !((m >> (lane - 1)) & 1u);
+    const bool head = first || prev != k;
+    const bool thead = first || (prev ^ k) >> 6;
+    // a run ends before the next head or the next inactive lane
+    auto end_of = [&](uint32_t heads) {
+        const uint32_t stop = (heads | ~m) & ~upto;
+        return stop ? __ffs(stop) - 1 : 32;
+    };
+    const uint32_t heads = __ballot_sync(m, head), theads = __ballot_sync(m, thead);
+    KeyRun r;
+    r.mask = m;
+    r.start = 31 - __clz(heads & upto);
+    r.base = head ? atomicAdd(&c.ccount[k], (uint32_t)(end_of(heads) - lane)) : 0u;
+    if (thead) atomicAdd(&c.tcount[k >> 6], (uint32_t)(end_of(theads) - lane));
+    return r;
+}
+__device__ __forceinline__ uint32_t run_slot(const KeyRun& r) {
+    return __shfl_sync(r.mask, r.base, r.start) + (uint32_t)((threadIdx.x & 31) - r.start);
 }
 
 // P2G variants: 0 = (cell, z-slice) register accumulation with a staged
@@ -147,25 +213,23 @@ cudaError_t radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t*
                              cudaStream_t st);
 
 // Per-step bin sort (pgmpm_sort.cu): keys_in (physical order) -> out_k /
-// out_v sorted by key, plus the occupied cell tiles, their ranges, the
-// active node tiles and their flags (View fields) and, when cell_range is
-// set, every cell's [begin, end) in the sorted order of the occupied tiles.
-// ccount and tcount must be zero on entry and are left zero.
+// out_v sorted by key, plus the occupied cell tiles with their ranges
+// (largest first), every cell's [begin, end) in the sorted order of the
+// occupied tiles, and the active node tiles and their flags (View fields).
+// The counters of cnt must be zero on entry, or (counted) hold the counts of
+// keys_in, and are left zero; V.sort_work must be zero, and the step's grid
+// update clears it again.
 struct BinSortBufs {
     const uint32_t* keys_in;
-    uint32_t* ccount;      // total_ct * 64 + 1 words (cells + overflow bin), zero between steps
-    uint32_t* coff;        // total_ct * 64 words
-    uint32_t* tcount;      // total_ct + 1 words, zero between steps
-    uint32_t* toff;        // total_ct + 1 words
-    uint32_t* bsum;        // bin_sort_scan_blocks(total_ct) words
-    uint32_t* slot;        // N words
+    SortCounts cnt;
     uint32_t *out_k, *out_v;  // N words each
-    uint2* cell_range;     // total_ct * 64, or null
-    uint32_t* ptile_list;  // total_ct: occupied tiles by size class, largest first (null: not built)
-    uint32_t* tile_rank;   // total_ct: class and rank of each ctile_list entry (scratch, with ptile_list)
+    uint2* cell_range;     // total_ct * 64
+    uint4* ptile;          // total_ct: see View::ptile
+    uint4* tile_info;      // total_ct: (tile, begin, end, class << 28 | rank) in order of discovery (scratch)
+    uint32_t* gsum;        // bin_sort_groups(total_ct) words (scratch)
 };
-int64_t bin_sort_scan_blocks(int total_ct);
-cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, cudaStream_t st);
+int64_t bin_sort_groups(int64_t total_ct);
+cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool counted, cudaStream_t st);
 
 // pgmpm_kernels.cu
 struct PhysFlags {

@@ -340,9 +340,10 @@ __global__ void __launch_bounds__(P2G_T, 3) k_p2g_tiles(View V, AdjView AV) {
         __syncthreads();
         const uint32_t w = s_work;
         if (w >= ntiles) break;
-        const uint32_t ct = V.ptile_list ? V.ptile_list[w] : V.ctile_list[w];  // largest tiles first
-        const uint2 rg = V.ctile_range[ct];
-        const int s = scene_of_cell_tile(V, (int)ct);
+        const TileWork work = tile_work(V, w);  // largest tiles first
+        const uint32_t ct = work.ct;
+        const uint2 rg = work.rg;
+        const int s = work.s;
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -657,9 +658,10 @@ __global__ void __launch_bounds__(P2GC_T, 6) k_p2g_cells(View V, AdjView AV) {
         if (w >= nwork) break;
         if (early && c == 0) next_work = atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
         const uint32_t wt = w / S, slice = w - wt * S;
-        const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];  // largest tiles first
-        const uint2 rg = V.ctile_range[ct];
-        const int s = scene_of_cell_tile(V, (int)ct);
+        const TileWork work = tile_work(V, wt);  // largest tiles first
+        const uint32_t ct = work.ct;
+        const uint2 rg = work.rg;
+        const int s = work.s;
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -832,9 +834,10 @@ __global__ void __launch_bounds__(P2GP_T, 5) k_p2g_pairs(View V) {
         if (w >= nwork) break;
         if (early && threadIdx.x == 0) next_work = atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
         const uint32_t wt = w / S, slice = w - wt * S;
-        const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
-        const uint2 rg = V.ctile_range[ct];
-        const int s = scene_of_cell_tile(V, (int)ct);
+        const TileWork work = tile_work(V, wt);  // largest tiles first
+        const uint32_t ct = work.ct;
+        const uint2 rg = work.rg;
+        const int s = work.s;
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -964,9 +967,10 @@ __global__ void __launch_bounds__(P2GR_T, 5) k_p2g_runs(View V) {
         if (w >= nwork) break;
         if (early && threadIdx.x == 0) next_work = atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
         const uint32_t wt = w / S, slice = w - wt * S;
-        const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
-        const uint2 rg = V.ctile_range[ct];
-        const int s = scene_of_cell_tile(V, (int)ct);
+        const TileWork work = tile_work(V, wt);  // largest tiles first
+        const uint32_t ct = work.ct;
+        const uint2 rg = work.rg;
+        const int s = work.s;
         const SceneDev& sc = scene_ref(V, s);
         int ox, oy, oz0;
         tile_origin(V, sc, ct, ox, oy, oz0);
@@ -1160,9 +1164,10 @@ __global__ void __launch_bounds__(ADJR_T, 6) k_adj_runs(View V, AdjView AV) {
         if (w >= nwork) break;
         if (early && threadIdx.x == 0) next_work = atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
         const uint32_t wt = w / S, slice = w - wt * S;
-        const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
-        const uint2 rg = V.ctile_range[ct];
-        const int s = scene_of_cell_tile(V, (int)ct);
+        const TileWork work = tile_work(V, wt);  // largest tiles first
+        const uint32_t ct = work.ct;
+        const uint2 rg = work.rg;
+        const int s = work.s;
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -1309,6 +1314,8 @@ __global__ void k_grid(View V) {
     // P2G has finished with its work cursor: leave it at zero for the reverse
     // of this step, whose scatter takes work from the same cursor
     if (blockIdx.x == 0 && threadIdx.x == 0) V.counters[CNT_P2G_CURSOR] = 0u;
+    // and the sort's list counters, for the next sort
+    if (V.sort_work && blockIdx.x == 0 && threadIdx.x < SW_WORDS) V.sort_work[threadIdx.x] = 0u;
     const uint32_t count = V.counters[CNT_TILES];
     const int tiles_per_block = blockDim.x >> 6;
     const int l = threadIdx.x & 63;
@@ -1463,7 +1470,9 @@ __device__ __forceinline__ void mls_advance(const View& V, const SceneDev& sc, i
 // forward recorded for the next step; a new key that differs replaces it and
 // sets *V.resort, so that the next step sorts again instead of keeping the
 // recorded sort.
-template <int PHYS, bool MULTI, bool FLUID, bool PLASTIC, class Fetch, bool SPARSE = false, bool CHECK = false>
+// COUNT: the new keys are counted for the next step's sort (V.cnt).
+template <int PHYS, bool MULTI, bool FLUID, bool PLASTIC, class Fetch, bool SPARSE = false, bool CHECK = false,
+          bool COUNT = false>
 __device__ __forceinline__ void g2p_particle(const View& V, const SceneDev& sc, uint32_t p, const Fetch& fetch,
                                              uint32_t& flags) {
     const int64_t N = V.N;
@@ -1482,6 +1491,7 @@ __device__ __forceinline__ void g2p_particle(const View& V, const SceneDev& sc, 
             const uint32_t okey = V.keys[p];
             if (okey >= (uint32_t)V.total_ct * 64u) {  // no slot (a full pool): the particle is left as is
                 flags |= FLAG_TILE_POOL;
+                if (COUNT) V.cnt.slot[p] = run_slot(count_key(V.cnt, V.cnt.ncells));
                 return;
             }
             oslot = okey >> 6;
@@ -1547,21 +1557,31 @@ __device__ __forceinline__ void g2p_particle(const View& V, const SceneDev& sc, 
             so[a] = stencil_origin(x[a], sc.origin[a], sc.dx, sc.inv_dx, sc.n[a], PHYS, u, flags);
             fn[a] = fminf(fmaxf(__fsub_rn(u, (float)so[a]), 0.5f), 1.5f);
         }
+        uint32_t nkey;
         if (SPARSE) {
             const int tx = so[0] >> 2, ty = so[1] >> 2, tz = so[2] >> 2;
             const uint32_t slot = (4 * tx == ox && 4 * ty == oy && 4 * tz == oz)
                                       ? oslot
                                       : sp_find_or_insert(V.sp, sp_code(tx, ty, tz), flags);
-            V.keys[p] = slot == SP_NONE ? SP_NONE
-                                        : slot * 64u + (uint32_t)((so[2] & 3) * 16 + (so[1] & 3) * 4 + (so[0] & 3));
+            nkey = slot == SP_NONE ? SP_NONE
+                                   : slot * 64u + (uint32_t)((so[2] & 3) * 16 + (so[1] & 3) * 4 + (so[0] & 3));
+            V.keys[p] = nkey;
         } else if (CHECK) {
-            const uint32_t nk = cell_key(sc, so);
-            if (V.keys[p] != nk) {  // rare: the replay rounded across a cell face
-                V.keys[p] = nk;
+            nkey = cell_key(sc, so);
+            if (V.keys[p] != nkey) {  // rare: the replay rounded across a cell face
+                V.keys[p] = nkey;
                 atomicOr(V.resort, 1u);
             }
         } else {
-            V.keys[p] = cell_key(sc, so);
+            nkey = cell_key(sc, so);
+            V.keys[p] = nkey;
+        }
+        // counted for the next step's sort (the atomics are in flight while
+        // the payload is formed)
+        KeyRun run;
+        if (COUNT) {
+            if (SPARSE && nkey >= V.cnt.ncells) flags |= FLAG_TILE_RANGE;
+            run = count_key(V.cnt, min(nkey, V.cnt.ncells));
         }
         if (V.pay_out) {
             const float2 mv = V.mV[p];
@@ -1572,6 +1592,7 @@ __device__ __forceinline__ void g2p_particle(const View& V, const SceneDev& sc, 
             V.pay_out[2 * N + p] = a2;
             V.pay_out[3 * N + p] = a3;
         }
+        if (COUNT) V.cnt.slot[p] = run_slot(run);
         return;
     } else {
         // material_point_method.h:599-666 in the same order of operations
@@ -1610,7 +1631,9 @@ __device__ __forceinline__ void g2p_particle(const View& V, const SceneDev& sc, 
         float u;
         so[a] = stencil_origin(x[a], sc.origin[a], sc.dx, sc.inv_dx, sc.n[a], PHYS, u, flags);
     }
-    V.keys[p] = cell_key(sc, so);
+    const uint32_t nkey = cell_key(sc, so);
+    V.keys[p] = nkey;
+    if (COUNT) V.cnt.slot[p] = run_slot(count_key(V.cnt, nkey));
 }
 
 // G2P variants 1 and 2: one thread per particle, 27 gathers through L1.
@@ -1619,11 +1642,14 @@ __device__ __forceinline__ void g2p_particle(const View& V, const SceneDev& sc, 
 // sorted at upload and particles drift less than a cell per step, so
 // neighbouring threads still share grid nodes, and the state loads are fully
 // coalesced with no dependent load of the order array.
-template <int PHYS, bool MULTI, bool FLUID, bool PHYS_ORDER, bool PLASTIC, bool SPARSE = false, bool CHECK = false>
+template <int PHYS, bool MULTI, bool FLUID, bool PHYS_ORDER, bool PLASTIC, bool SPARSE = false, bool CHECK = false,
+          bool COUNT = false>
 __device__ __forceinline__ void k_g2p_impl(const View& V) {
     const int64_t N = V.N;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     uint32_t flags = 0;
+    // counting the next keys makes them a new step's: its stamp
+    if (SPARSE && COUNT && blockIdx.x == 0 && threadIdx.x == 0) V.counters[CNT_STAMP] += 1u;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
         const uint32_t p = PHYS_ORDER ? (uint32_t)i : V.order[i];
         if (p >= (uint32_t)N) {
@@ -1634,7 +1660,7 @@ __device__ __forceinline__ void k_g2p_impl(const View& V) {
         const SceneDev& sc = scene_ref(V, s);
         const float4* gv = V.grid_v;
         auto fetch = [&](int, int, int, int idx) { return __ldg(&gv[idx]); };
-        g2p_particle<PHYS, MULTI, FLUID, PLASTIC, decltype(fetch), SPARSE, CHECK>(V, sc, p, fetch, flags);
+        g2p_particle<PHYS, MULTI, FLUID, PLASTIC, decltype(fetch), SPARSE, CHECK, COUNT>(V, sc, p, fetch, flags);
     }
     if (flags) atomicOr(&V.counters[CNT_FLAGS], flags);
 }
@@ -1645,14 +1671,14 @@ __global__ void k_g2p(View V) {
 }
 // 64 registers (4 blocks of 256 threads per SM): the gathers' latency wants
 // the occupancy more than the few spilled words cost
-template <int PHYS, bool MULTI, bool FLUID>
+template <int PHYS, bool MULTI, bool FLUID, bool COUNT>
 __global__ void __launch_bounds__(512, 2) k_g2p_phys(View V) {
-    k_g2p_impl<PHYS, MULTI, FLUID, true, false>(V);
+    k_g2p_impl<PHYS, MULTI, FLUID, true, false, false, false, COUNT>(V);
 }
 // the same with the von Mises cap (an ELASTOPLASTIC material is present)
-template <int PHYS, bool MULTI, bool FLUID>
+template <int PHYS, bool MULTI, bool FLUID, bool COUNT>
 __global__ void __launch_bounds__(512, 2) k_g2p_phys_vm(View V) {
-    k_g2p_impl<PHYS, MULTI, FLUID, true, true>(V);
+    k_g2p_impl<PHYS, MULTI, FLUID, true, true, false, false, COUNT>(V);
 }
 // replay of recorded steps (MLS, dense): the new keys are checked against
 // the recorded ones (see g2p_particle's CHECK)
@@ -1661,9 +1687,9 @@ __global__ void __launch_bounds__(512, 2) k_g2p_check(View V) {
     k_g2p_impl<PHYS_MLS, MULTI, FLUID, true, PLASTIC, false, true>(V);
 }
 // sparse grids (MLS)
-template <bool MULTI, bool FLUID, bool PLASTIC>
+template <bool MULTI, bool FLUID, bool PLASTIC, bool COUNT>
 __global__ void __launch_bounds__(512, 2) k_g2p_sparse(View V) {
-    k_g2p_impl<PHYS_MLS, MULTI, FLUID, true, PLASTIC, true>(V);
+    k_g2p_impl<PHYS_MLS, MULTI, FLUID, true, PLASTIC, true, false, COUNT>(V);
 }
 
 // G2P variant 0: one block per occupied cell tile; the tile's 6^3 node
@@ -1681,9 +1707,10 @@ __global__ void __launch_bounds__(256) k_g2p_tiles(View V) {
         __syncthreads();
         const uint32_t w = s_work;
         if (w >= ntiles) break;
-        const uint32_t ct = V.ctile_list[w];
-        const uint2 rg = V.ctile_range[ct];
-        const int s = scene_of_cell_tile(V, (int)ct);
+        const TileWork work = tile_work(V, w);
+        const uint32_t ct = work.ct;
+        const uint2 rg = work.rg;
+        const int s = work.s;
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -1810,9 +1837,10 @@ __global__ void __launch_bounds__(G2_T, MINB) k_g2p2g(View V) {
         if (w >= nwork) break;
         if (early && threadIdx.x == 0) next_work = atomicAdd(&V.counters[CNT_G2P_CURSOR], 1u);
         const uint32_t wt = w / S, slice = w - wt * S;
-        const uint32_t ct = V.ptile_list ? V.ptile_list[wt] : V.ctile_list[wt];
-        const uint2 rg = V.ctile_range[ct];
-        const int s = scene_of_cell_tile(V, (int)ct);
+        const TileWork work = tile_work(V, wt);  // largest tiles first
+        const uint32_t ct = work.ct;
+        const uint2 rg = work.rg;
+        const int s = work.s;
         const SceneDev& sc = scene_ref(V, s);
         const int lt = (int)ct - sc.ct_base;
         const int ox = 4 * (lt % sc.ct[0]), oy = 4 * ((lt / sc.ct[0]) % sc.ct[1]),
@@ -2328,23 +2356,24 @@ cudaError_t launch_grid(const View& V, const PhysFlags& pf, const Tuning& t, int
     return cudaGetLastError();
 }
 
-#define PGMPM_G2P_DISPATCH(KERNEL, GRID, BLOCK)                                  \
-    do {                                                                         \
-        if (pf.physics == PHYS_MLS) {                                            \
-            if (pf.multi_mat) {                                                  \
-                if (pf.has_fluid)                                                \
-                    KERNEL<PHYS_MLS, true, true><<<GRID, BLOCK, 0, st>>>(V);     \
-                else                                                             \
-                    KERNEL<PHYS_MLS, true, false><<<GRID, BLOCK, 0, st>>>(V);    \
-            } else {                                                             \
-                if (pf.has_fluid)                                                \
-                    KERNEL<PHYS_MLS, false, true><<<GRID, BLOCK, 0, st>>>(V);    \
-                else                                                             \
-                    KERNEL<PHYS_MLS, false, false><<<GRID, BLOCK, 0, st>>>(V);   \
-            }                                                                    \
-        } else {                                                                 \
-            KERNEL<PHYS_REF, false, false><<<GRID, BLOCK, 0, st>>>(V);           \
-        }                                                                        \
+// ...: further template arguments of KERNEL
+#define PGMPM_G2P_DISPATCH(KERNEL, GRID, BLOCK, ...)                                                  \
+    do {                                                                                              \
+        if (pf.physics == PHYS_MLS) {                                                                 \
+            if (pf.multi_mat) {                                                                       \
+                if (pf.has_fluid)                                                                     \
+                    KERNEL<PHYS_MLS, true, true __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);   \
+                else                                                                                  \
+                    KERNEL<PHYS_MLS, true, false __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);  \
+            } else {                                                                                  \
+                if (pf.has_fluid)                                                                     \
+                    KERNEL<PHYS_MLS, false, true __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);  \
+                else                                                                                  \
+                    KERNEL<PHYS_MLS, false, false __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V); \
+            }                                                                                         \
+        } else {                                                                                      \
+            KERNEL<PHYS_REF, false, false __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);     \
+        }                                                                                             \
     } while (0)
 
 cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int num_sms, cudaStream_t st) {
@@ -2352,7 +2381,13 @@ cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int 
     if (V.sp.cap) {  // sparse grids run the physical-order MLS G2P only
         if (pf.physics != PHYS_MLS) return cudaErrorNotSupported;
         const int nb = grid_for(V.N, t.g2p_block, 1 << 30);
-#define PGMPM_G2PS(M_, F_, P_) k_g2p_sparse<M_, F_, P_><<<nb, t.g2p_block, 0, st>>>(V)
+#define PGMPM_G2PS(M_, F_, P_)                                           \
+    do {                                                                 \
+        if (V.cnt.ccount)                                                \
+            k_g2p_sparse<M_, F_, P_, true><<<nb, t.g2p_block, 0, st>>>(V);  \
+        else                                                             \
+            k_g2p_sparse<M_, F_, P_, false><<<nb, t.g2p_block, 0, st>>>(V); \
+    } while (0)
         if (pf.multi_mat) {
             if (pf.has_fluid) {
                 if (pf.has_plastic) PGMPM_G2PS(true, true, true); else PGMPM_G2PS(true, true, false);
@@ -2397,10 +2432,15 @@ cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int 
         PGMPM_G2P_DISPATCH(k_g2p, nb, t.g2p_block);
     } else {
         const int nb = grid_for(V.N, t.g2p_block, 1 << 30);
-        if (pf.has_plastic)
-            PGMPM_G2P_DISPATCH(k_g2p_phys_vm, nb, t.g2p_block);
+        const bool count = V.cnt.ccount != nullptr;
+        if (pf.has_plastic && count)
+            PGMPM_G2P_DISPATCH(k_g2p_phys_vm, nb, t.g2p_block, true);
+        else if (pf.has_plastic)
+            PGMPM_G2P_DISPATCH(k_g2p_phys_vm, nb, t.g2p_block, false);
+        else if (count)
+            PGMPM_G2P_DISPATCH(k_g2p_phys, nb, t.g2p_block, true);
         else
-            PGMPM_G2P_DISPATCH(k_g2p_phys, nb, t.g2p_block);
+            PGMPM_G2P_DISPATCH(k_g2p_phys, nb, t.g2p_block, false);
     }
     return cudaGetLastError();
 }

@@ -72,7 +72,7 @@ struct StepBufs {
     uint32_t* ctile_list;
     uint2* ctile_range;
     uint2* cell_range;     // per-cell ranges written by the bin sort (null: not kept)
-    uint32_t* ptile_list;  // occupied tiles largest first, built by the bin sort (null: not kept)
+    uint4* ptile;          // occupied tiles largest first, built by the bin sort (null: not kept)
     uint32_t* counters;
     // Replay of a recorded step (bin sort only): the sort's outputs above are
     // the forward's, valid while keys_in equals the forward's keys.  The step
@@ -124,8 +124,8 @@ struct pgmpm_solver_s {
     pgmpm::DevBuf scene_tab;  // more than one scene: see scene_of_particle
     pgmpm::DevBuf d_scenes, d_mats, q, pay, mV, mat, user_of_phys, phys_of_user, keys, ka, va, kb, vb, sort_scratch;
     pgmpm::DevBuf grid_mp, grid_v, grid_vpre, tile_flags, tile_list, ctile_list, ctile_range, counters, staging;
-    pgmpm::DevBuf bs_ccount, bs_coff, bs_tcount, bs_toff, bs_bsum, bs_slot, cell_range;  // per-step bin sort
-    pgmpm::DevBuf ptile_list, tile_rank;  // largest-first occupied tile list (bin sort)
+    pgmpm::DevBuf bs_ccount, bs_tcount, bs_gsum, bs_slot, bs_work, cell_range;  // per-step bin sort
+    pgmpm::DevBuf ptile, tile_info;  // largest-first occupied tile list (bin sort)
     // sparse grid (sp_cap > 0): tile pool hash (slot codes) and the per-tile
     // node-tile slots; total_ct == total_nt == sp_cap
     pgmpm::DevBuf sp_code, sp_nbr, sp_box, sp_rev;
@@ -144,11 +144,12 @@ struct pgmpm_solver_s {
     // then stale).  Cleared by pgmpm::unprime.
     bool primed = false;
 
-    // graphs, one per step kind and [0] the call's last step / [1] a step
-    // that another step of the same call follows (v, C not stored)
+    // graphs, one per step kind and place in its call: bit 0, a step of the
+    // same call follows (v, C not stored, the next keys counted); bit 1, a
+    // step of the same call went before (its G2P counted this step's keys)
     cudaStream_t cap_stream = nullptr;
-    cudaGraphExec_t step_exec[pgmpm::STEP_KINDS][2] = {};
-    cudaGraph_t step_graph[pgmpm::STEP_KINDS][2] = {};
+    cudaGraphExec_t step_exec[pgmpm::STEP_KINDS][4] = {};
+    cudaGraph_t step_graph[pgmpm::STEP_KINDS][4] = {};
     cudaEvent_t ev[6] = {};
 
     // metrics
@@ -211,7 +212,7 @@ struct pgmpm_solver_s {
         b.ctile_list = ctile_list.as<uint32_t>();
         b.ctile_range = ctile_range.as<uint2>();
         b.cell_range = cell_range.as<uint2>();
-        b.ptile_list = ptile_list.as<uint32_t>();
+        b.ptile = ptile.as<uint4>();
         b.counters = counters.as<uint32_t>();
         return b;
     }
@@ -243,7 +244,9 @@ struct pgmpm_solver_s {
         V.ctile_list = b.ctile_list;
         V.ctile_range = b.ctile_range;
         V.cell_range = tune.step_sort == 0 ? b.cell_range : nullptr;
-        V.ptile_list = tune.step_sort == 0 ? b.ptile_list : nullptr;
+        V.ptile = tune.step_sort == 0 ? b.ptile : nullptr;
+        V.sort_work = bs_work.as<uint32_t>();
+        V.cnt = pgmpm::SortCounts{};
         V.counters = b.counters;
         V.total_ct = total_ct;
         V.total_nt = total_nt;
@@ -271,13 +274,34 @@ struct pgmpm_solver_s {
 
     void drop_graph() {
         for (int k = 0; k < pgmpm::STEP_KINDS; ++k)
-            for (int m = 0; m < 2; ++m) {
+            for (int m = 0; m < 4; ++m) {
                 if (step_exec[k][m]) cudaGraphExecDestroy(step_exec[k][m]);
                 if (step_graph[k][m]) cudaGraphDestroy(step_graph[k][m]);
                 step_exec[k][m] = nullptr;
                 step_graph[k][m] = nullptr;
             }
         drop_tape_graphs();
+    }
+
+    pgmpm::SortCounts sort_counts() const {
+        pgmpm::SortCounts c;
+        c.ccount = bs_ccount.as<uint32_t>();
+        c.tcount = bs_tcount.as<uint32_t>();
+        c.slot = bs_slot.as<uint32_t>();
+        c.ncells = (uint32_t)total_ct * 64u;
+        return c;
+    }
+
+    // split steps whose G2P counts its new keys for the sort of the step
+    // that follows in the same call.  Up to this many particles it saves more
+    // than it costs; with more, whose state outgrows L2, its atomics hold the
+    // warps that hide the gathers' latency, and a counting pass of its own is
+    // cheaper.  G2P with and without it, and the pass: 32 K particles 7.0, 6.1
+    // and 4.8 us; 262 K 16.8, 15.2 and 4.9 us; 1 M 52.8, 51.3 and 8.7 us;
+    // 2 M 114, 97 and 12.6 us; 3.9 M 246, 221 and 19 us.
+    static constexpr int64_t kCountAheadMax = (int64_t)1 << 20;
+    bool counts_ahead() const {
+        return tune.step_sort == 0 && tune.g2p_variant == 2 && !fused() && N <= kCountAheadMax;
     }
 
     // the live steps run the fused G2P -> P2G kernel
@@ -314,8 +338,11 @@ int alloc_bin_sort(pgmpm_solver s);
 // (state planes 3-5) unwritten when the next step follows in the same call:
 // that step reads them only through the payload (or the fused kernel does
 // not read them), and the call's last step writes them.
+// counted: the bin sort's counters hold the counts of b.keys_in already;
+// count_next: this step's G2P counts the keys it writes (counts_ahead(); the
+// step that sorts b.keys_out must be recorded next, counted).
 int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, bool write_vc = true,
-                StepKind kind = STEP_SPLIT);
+                StepKind kind = STEP_SPLIT, bool counted = false, bool count_next = false);
 // The kind of step k of n consecutive steps that start from a state whose
 // P2G is (primed) or is not already in grid_mp; drain: the last step leaves
 // nothing pending (G2P instead of G2P2G).

@@ -14,6 +14,8 @@
 // orders blocks.  The result is therefore identical to a stable CPU sort.
 // Scratch: hist (digits x blocks u32), totals (256 u32), and ping-pong
 // (key, value) buffers of n pairs, provided by the caller.
+#include <algorithm>
+
 #include "pgmpm_internal.h"
 
 namespace pgmpm {
@@ -202,39 +204,47 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint32_t* __restr
 // --------------------------------------------------- per-step bin sort
 // The MPM step groups particles by cell with a counting sort over the cells
 // (key = cell tile << 6 | cell in tile) instead of a full radix sort:
-//   bs_count     clears the step's counters (words [0, CNT_RESET));
-//                particles per cell and per cell tile, and each particle's
-//                slot in its cell.  Lanes holding equal keys in a run (the
-//                physical order stays close to cell order) share one atomic:
-//                the run's first lane adds the run length.  8 keys per thread
-//                with their loads and atomics issued back to back.
-//   bs_reduce / bs_down
-//                exclusive scan of the tile counts (block totals, then each
-//                block adds the totals before it; on grids of up to 64 Ki
-//                cell tiles bs_down sums the counts before its range itself
-//                and bs_reduce is not launched); bs_down also emits each
-//                occupied tile (sorted range, entry in the occupied-tile
-//                list, rank in its size class).
-//   bs_finish    (a) one warp per occupied tile: scan of its 64 cell counts
-//                -> every cell's first sorted position and range, clearing
-//                the cell and tile counters, and the tile's slot in the
-//                largest-first list P2G takes work from (the last tiles a
+//   bs_count     particles per cell and per cell tile, and each particle's
+//                slot in its cell.  Lanes holding equal keys
+//                in a run (the physical order stays close to cell order)
+//                share one atomic: the run's first lane adds the run length.
+//                Launched for the first step of a call only: the G2P of a
+//                step that another one follows counts the keys it writes.
+//   bs_groups    on grids of more than BS_DIRECT_TILES cell tiles: sums of the
+//                tile counts over groups of BS_GROUP tiles.
+//   bs_tiles     (a) one block per 8 or 64 cell tiles: sums the counts before
+//                its range, and one warp per occupied tile scans its 64 cell
+//                counts -> every cell's range, clearing the cell
+//                counters, and lists the tile with its rank in its size
+//                class; (b) one thread per node tile: active iff one of the 8
+//                cell tiles around it is occupied.
+//   bs_scatter   particle -> cell begin + slot; the occupied tiles' places in
+//                the largest-first list P2G takes work from (the last tiles a
 //                persistent P2G block picks up are then small ones, which
-//                shortens the kernel's tail); (b) one thread per node tile:
-//                active iff one of the 8 cell tiles around it is occupied.
-//   bs_scatter   particle -> cell offset + slot.
+//                shortens the kernel's tail); clears the tile and group
+//                counters and publishes the step's counter words.
 // The counters are left zero for the next step by their readers, so a step
 // costs O(N + occupied cells + tiles) with no clearing pass.  Keys come out
 // sorted; particles that share a cell in atomic-arrival order, which the
 // step does not rely on.
+//
+// Small scenes are bound by the launches (each kernel is a chain of a few
+// dependent L2 reads, 3-5 us), large ones by the passes over the particles:
+// counting inside G2P, where the keys are in registers, and scanning tiles
+// and cells in one kernel took the sort from four kernels to two per step: 50
+// steps of 32,768 particles 2148 -> 1725 us, 20 steps of 2 M particles (which
+// keep the counting pass) 5464 -> 5308 us.
 constexpr int BS_T = 256;
 constexpr int BS_ITEMS = 8;                 // keys per thread in bs_count / bs_scatter
 constexpr int BS_TILE = BS_T * BS_ITEMS;    // keys per block
-constexpr int BS_SCAN = 1024;               // tile counts per scan block
-// up to this many scan blocks (64 Ki cell tiles, a 256^3 grid) bs_down sums
-// the counts before its range directly, without bs_reduce: the last block
-// reads at most 63 Ki words from L2
-constexpr int BS_DIRECT_BLOCKS = 64;
+// cell tiles per warp of bs_tiles: a warp takes its occupied tiles in turn
+// (~1 us each: a sparse grid's claims are chains of L2 reads), so few per warp
+// are better until the blocks' reads of the counts before them (tiles^2 / 2
+// words over all blocks) outgrow that
+constexpr int BT_FEW = 1, BT_MANY = 8;
+constexpr int64_t BT_FEW_TILES = 8192;      // most cell tiles for BT_FEW
+constexpr int64_t BS_DIRECT_TILES = 65536;  // most cell tiles whose counts bs_tiles sums without bs_groups
+constexpr int BS_GROUP = 1024;              // cell tiles per group of bs_groups
 
 // Run structure of `bin` over a warp: first lane of this lane's run and one
 // past its last lane.  A run is a maximal stretch of consecutive lanes with
@@ -250,13 +260,9 @@ __device__ __forceinline__ void bs_run(uint32_t bin, bool ok, int lane, int& sta
     end = after ? __ffs(after) - 1 : 32;
 }
 
-__global__ void __launch_bounds__(BS_T) bs_count(const uint32_t* __restrict__ keys, int64_t n, uint32_t ncells,
-                                                 uint32_t* __restrict__ ccount, uint32_t* __restrict__ tcount,
-                                                 uint32_t* __restrict__ slot, uint32_t* __restrict__ counters) {
+__global__ void __launch_bounds__(BS_T) bs_count(const uint32_t* __restrict__ keys, int64_t n, SortCounts c,
+                                                 uint32_t* __restrict__ counters) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // the step's per-step counters start at zero: this is the step's first
-    // kernel and it reads none of them (the step recording issues no memset)
-    if (blockIdx.x == 0 && threadIdx.x < CNT_RESET) counters[threadIdx.x] = 0u;
     // a new step stamp (sparse grids mark active node tiles with it)
     if (blockIdx.x == 0 && threadIdx.x == 0) counters[CNT_STAMP] += 1u;
     const int64_t base = (int64_t)blockIdx.x * BS_TILE + warp * (32 * BS_ITEMS);
@@ -267,9 +273,9 @@ __global__ void __launch_bounds__(BS_T) bs_count(const uint32_t* __restrict__ ke
     for (int r = 0; r < BS_ITEMS; ++r) {
         const int64_t i = base + r * 32 + lane;
         k[r] = i < n ? keys[i] : 0u;
-        if (i < n && k[r] >= ncells) {  // out-of-range key: overflow bin after the last cell
+        if (i < n && k[r] >= c.ncells) {  // out-of-range key: overflow bin after the last cell
             bad = true;
-            k[r] = ncells;
+            k[r] = c.ncells;
         }
     }
 #pragma unroll
@@ -279,25 +285,16 @@ __global__ void __launch_bounds__(BS_T) bs_count(const uint32_t* __restrict__ ke
         bs_run(k[r], ok, lane, st[r], e);
         bs_run(k[r] >> 6, ok, lane, ts, te);
         cb[r] = 0u;
-        if (ok && lane == st[r]) cb[r] = atomicAdd(&ccount[k[r]], (uint32_t)(e - st[r]));
-        if (ok && lane == ts) atomicAdd(&tcount[k[r] >> 6], (uint32_t)(te - ts));
+        if (ok && lane == st[r]) cb[r] = atomicAdd(&c.ccount[k[r]], (uint32_t)(e - st[r]));
+        if (ok && lane == ts) atomicAdd(&c.tcount[k[r] >> 6], (uint32_t)(te - ts));
     }
 #pragma unroll
     for (int r = 0; r < BS_ITEMS; ++r) {
         const int64_t i = base + r * 32 + lane;
         const uint32_t b = __shfl_sync(0xFFFFFFFFu, cb[r], st[r]);
-        if (i < n) slot[i] = b + (uint32_t)(lane - st[r]);
+        if (i < n) c.slot[i] = b + (uint32_t)(lane - st[r]);
     }
     if (bad) atomicOr(&counters[CNT_FLAGS], FLAG_TILE_RANGE);
-}
-
-__global__ void __launch_bounds__(BS_SCAN) bs_reduce(const uint32_t* __restrict__ tcount, int64_t n,
-                                                     uint32_t* __restrict__ bsum) {
-    __shared__ uint32_t sh[32];
-    const int64_t i = (int64_t)blockIdx.x * BS_SCAN + threadIdx.x;
-    uint32_t tot;
-    block_excl_scan(i < n ? tcount[i] : 0u, sh, tot);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = tot;
 }
 
 // Warp-aggregated append of `item` (lanes with want) to list / counter;
@@ -311,7 +308,7 @@ __device__ __forceinline__ uint32_t bs_append(uint32_t* list, uint32_t* counter,
     if (lane == leader) b = atomicAdd(counter, (uint32_t)__popc(m));
     b = __shfl_sync(0xFFFFFFFFu, b, leader);
     const uint32_t slot = b + __popc(m & ((1u << lane) - 1u));
-    if (want) list[slot] = item;
+    if (want && list) list[slot] = item;
     return slot;
 }
 
@@ -322,95 +319,115 @@ __device__ __forceinline__ int bs_class(uint32_t count) {
     return min(CNT_BUCKETS - 1, max(0, 10 - lg));
 }
 
-// bsum: the per-block totals of bs_reduce, or null when the blocks are few
-// (BS_DIRECT_BLOCKS): each block then sums the tile counts before its own
-// range itself, and the step has no bs_reduce launch.  The tile counts are
-// left for bs_finish to clear, since later blocks read earlier blocks' range.
-__global__ void __launch_bounds__(BS_SCAN) bs_down(View V, const uint32_t* __restrict__ tcount, int64_t n,
-                                                   const uint32_t* __restrict__ bsum, uint32_t* __restrict__ toff,
-                                                   uint32_t* __restrict__ ccount_overflow,
-                                                   uint32_t* __restrict__ tile_rank) {
-    __shared__ uint32_t sh[32];
-    const int lane = threadIdx.x & 31;
-    // this block's first position: the tile totals of the blocks before it
-    uint32_t part = 0u;
-    if (bsum) {
-        for (uint32_t b = threadIdx.x; b < blockIdx.x; b += BS_SCAN) part += bsum[b];
-    } else {
-        const int64_t end = (int64_t)blockIdx.x * BS_SCAN;
-        for (int64_t i = threadIdx.x; i < end; i += BS_SCAN) part += tcount[i];
-    }
-    uint32_t base;
-    block_excl_scan(part, sh, base);
-    const int64_t t = (int64_t)blockIdx.x * BS_SCAN + threadIdx.x;
-    const uint32_t c = t < n ? tcount[t] : 0u;
-    uint32_t tot;
-    const uint32_t ex = block_excl_scan(c, sh, tot) + base;
-    if (t < n) toff[t] = ex;
-    if (t == n - 1) *ccount_overflow = 0u;
-    const bool occ = t < (int64_t)V.total_ct && c > 0u;  // not the overflow bin
-    if (occ) V.ctile_range[t] = make_uint2(ex, ex + c);
-    const uint32_t w = bs_append(V.ctile_list, &V.counters[CNT_CTILES], occ, (uint32_t)t, lane);
-    if (tile_rank) {
-        // rank inside the tile's size class (lanes of one class share an atomic)
-        const uint32_t cls = occ ? (uint32_t)bs_class(c) : (uint32_t)(CNT_BUCKETS + lane);
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls);
-        const int leader = __ffs(peers) - 1;
-        uint32_t b = 0;
-        if (occ && lane == leader) b = atomicAdd(&V.counters[CNT_BUCKET + cls], (uint32_t)__popc(peers));
-        b = __shfl_sync(0xFFFFFFFFu, b, leader);
-        if (occ) tile_rank[w] = (cls << 28) | (b + (uint32_t)__popc(peers & ((1u << lane) - 1u)));
+// tcount holds a multiple of 4 words past the tiles' and the overflow bin's
+// (zero), so a group of BS_GROUP or a run of 4 may be read whole
+__global__ void __launch_bounds__(BS_T) bs_groups(const uint32_t* __restrict__ tcount, int64_t n,
+                                                  uint32_t* __restrict__ gsum) {
+    static_assert(BS_GROUP == 4 * BS_T, "one 16-byte load per thread");
+    __shared__ uint32_t s_sum[BS_T / 32];
+    const int64_t i = (int64_t)blockIdx.x * BS_GROUP + 4 * threadIdx.x;
+    const uint4 c = i < n ? *reinterpret_cast<const uint4*>(tcount + i) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t w = __reduce_add_sync(0xFFFFFFFFu, c.x + c.y + c.z + c.w);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = w;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0u;
+#pragma unroll
+        for (int k = 0; k < BS_T / 32; ++k) t += s_sum[k];
+        gsum[blockIdx.x] = t;
     }
 }
 
 // Blocks [0, cell_blocks): (a), the rest: (b).  See the overview above.
-// (a) also clears the tile counts bs_count wrote (the occupied tiles' and
-// the overflow bin's, the only non-zero ones) for the next step.
-__global__ void __launch_bounds__(BS_T) bs_finish(View V, uint32_t* __restrict__ ccount,
-                                                  uint32_t* __restrict__ tcount,
-                                                  const uint32_t* __restrict__ toff, uint32_t* __restrict__ coff,
-                                                  uint2* __restrict__ cell_range, const uint32_t* __restrict__ tile_rank,
-                                                  uint32_t* __restrict__ ptile_list, int cell_blocks) {
-    const int lane = threadIdx.x & 31;
+// gsum: the groups' sums, or null where the tile counts are summed directly.
+template <int BT_PER_WARP>
+__global__ void __launch_bounds__(BS_T) bs_tiles(View V, SortCounts c, const uint32_t* __restrict__ gsum,
+                                                 uint2* __restrict__ cell_range, uint4* __restrict__ tile_info,
+                                                 int cell_blocks) {
+    constexpr int BT_TILES = BT_PER_WARP * (BS_T / 32);
+    static_assert(BT_TILES <= 64 && BT_TILES % 4 == 0, "two tiles per lane in the scan, 16-byte reads of the counts");
+    __shared__ uint32_t s_cnt[BT_TILES], s_slot[BT_TILES], s_rank[BT_TILES], s_sum[BS_T / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if ((int)blockIdx.x < cell_blocks) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) tcount[V.total_ct] = 0u;
-        const uint32_t ntiles = V.counters[CNT_CTILES];
-        const uint32_t nwarps = (uint32_t)cell_blocks * (BS_T / 32);
-        // first slot of each size class in the largest-first list
-        uint32_t cls_off = 0u;
-        if (ptile_list) {
-            const uint32_t cnt = lane < CNT_BUCKETS ? V.counters[CNT_BUCKET + lane] : 0u;
-            uint32_t x = cnt;
-#pragma unroll
-            for (int o = 1; o < CNT_BUCKETS; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-                if (lane >= o) x += y;
-            }
-            cls_off = x - cnt;
+        const int64_t t0 = (int64_t)blockIdx.x * BT_TILES;
+        uint32_t cnt = 0u;
+        if (threadIdx.x < BT_TILES) {
+            const int64_t t = t0 + threadIdx.x;
+            cnt = t < (int64_t)V.total_ct ? c.tcount[t] : 0u;
+            s_cnt[threadIdx.x] = cnt;
         }
-        for (uint32_t w = (blockIdx.x * BS_T + threadIdx.x) >> 5; w < ntiles; w += nwarps) {
-            const uint32_t t = V.ctile_list[w];
-            if (lane == 0) tcount[t] = 0u;
-            if (ptile_list) {
-                const uint32_t tr = tile_rank[w];
-                const uint32_t off = __shfl_sync(0xFFFFFFFFu, cls_off, (int)(tr >> 28));
-                if (lane == 0) ptile_list[off + (tr & 0x0FFFFFFFu)] = t;
+        if (blockIdx.x == 0 && threadIdx.x == 0) V.sort_work[SW_VALID] = (uint32_t)V.N - c.tcount[V.total_ct];
+        if (!__syncthreads_or(cnt > 0u)) return;
+        // this warp's cell counts, in flight while the offsets are summed
+        uint2 cc[BT_PER_WARP];
+#pragma unroll
+        for (int j = 0; j < BT_PER_WARP; ++j) {
+            const int i = warp * BT_PER_WARP + j;
+            cc[j] = s_cnt[i] ? reinterpret_cast<const uint2*>(c.ccount + (size_t)(t0 + i) * 64)[lane]
+                             : make_uint2(0u, 0u);
+        }
+        // particles in the tiles before this block's: whole groups, then tiles
+        uint32_t part = 0u;
+        int64_t first = 0;
+        if (gsum) {
+            const int64_t g = t0 / BS_GROUP;
+            for (int64_t i = threadIdx.x; i < g; i += BS_T) part += gsum[i];
+            first = g * BS_GROUP;
+        }
+#pragma unroll 8
+        for (int64_t i = first + 4 * threadIdx.x; i < t0; i += 4 * BS_T) {
+            const uint4 w = *reinterpret_cast<const uint4*>(c.tcount + i);  // t0 is a multiple of 4
+            part += w.x + w.y + w.z + w.w;
+        }
+        part = __reduce_add_sync(0xFFFFFFFFu, part);
+        if (lane == 0) s_sum[warp] = part;
+        if (threadIdx.x < (BT_TILES < 32 ? 32 : BT_TILES)) {  // whole warps
+            const bool occ = cnt > 0u;
+            const uint32_t lslot = bs_append(nullptr, &V.sort_work[SW_CTILES], occ, 0u, lane);
+            // rank inside the tile's size class (lanes of one class share an atomic)
+            const uint32_t cls = occ ? (uint32_t)bs_class(cnt) : (uint32_t)(CNT_BUCKETS + lane);
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls);
+            const int leader = __ffs(peers) - 1;
+            uint32_t b = 0;
+            if (occ && lane == leader) b = atomicAdd(&V.sort_work[SW_BUCKET + cls], (uint32_t)__popc(peers));
+            b = __shfl_sync(0xFFFFFFFFu, b, leader);
+            if (occ) {
+                s_slot[threadIdx.x] = lslot;
+                s_rank[threadIdx.x] = (cls << 28) | (b + (uint32_t)__popc(peers & ((1u << lane) - 1u)));
             }
-            uint2* cc2 = reinterpret_cast<uint2*>(ccount + (size_t)t * 64) + lane;
-            const uint2 cc = *cc2;
-            *cc2 = make_uint2(0u, 0u);  // left clear for the next step
-            uint32_t x = cc.x + cc.y;
+        }
+        __syncthreads();
+        uint32_t base = 0u;
+#pragma unroll
+        for (int w = 0; w < BS_T / 32; ++w) base += s_sum[w];
+        // exclusive scan of the block's tile counts, tiles 2 lane and 2 lane + 1 per lane
+        const uint32_t ca = 2 * lane < BT_TILES ? s_cnt[2 * lane] : 0u;
+        const uint32_t cb = 2 * lane < BT_TILES ? s_cnt[2 * lane + 1] : 0u;
+        uint32_t tx = ca + cb;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, tx, o);
+            if (lane >= o) tx += y;
+        }
+        const uint32_t te = base + tx - ca - cb;  // first position of tile 2 lane
+#pragma unroll
+        for (int j = 0; j < BT_PER_WARP; ++j) {
+            const int i = warp * BT_PER_WARP + j;
+            const uint32_t tcnt = s_cnt[i];
+            const uint32_t tb = __shfl_sync(0xFFFFFFFFu, (i & 1) ? te + ca : te, i >> 1);
+            if (tcnt == 0u) continue;
+            const uint32_t t = (uint32_t)t0 + (uint32_t)i;
+            uint32_t x = cc[j].x + cc[j].y;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
                 const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
                 if (lane >= o) x += y;
             }
-            const uint32_t e = toff[t] + x - cc.x - cc.y;  // first position of cell 2*lane
-            reinterpret_cast<uint2*>(coff + (size_t)t * 64)[lane] = make_uint2(e, e + cc.x);
-            if (cell_range) {
-                cell_range[(size_t)t * 64 + 2 * lane] = make_uint2(e, e + cc.x);
-                cell_range[(size_t)t * 64 + 2 * lane + 1] = make_uint2(e + cc.x, e + cc.x + cc.y);
-            }
+            const uint32_t e = tb + x - cc[j].x - cc[j].y;  // first position of cell 2 lane
+            reinterpret_cast<uint4*>(cell_range + (size_t)t * 64)[lane] =
+                make_uint4(e, e + cc[j].x, e + cc[j].x, e + cc[j].x + cc[j].y);
+            reinterpret_cast<uint2*>(c.ccount + (size_t)t * 64)[lane] = make_uint2(0u, 0u);  // clear for the next step
+            if (lane == 0) tile_info[s_slot[i]] = make_uint4(t, tb, tb + tcnt, s_rank[i]);
             if (V.sp.cap) {
                 // sparse grid: lanes 0..7 find (or claim) the slots of the 8
                 // node tiles the cell tile's stencils reach, list them for the
@@ -419,9 +436,9 @@ __global__ void __launch_bounds__(BS_T) bs_finish(View V, uint32_t* __restrict__
                 uint32_t nslot = SP_NONE;
                 uint32_t f = 0;
                 if (lane < 8) {
-                    int tx, ty, tz;
-                    sp_decode(V.sp.code[t], tx, ty, tz);
-                    nslot = sp_find_or_insert(V.sp, sp_code(tx + (lane & 1), ty + ((lane >> 1) & 1), tz + (lane >> 2)),
+                    int sx, sy, sz;
+                    sp_decode(V.sp.code[t], sx, sy, sz);
+                    nslot = sp_find_or_insert(V.sp, sp_code(sx + (lane & 1), sy + ((lane >> 1) & 1), sz + (lane >> 2)),
                                               f);
                     reinterpret_cast<uint32_t*>(V.sp.nbr + 2 * (size_t)t)[lane] = nslot == SP_NONE ? 0u : nslot;
                 }
@@ -431,7 +448,7 @@ __global__ void __launch_bounds__(BS_T) bs_finish(View V, uint32_t* __restrict__
                 // writer per (node tile, offset): t = nslot - offset)
                 if (lane < 8 && nslot != SP_NONE) V.sp.rev[8 * (size_t)nslot + lane] = make_uint2(t, stamp);
                 const bool fresh = lane < 8 && nslot != SP_NONE && atomicExch(&V.tile_flags[nslot], stamp) != stamp;
-                bs_append(V.tile_list, &V.counters[CNT_TILES], fresh, nslot, lane);
+                bs_append(V.tile_list, &V.sort_work[SW_TILES], fresh, nslot, lane);
             }
         }
         return;
@@ -439,38 +456,64 @@ __global__ void __launch_bounds__(BS_T) bs_finish(View V, uint32_t* __restrict__
     const int64_t nt = (int64_t)(blockIdx.x - cell_blocks) * BS_T + threadIdx.x;
     bool act = false;
     if (nt < V.total_nt) {
-        const int s = scene_of_node_tile(V, (int)nt);
-        const SceneDev& sc = V.scenes[s];
+        const SceneDev& sc = V.scenes[scene_of_node_tile(V, (int)nt)];
         const int l = (int)nt - sc.nt_base;
         const int x = l % sc.nt[0], y = (l / sc.nt[0]) % sc.nt[1], z = l / (sc.nt[0] * sc.nt[1]);
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             const int cx = x - (k & 1), cy = y - ((k >> 1) & 1), cz = z - (k >> 2);
             if (cx < 0 || cy < 0 || cz < 0 || cx >= sc.ct[0] || cy >= sc.ct[1] || cz >= sc.ct[2]) continue;
-            const int ct = sc.ct_base + (cz * sc.ct[1] + cy) * sc.ct[0] + cx;
-            act |= toff[ct + 1] > toff[ct];
+            act |= c.tcount[sc.ct_base + (cz * sc.ct[1] + cy) * sc.ct[0] + cx] > 0u;
         }
         V.tile_flags[nt] = act ? 1u : 0u;
     }
-    bs_append(V.tile_list, &V.counters[CNT_TILES], act, (uint32_t)nt, lane);
+    bs_append(V.tile_list, &V.sort_work[SW_TILES], act, (uint32_t)nt, lane);
 }
 
-__global__ void __launch_bounds__(BS_T) bs_scatter(const uint32_t* __restrict__ keys, int64_t n, uint32_t ncells,
-                                                   const uint32_t* __restrict__ slot,
-                                                   const uint32_t* __restrict__ coff,
-                                                   const uint32_t* __restrict__ toff_overflow,
-                                                   uint32_t* __restrict__ ok_, uint32_t* __restrict__ ov) {
+// Blocks [0, tile_blocks): the work list and the counters, the rest: the
+// particles.
+__global__ void __launch_bounds__(BS_T) bs_scatter(View V, const uint32_t* __restrict__ keys, SortCounts c,
+                                                   const uint2* __restrict__ cell_range,
+                                                   const uint4* __restrict__ tile_info, uint4* __restrict__ ptile,
+                                                   uint32_t* __restrict__ ok_, uint32_t* __restrict__ ov,
+                                                   int tile_blocks) {
+    const int64_t n = V.N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = (int64_t)blockIdx.x * BS_TILE + warp * (32 * BS_ITEMS);
+    if ((int)blockIdx.x < tile_blocks) {
+        // the largest-first work list, and the counters cleared for the next sort
+        const int gid = (int)blockIdx.x * BS_T + threadIdx.x, threads = tile_blocks * BS_T;
+        const uint32_t ntiles = V.sort_work[SW_CTILES];
+        uint32_t in_class[CNT_BUCKETS];
+#pragma unroll
+        for (int b = 0; b < CNT_BUCKETS; ++b) in_class[b] = V.sort_work[SW_BUCKET + b];
+        for (uint32_t i = gid; i < ntiles; i += threads) {
+            const uint4 t = tile_info[i];
+            const uint32_t cls = t.w >> 28;
+            uint32_t off = t.w & 0x0FFFFFFFu;
+#pragma unroll
+            for (uint32_t b = 0; b < (uint32_t)CNT_BUCKETS; ++b) off += b < cls ? in_class[b] : 0u;
+            ptile[off] = make_uint4(t.x, t.y, t.z, (uint32_t)scene_of_cell_tile(V, (int)t.x));
+            c.tcount[t.x] = 0u;
+        }
+        if (gid < CNT_RESET)
+            V.counters[gid] = gid == CNT_TILES ? V.sort_work[SW_TILES] : gid == CNT_CTILES ? ntiles : 0u;
+        if (gid == 0) {
+            c.tcount[V.total_ct] = 0u;
+            c.ccount[c.ncells] = 0u;
+        }
+        return;
+    }
+    const int64_t base = (int64_t)(blockIdx.x - tile_blocks) * BS_TILE + warp * (32 * BS_ITEMS);
     uint32_t k[BS_ITEMS], sl[BS_ITEMS], pos[BS_ITEMS];
 #pragma unroll
     for (int r = 0; r < BS_ITEMS; ++r) {
         const int64_t i = base + r * 32 + lane;
         k[r] = i < n ? keys[i] : 0u;
-        sl[r] = i < n ? slot[i] : 0u;
+        sl[r] = i < n ? c.slot[i] : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < BS_ITEMS; ++r) pos[r] = (k[r] < ncells ? coff[k[r]] : *toff_overflow) + sl[r];
+    for (int r = 0; r < BS_ITEMS; ++r)
+        pos[r] = (k[r] < c.ncells ? cell_range[k[r]].x : V.sort_work[SW_VALID]) + sl[r];
 #pragma unroll
     for (int r = 0; r < BS_ITEMS; ++r) {
         const int64_t i = base + r * 32 + lane;
@@ -482,26 +525,30 @@ __global__ void __launch_bounds__(BS_T) bs_scatter(const uint32_t* __restrict__ 
 }
 }  // namespace
 
-int64_t bin_sort_scan_blocks(int total_ct) { return ((int64_t)total_ct + 1 + BS_SCAN - 1) / BS_SCAN; }
+int64_t bin_sort_groups(int64_t total_ct) { return (total_ct + BS_GROUP) / BS_GROUP; }
 
-cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, cudaStream_t st) {
+cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool counted, cudaStream_t st) {
     const int64_t n = V.N;
     if (n <= 0) return cudaSuccess;
-    const uint32_t ncells = (uint32_t)V.total_ct * 64u;
-    const int64_t ntb = (int64_t)V.total_ct + 1;  // tiles + overflow bin
-    const int nb = (int)bin_sort_scan_blocks(V.total_ct);
+    if (!B.cell_range || !B.ptile || !V.sort_work) return cudaErrorInvalidValue;
     const int gk = (int)((n + BS_TILE - 1) / BS_TILE);
-    bs_count<<<gk, BS_T, 0, st>>>(B.keys_in, n, ncells, B.ccount, B.tcount, B.slot, V.counters);
-    const bool direct = nb <= BS_DIRECT_BLOCKS;
-    if (!direct) bs_reduce<<<nb, BS_SCAN, 0, st>>>(B.tcount, ntb, B.bsum);
-    bs_down<<<nb, BS_SCAN, 0, st>>>(V, B.tcount, ntb, direct ? nullptr : B.bsum, B.toff, B.ccount + ncells,
-                                    B.ptile_list ? B.tile_rank : nullptr);
-    const int cell_blocks = num_sms * 2;
+    const int64_t nct = V.total_ct;
+    if (!counted) bs_count<<<gk, BS_T, 0, st>>>(B.keys_in, n, B.cnt, V.counters);
+    const uint32_t* gsum = nct > BS_DIRECT_TILES ? B.gsum : nullptr;
+    if (gsum) bs_groups<<<(int)bin_sort_groups(nct), BS_T, 0, st>>>(B.cnt.tcount, nct + 1, B.gsum);
     // sparse grids mark their node tiles from the occupied cell tiles
     const int node_blocks = V.sp.cap ? 0 : (V.total_nt + BS_T - 1) / BS_T;
-    bs_finish<<<cell_blocks + node_blocks, BS_T, 0, st>>>(V, B.ccount, B.tcount, B.toff, B.coff, B.cell_range,
-                                                           B.tile_rank, B.ptile_list, cell_blocks);
-    bs_scatter<<<gk, BS_T, 0, st>>>(B.keys_in, n, ncells, B.slot, B.coff, B.toff + V.total_ct, B.out_k, B.out_v);
+    const int per_block = (nct <= BT_FEW_TILES ? BT_FEW : BT_MANY) * (BS_T / 32);
+    const int cell_blocks = (int)((nct + per_block - 1) / per_block);
+    if (nct <= BT_FEW_TILES)
+        bs_tiles<BT_FEW><<<cell_blocks + node_blocks, BS_T, 0, st>>>(V, B.cnt, gsum, B.cell_range, B.tile_info,
+                                                                    cell_blocks);
+    else
+        bs_tiles<BT_MANY><<<cell_blocks + node_blocks, BS_T, 0, st>>>(V, B.cnt, gsum, B.cell_range, B.tile_info,
+                                                                     cell_blocks);
+    const int tile_blocks = (int)std::min<int64_t>(num_sms, (nct + BS_T - 1) / BS_T);
+    bs_scatter<<<tile_blocks + gk, BS_T, 0, st>>>(V, B.keys_in, B.cnt, B.cell_range, B.tile_info, B.ptile, B.out_k,
+                                                 B.out_v, tile_blocks);
     return cudaGetLastError();
 }
 

@@ -50,3 +50,34 @@ def test_many_small_scenes_find_their_particles_and_tiles(gpu):
             one.step(6)
             _close({k: v[b:b + c] for k, v in out.items()}, one.download())
         b += c
+
+
+@pytest.mark.parametrize("N,n,boundary", [(1, (4, 4, 4), 0), (33, (5, 4, 7), 1), (255, (20, 11, 6), 2),
+                                          (2049, (35, 35, 35), 1), (5000, (66, 34, 70), 3)])
+def test_sorts_inside_a_call_equal_single_step_calls(gpu, N, n, boundary):
+    """A call of several steps counts each step's keys in the G2P before it;
+    calls of one step count them in the sort.  Both give the same particles,
+    and a sorted order that is a permutation with sorted keys."""
+    from physgrad_b200 import _capi as C
+    rng = np.random.default_rng(N)
+    dx = 1.0 / 32
+    scene = gpu.Scene(n, dx, 1e-3, (0.3, -9.8, 0.1), (0.0, 0.0, 0.0), 0, boundary, 1)
+    st = _scene_state(rng, N, n, dx)
+    st["v"] *= 4.0  # a tenth of the particles change cell in a step
+    mats = [gpu.createElasticMaterial(1000.0, 1e3, 0.3)]
+    a, b = gpu.Simulator([scene], [N], mats), gpu.Simulator([scene], [N], mats)
+    for s in (a, b):
+        s.upload(st["x"], st["v"], st["C"], st["F"], st["m"], st["V0"])
+    for calls in ((5, (1, 1, 1, 1, 1)), (2, (1, 1)), (1, (1,)), (3, (2, 1))):
+        keys = a.get_array(C.ARRAY_KEYS)
+        if calls[0] == 1:
+            before = keys
+        a.step(calls[0])
+        for k in calls[1]:
+            b.step(k)
+        if calls[0] == 1:  # the sort of this step is that of the keys before it
+            order, sk = a.get_array(C.ARRAY_SORTED_ORDER), a.get_array(C.ARRAY_SORTED_KEYS)
+            assert np.array_equal(np.sort(order), np.arange(N)) and np.array_equal(before[order], np.sort(before))
+            assert np.array_equal(sk, np.sort(before))
+    assert a.status() == b.status()
+    _close(a.download(), b.download())
