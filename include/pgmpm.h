@@ -238,10 +238,9 @@ PGMPM_API int pgmpm_set_tuning(pgmpm_solver s, int32_t p2g_block, int32_t ppt, i
  * 2: one thread per cell with 108 register accumulators;
  * 3: variant 2 with each cell's accumulators split over two lanes (MLS
  * forward; p2g_tiles_per_sm capped at 5);
- * 4: variant 3's lane pairs walking equal runs of each tile's sorted
- * particles instead of one cell each, cells shared by runs merged in shared
- * memory (MLS forward with the bin sort; with the radix step sort it runs
- * variant 3);
+ * 4: three threads per cell, one per z-offset of its stencil (MLS forward
+ * with the bin sort; with the radix step sort it runs variant 3;
+ * p2g_tiles_per_sm capped at 4);
  * 5: variant 4, fused with G2P: from the second step of a chain, each
  * step's G2P kernel also does the next step's P2G (one lane per run of a
  * tile's sorted particles, the tile's node velocities staged in shared

@@ -494,7 +494,7 @@ int pgmpm_create_ex(const pgmpm_scene_desc* scenes, int32_t n_scenes, const int6
     // the bin sort keeps 8 bytes per cell: default for grids with at most ~8
     // cells per particle, the radix sort (O(N) per pass) for sparser ones
     s->tune.step_sort = sparse || (int64_t)ct_base * 64 <= 8 * std::max<int64_t>(N, 1) + (1 << 20) ? 0 : 1;
-    // P2G (MLS): balanced particle runs over the bin sort's cell table;
+    // P2G (MLS): three threads per cell over the bin sort's cell table;
     // without it, two lanes per cell pays off when the occupied tiles
     // outnumber the resident blocks (many particles), one lane otherwise
     s->tune.p2g_variant = s->pf.physics != PHYS_MLS ? 2
@@ -930,6 +930,7 @@ int pgmpm_get_metrics(pgmpm_solver s, pgmpm_metrics* out) {
     s->met.g2p_variant = s->tune.g2p_variant;
     s->met.p2g_tiles_per_sm = s->tune.p2g_variant == 5   ? s->tune.g2p2g_blocks_per_sm
                               : s->tune.p2g_variant == 2 ? s->tune.cell_blocks_per_sm
+                              : s->tune.p2g_variant == 4 ? std::min(4, s->tune.pair_blocks_per_sm)
                               : s->tune.p2g_variant >= 3 ? s->tune.pair_blocks_per_sm
                                                          : s->tune.tile_blocks_per_sm;
     s->met.g2p_tiles_per_sm = s->tune.g2p_tiles_per_sm;
@@ -961,7 +962,7 @@ int pgmpm_autotune(pgmpm_solver s, int32_t reps, void* stream) {
     struct Cand {
         int variant, block, ppt, tiles_per_sm;
     };
-    const Cand p2g_c[] = {{4, 128, 0, 4}, {4, 128, 0, 5}, {3, 128, 0, 4}, {3, 128, 0, 5}, {2, 64, 0, 4}, {2, 64, 0, 6}, {2, 64, 0, 8},
+    const Cand p2g_c[] = {{4, 192, 0, 3}, {4, 192, 0, 4}, {3, 128, 0, 4}, {3, 128, 0, 5}, {2, 64, 0, 4}, {2, 64, 0, 6}, {2, 64, 0, 8},
                           {0, 192, 0, 2}, {0, 192, 0, 3}, {1, 256, 512, 0}, {1, 256, 1024, 0}};
     const Cand g2p_c[] = {{2, 128, 0, 0}, {2, 256, 0, 0}, {2, 512, 0, 0}, {0, 256, 0, 2},
                           {1, 128, 0, 0}, {1, 256, 0, 0}};

@@ -4,15 +4,16 @@
 //   [sort]   bin sort of the cell keys written by the previous G2P
 //            (pgmpm_sort.cu): occupied cell tiles, their sorted ranges, each
 //            cell's range, and the active node tiles
-//   P2G      default k_p2g_cells: one 64-thread block per occupied 4^3 cell
-//            tile, thread c owns cell c and the 27 nodes of its stencil (108
-//            register accumulators), walks its cell's particles and adds the
-//            payload (m, b, affine matrix, stencil fraction) precomputed by
-//            the previous G2P; the block then sums the 6^3 nodes the tile
-//            touches in shared memory and flushes each with one vector atomic
-//            (red.global.add.v4.f32) into grid_mp.  k_p2g_tiles (cell x
-//            z-slice) and k_p2g (chunks, shared atomics) are the other
-//            variants.
+//   P2G      default k_p2g_slices (MLS): a block per occupied 4^3 cell tile,
+//            three threads per cell, each summing the 9 nodes of one z-offset
+//            of the cell's stencil over the cell's particles (payload (m, b,
+//            affine matrix, stencil fraction) precomputed by the previous
+//            G2P); the block then sums the 6^3 nodes the tile touches in
+//            shared memory and flushes each with one vector atomic
+//            (red.global.add.v4.f32) into grid_mp.  k_p2g_cells (thread per
+//            cell; REF physics), k_p2g_pairs (lane pair per cell), k_p2g_tiles
+//            (cell x z-slice, payload staged) and k_p2g (chunks, shared
+//            atomics) are the other variants.
 //   k_grid   active node tiles only: v = p/m + dt g, walls, (v, m) -> grid_v,
 //            grid_mp cleared for the next step.
 //   G2P      default k_g2p_phys: one thread per particle in physical order:
@@ -922,193 +923,204 @@ __global__ void __launch_bounds__(P2GP_T, 5) k_p2g_pairs(View V) {
     if (flags) atomicOr(&V.counters[CNT_FLAGS], flags);
 }
 
-// ------------------------------------ P2G, balanced particle runs (MLS)
-// Variant 4: variant 3's lane pairs and accumulators, with the work split by
-// particles instead of by cells.  A work item's sorted particles (a tile, or
-// a slice of one) are cut into 4 warp parts at the cell boundaries nearest
-// the quarter points, and each warp cuts its part into 16 equal runs, one per
-// lane pair.  A pair walks its run in key order; when it passes the last
-// particle of a cell it owns that cell and writes the cell's 27 node sums to
-// the flush table (one writer per cell).  A run that ends inside a cell
-// leaves a partial sum: after the walk, a segmented scan over the warp's
-// pairs (shuffles) gathers each cell's partials into the last of them, which
-// adds them to the owner's entry.  Warp parts end at cell boundaries, so a
-// cell never spans two warps.  A tile's longest walk is then about its
-// particle count / 64 instead of its fullest cell's count.  Needs the sort's
-// cell table (contiguous ranges of the tile's 64 cells).
-constexpr int P2GR_T = 128;
+// Asynchronous global -> shared copies (cp.async, no registers held while
+// the copy is in flight); completion per thread with cp_async_wait<n>.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+template <int N_>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N_) : "memory");
+}
 
-__device__ __forceinline__ void runs_store(float4* T4, uint32_t c, int h, const float* accA, const float* accB) {
+// ------------------------------------------ P2G, cell z-slices (MLS)
+// Variant 4: a 192-thread block per occupied cell tile; thread 3 c + k walks
+// cell c's particles and sums the 9 nodes at z-offset k of its stencil (36
+// accumulators, 80 registers, 4 blocks per SM).  The three threads of a cell
+// read the same payload with one request.  Between the tiles of a block only
+// two barriers: the next tile's record is copied to shared memory during the
+// walk, its cell ranges and first particle indices are loaded while the nodes
+// are summed, and a block's first tile needs no claim.
+//
+// What bounds it: up to a few tens of thousands of particles the chain of
+// dependent reads (list -> cell range -> order -> payload -> sums), above that
+// instructions (47% of the issue slots) and the payload loads' latency, and on
+// thinly filled grids the node sums.  Balanced particle runs (a lane pair per
+// 1/64 of a tile, partial sums of split cells joined by a segmented scan), the
+// former variant 4, kept every lane busy but spent two thirds of their
+// instructions on the flush.  P2G per step, runs -> slices: 4,096 particles
+// 9.7 -> 5.1 us, 32,768: 13.4 -> 8.2, 150 K: 18.3 -> 15.4, 262 K sparse: 22.0
+// -> 17.7, 2 M (two densities): 98.0 -> 89.9, 64 scenes of 3.9 M (2 per cell):
+// 268 -> 237.  Slower: 5 blocks per SM (64 registers, spills: 109 us at 2 M),
+// half tiles in 96-thread blocks (104), cells dealt to the warps by particle
+// count (102: the ranking's barriers, and neighbouring lanes no longer share
+// sectors), the next payload prefetched into registers (115), the sums on
+// packed FP32 pairs (91.6: the doubled weights cost moves).
+constexpr int P2GS_T = 192;
+constexpr int P2GS_BLOCKS = 4;          // resident blocks per SM
+constexpr int P2GS_PLANE = 9 * 64 + 3;  // float4s per z-offset of the flush table (3 more: see the stores)
+
+// Sum of the contributions to node (nx, ny, nz) of the 6^3 node block of a
+// 4^3 cell tile, from T4[z-offset][x-offset + 3 y-offset][cell].  Offsets
+// whose cell falls outside the tile are skipped: z-offsets by the whole warp
+// where it can (its lanes mostly share nz), the others by predicate.
+__device__ __forceinline__ float4 slices_node_sum(const float4* T4, int nx, int ny, int nz) {
+    const uint32_t vx = (nx <= 3 ? 1u : 0u) | (nx >= 1 && nx <= 4 ? 2u : 0u) | (nx >= 2 ? 4u : 0u);
+    const uint32_t vy = (ny <= 3 ? 1u : 0u) | (ny >= 1 && ny <= 4 ? 2u : 0u) | (ny >= 2 ? 4u : 0u);
+    const int cn = nx + 4 * ny + 16 * nz;
+    float2 a = f2(0.f), b = f2(0.f);
 #pragma unroll
-    for (int o = 0; o < 27; ++o) reinterpret_cast<float2*>(&T4[o * 64 + c])[h] = make_float2(accA[o], accB[o]);
+    for (int zz = 0; zz < 3; ++zz) {
+        if ((unsigned)(nz - zz) > 3u) continue;
+        const float4* plane = T4 + zz * (P2GS_PLANE - 16) + cn;
+#pragma unroll
+        for (int yy = 0; yy < 3; ++yy)
+#pragma unroll
+            for (int xx = 0; xx < 3; ++xx)
+                if ((vx >> xx) & (vy >> yy) & 1u) {
+                    const float4 t = plane[(xx + 3 * yy) * 64 - (xx + 4 * yy)];
+                    a = f2_add(a, make_float2(t.x, t.y));
+                    b = f2_add(b, make_float2(t.z, t.w));
+                }
+    }
+    return make_float4(a.x, a.y, b.x, b.y);
 }
 
 template <bool SPARSE>
-__global__ void __launch_bounds__(P2GR_T, 5) k_p2g_runs(View V) {
-    __shared__ float4 T4[27 * 64];                // [offset o][cell]: the 4 channels of cell's node o
-    __shared__ uint32_t s_end[P2GR_T / 32][64];   // per warp: end of each cell's range in the item
-    __shared__ uint32_t s_work;
-    constexpr uint32_t FULL = 0xFFFFFFFFu;
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int q = lane >> 1, h = lane & 1;
+__global__ void __launch_bounds__(P2GS_T, P2GS_BLOCKS) k_p2g_slices(View V) {
+    __shared__ float4 T4[3 * P2GS_PLANE];  // [z-offset][x-offset + 3 y-offset][cell]: (m, p) of the cell's node
+    __shared__ uint4 s_item[2];            // this and the next item's tile (see View::ptile)
+    __shared__ uint32_t s_slice[2];        // and its slice; ~0: no item
+    constexpr uint32_t NONE = 0xFFFFFFFFu;
+    const int t = threadIdx.x;
+    const int q = t / 3, k = t - 3 * (t / 3);
+    const float kf = (float)k;
+    const float wo = k == 0 ? 1.5f : k == 1 ? 1.0f : 0.5f;  // w_k(f) is a quadratic in f - wo
     const int64_t N = V.N;
-    uint32_t flags = 0;
-    uint32_t* const wend = s_end[wp];
     const uint32_t ntiles = V.counters[CNT_CTILES];
-    // slices of a tile's particles when tiles are few (see k_p2g_cells)
+    // slices of a cell's particles when tiles are few: one work item per
+    // (tile, slice)
     const uint32_t S = ntiles ? min(4u, max(1u, (gridDim.x + ntiles - 1) / ntiles)) : 1u;
     const uint32_t nwork = ntiles * S;
+    // items [0, gridDim.x) are the blocks' first; further ones are claimed,
+    // one ahead when there are enough of them that no block holds a claim
+    // another one idles for
+    const bool more = nwork > gridDim.x;
     const bool early = nwork >= 2u * gridDim.x;
-    uint32_t next_work = 0;
-    if (threadIdx.x == 0) s_work = atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
-    for (;;) {
-        __syncthreads();
-        const uint32_t w = s_work;
-        if (w >= nwork) break;
-        if (early && threadIdx.x == 0) next_work = atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
-        const uint32_t wt = w / S, slice = w - wt * S;
-        const TileWork work = tile_work(V, wt);  // largest tiles first
-        const uint32_t ct = work.ct;
-        const uint2 rg = work.rg;
-        const int s = work.s;
-        const SceneDev& sc = scene_ref(V, s);
-        int ox, oy, oz0;
-        tile_origin(V, sc, ct, ox, oy, oz0);
-        // the item's particles [lo, hi) and its cells' ranges clamped to them
-        // (lane holds cells lane and lane + 32)
-        const uint32_t P = rg.y > rg.x ? rg.y - rg.x : 0u;
-        const uint32_t lo = rg.x + (uint32_t)(((uint64_t)P * slice) / S);
-        const uint32_t hi = rg.x + (uint32_t)(((uint64_t)P * (slice + 1)) / S);
-        const uint2 r0 = V.cell_range[(size_t)ct * 64 + lane], r1 = V.cell_range[(size_t)ct * 64 + 32 + lane];
-        const uint32_t s0 = min(max(r0.x, lo), hi), s1 = min(max(r1.x, lo), hi);
-        const uint32_t e0 = min(max(r0.y, lo), hi), e1 = min(max(r1.y, lo), hi);
-        if ((lane == 0 && s0 != lo) || (lane == 31 && e1 != hi)) flags |= FLAG_TILE_RANGE;
-        wend[lane] = e0;
-        wend[lane + 32] = e1;
-        // warp part [b0, b1): the cell starts nearest the quarter points
-        auto bound = [&](int k) -> uint32_t {
-            if (k == 0) return lo;
-            if (k == 4) return hi;
-            const uint32_t t = lo + (uint32_t)(((uint64_t)(hi - lo) * (uint32_t)k) / 4u);
-            const uint32_t a = __reduce_max_sync(FULL, max(s0 <= t ? s0 : lo, s1 <= t ? s1 : lo));
-            const uint32_t b = __reduce_min_sync(FULL, min(s0 >= t ? s0 : hi, s1 >= t ? s1 : hi));
-            return t - a <= b - t ? a : b;
-        };
-        const uint32_t b0 = bound(wp), b1 = max(bound(wp + 1), b0);
-        const uint32_t len = (b1 - b0 + 15u) >> 4;
-        const uint32_t i0 = min(b0 + (uint32_t)q * len, b1), i1 = min(i0 + len, b1);
-        __syncwarp();
-        // cells without particles in the item get a zero entry (warp wp: cells
-        // 16 wp .. 16 wp + 15, the half-warps take alternate offsets)
-        {
-            const int zc = 16 * wp + (lane & 15);
-            const uint32_t zs = zc == 0 ? lo : wend[zc - 1];
-            if (wend[zc] == zs)
-                for (int o = lane >> 4; o < 27; o += 2) T4[o * 64 + zc] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // thread 0: work item w's tile record to s_item[c], asynchronously
+    auto fetch = [&](uint32_t w, int c) {
+        uint32_t slice = NONE;
+        if (w < nwork) {
+            const uint32_t wi = w / S;
+            cp_async16(&s_item[c], &V.ptile[wi]);
+            slice = w - wi * S;
         }
-        float accA[27], accB[27];
-#pragma unroll
-        for (int o = 0; o < 27; ++o) accA[o] = accB[o] = 0.f;
-        // the cell of particle i0: the first cell whose range ends after it
-        uint32_t c = 0, cend = 0;
-        if (i0 < i1) {
-            uint32_t l = 0, r = 63;
-            while (l < r) {
-                const uint32_t m = (l + r) >> 1;
-                if (wend[m] > i0) r = m; else l = m + 1;
-            }
-            c = l;
-            cend = wend[c];
+        s_slice[c] = slice;
+    };
+    uint32_t claimed = NONE;
+    if (t == 0) {
+        fetch(blockIdx.x, 0);
+        if (early) claimed = gridDim.x + atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
+        cp_async_wait_all();
+    }
+    __syncthreads();
+    // this thread's cell of the current item: particles b, b + S, .. < e
+    uint32_t b = 0, e = 0, pn = 0;
+    bool work = s_slice[0] != NONE;
+    if (work) {
+        const uint4 item = s_item[0];
+        const uint2 r = V.cell_range[(size_t)item.x * 64 + q];
+        b = max(r.x, item.y) + s_slice[0];
+        e = min(r.y, item.z);
+        pn = b < e ? V.order[b] : 0u;
+    }
+    int cur = 0;
+    while (work) {
+        // thread 0: the next item's tile, in flight during the walk
+        if (early && t == 0) {
+            fetch(claimed, cur ^ 1);
+            if (claimed < nwork) claimed = gridDim.x + atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
         }
-        // the next particle's index is loaded one iteration ahead, so an
-        // iteration's payload loads do not wait on its index load (P2G of the
-        // two-material drop: 110.5 -> 107.4 us)
-        uint32_t pn = i0 < i1 ? V.order[i0] : 0u;
-        for (uint32_t i = i0; i < i1; ++i) {
-            const uint32_t p = pn;
-            if (i + 1 < i1) pn = V.order[i + 1];
-            if (i == cend) {
-                // the run passed the last particle of cell c: its sums are final
-                runs_store(T4, c, h, accA, accB);
+        float acc[9][4];  // node (i, j, k) of the cell: (m, p)
 #pragma unroll
-                for (int o = 0; o < 27; ++o) accA[o] = accB[o] = 0.f;
-                while (c < 63) {  // next cell with particles (c stays a cell index)
-                    ++c;
-                    if (wend[c] > i) break;
-                }
-                cend = wend[c];
-            }
-            if (p >= (uint32_t)N) {
-                flags |= FLAG_TILE_RANGE;
-                continue;
-            }
+        for (int o = 0; o < 9; ++o) acc[o][0] = acc[o][1] = acc[o][2] = acc[o][3] = 0.f;
+        for (uint32_t i = b; i < e; i += S) {
+            // an index out of range (reported) reads the last particle; no
+            // branch here, so that the loads below issue together
+            if (pn >= (uint32_t)N) atomicOr(&V.counters[CNT_FLAGS], FLAG_TILE_RANGE);
+            const uint32_t p = min(pn, (uint32_t)N - 1u);
             const float4 a0 = V.pay[p], a1 = V.pay[N + p], a2 = V.pay[2 * N + p], a3 = V.pay[3 * N + p];
-            // channels as in k_p2g_pairs (lane 0: m, p_x; lane 1: p_y, p_z)
-            const float bA = h ? a0.y : a0.w, bB = h ? a0.z : a0.x;
-            const float gAx = h ? a1.w : 0.f, gAy = h ? a2.x : 0.f, gAz = h ? a2.y : 0.f;
-            const float gBx = h ? a2.z : a1.x, gBy = h ? a2.w : a1.y, gBz = h ? a3.x : a1.z;
-            float wt[3][3];
-            mls_weights(a3.y, wt[0]);
-            mls_weights(a3.z, wt[1]);
-            mls_weights(a3.w, wt[2]);
+            if (i + S < e) pn = V.order[i + S];  // the next particle's, in flight during this one's sums
+            // a0 = (b, m), a1 = Ad[0..3], a2 = Ad[4..7], a3 = (Ad[8], f);
+            // node o gets w_o (m, b + Ad o), stepped one matrix column per node
+            float wx[3], wy[3];
+            mls_weights(a3.y, wx);
+            mls_weights(a3.z, wy);
+            const float az = a3.w - wo;
+            const float az2 = az * az;
+            const float wz = k == 1 ? 0.75f - az2 : 0.5f * az2;
+            float X = a0.x + kf * a1.z, Y = a0.y + kf * a2.y, Z = a0.z + kf * a3.x;
 #pragma unroll
-            for (int zz = 0; zz < 3; ++zz) {
-                const float zA = bA + gAz * (float)zz, zB = bB + gBz * (float)zz;
+            for (int j = 0; j < 3; ++j) {
+                const float wyz = wy[j] * wz;
+                float x = X, y = Y, z = Z;
 #pragma unroll
-                for (int yy = 0; yy < 3; ++yy) {
-                    const float wyz = wt[1][yy] * wt[2][zz];
-                    float vA = zA + gAy * (float)yy, vB = zB + gBy * (float)yy;
-#pragma unroll
-                    for (int xx = 0; xx < 3; ++xx) {
-                        const int o = xx + 3 * yy + 9 * zz;
-                        const float wgt = wt[0][xx] * wyz;
-                        accA[o] += wgt * vA;
-                        accB[o] += wgt * vB;
-                        vA += gAx;
-                        vB += gBx;
+                for (int ii = 0; ii < 3; ++ii) {
+                    const float wgt = wx[ii] * wyz;
+                    float* a = acc[3 * j + ii];
+                    a[0] += wgt * a0.w;
+                    a[1] += wgt * x;
+                    a[2] += wgt * y;
+                    a[3] += wgt * z;
+                    if (ii < 2) {
+                        x += a1.x;
+                        y += a1.w;
+                        z += a2.z;
                     }
                 }
-            }
-        }
-        // a run that ends where its cell ends owns that cell; otherwise the
-        // cell's owner is a later pair of this warp and the sum is partial
-        const bool open = i0 < i1 && i1 != cend;
-        if (i0 < i1 && !open) runs_store(T4, c, h, accA, accB);
-        __syncwarp();
-        // segmented inclusive scan of the partial sums over consecutive pairs
-        // of the same cell; the last pair of a segment then holds its total
-        const uint32_t key = open ? c : FULL;
-        const uint32_t pkey = __shfl_up_sync(FULL, key, 2), nkey = __shfl_down_sync(FULL, key, 2);
-        const bool head = open && (q == 0 || pkey != key);
-        const uint32_t heads = __ballot_sync(FULL, head && h == 0);
-        const int dist = open ? q - ((31 - __clz(heads & (FULL >> (31 - lane)))) >> 1) : 0;
-        const int maxd = __reduce_max_sync(FULL, dist);
-        for (int d = 1; d <= maxd; d <<= 1) {
-            const bool take = dist >= d;
-#pragma unroll
-            for (int o = 0; o < 27; ++o) {
-                const float a = __shfl_up_sync(FULL, accA[o], 2 * d);
-                const float b = __shfl_up_sync(FULL, accB[o], 2 * d);
-                if (take) {
-                    accA[o] += a;
-                    accB[o] += b;
+                if (j < 2) {
+                    X += a1.y;
+                    Y += a2.x;
+                    Z += a2.w;
                 }
             }
         }
-        if (open && (q == 15 || nkey != key)) {
+        // flush: each thread stores its 9 nodes; then node n sums the offsets
+        // o whose cell n - o lies in the tile and issues one vector atomic.
+        // Planes 3 entries apart mod 8 keep a cell's three threads on
+        // different banks.
 #pragma unroll
-            for (int o = 0; o < 27; ++o) {
-                float2* t = reinterpret_cast<float2*>(&T4[o * 64 + c]) + h;
-                const float2 v = *t;
-                *t = make_float2(v.x + accA[o], v.y + accB[o]);
-            }
+        for (int o = 0; o < 9; ++o)
+            T4[k * P2GS_PLANE + o * 64 + q] = make_float4(acc[o][0], acc[o][1], acc[o][2], acc[o][3]);
+        const uint32_t ct = s_item[cur].x;
+        const SceneDev& sc = scene_ref(V, (int)s_item[cur].w);
+        cur ^= 1;
+        if (t == 0) {
+            if (!early) fetch(more ? gridDim.x + atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u) : NONE, cur);
+            cp_async_wait_all();
         }
         __syncthreads();
+        int ox, oy, oz0;
+        tile_origin(V, sc, ct, ox, oy, oz0);
+        // the next item's cells, in flight during the sums
+        work = s_slice[cur] != NONE;
+        uint2 r = make_uint2(0u, 0u);
+        if (work) r = V.cell_range[(size_t)s_item[cur].x * 64 + q];
         uint32_t nb[8];  // sparse: the slots of the 8 node tiles of the tile's node block
         if (SPARSE) sp_load_nbr(V.sp, ct, nb);
-        for (int n = threadIdx.x; n < TILE_NODES; n += P2GR_T) {
-            const int nx = n % TN, ny = (n / TN) % TN, nz = n / (TN * TN);
-            const float4 a4 = tile_node_sum(T4, nx, ny, nz);
+        auto flush = [&](int nx, int ny, int nz) {
+            const float4 a4 = slices_node_sum(T4, nx, ny, nz);
             const int gi = ox + nx, gj = oy + ny, gk = oz0 + nz;
             if (a4.x != 0.f && gi < sc.n[0] && gj < sc.n[1] && gk < sc.n[2]) {
                 if (SPARSE)
@@ -1116,17 +1128,23 @@ __global__ void __launch_bounds__(P2GR_T, 5) k_p2g_runs(View V) {
                 else
                     atomicAdd(&V.grid_mp[node_index(sc, gi, gj, gk)], a4);
             }
-        }
+        };
+        // warp z takes the first 32 of the 36 nodes of plane z; warp 0, whose
+        // plane has one z-offset, also the last 4 of every plane
+        const int l = t & 31, wp = t >> 5;
+        flush(l % TN, l / TN, wp);
+        b = max(r.x, s_item[cur].y) + s_slice[cur];
+        e = min(r.y, s_item[cur].z);
+        pn = work && b < e ? V.order[b] : 0u;
+        if (wp == 0 && l < 24) flush(2 + (l & 3), 5, l >> 2);
         __syncthreads();
-        if (threadIdx.x == 0) s_work = early ? next_work : atomicAdd(&V.counters[CNT_P2G_CURSOR], 1u);
     }
-    if (flags) atomicOr(&V.counters[CNT_FLAGS], flags);
 }
 
 // ------------------------------ adjoint scatter, balanced particle runs
-// Reverse of G2P (the adjoint payload scattered to the grid adjoint) with
-// k_p2g_runs' work split at one lane per run: a particle's adjoint payload
-// takes a whole thread's registers.  A 64-thread block takes a tile (or a
+// Reverse of G2P (the adjoint payload scattered to the grid adjoint): a
+// tile's particles cut into equal runs, one lane per run (a particle's adjoint
+// payload takes a whole thread's registers).  A 64-thread block takes a tile (or a
 // slice of one); its two warps take the halves split at the cell boundary
 // nearest the midpoint, and each lane an equal run of its half.  A run
 // stores the sums of each cell whose last particle it passes (one writer
@@ -1771,26 +1789,6 @@ __global__ void __launch_bounds__(256) k_g2p_tiles(View V) {
 // registers, no spills; 6: 168 registers, some spilled).
 constexpr int G2_T = 64;
 
-// Asynchronous global -> shared copies (cp.async, no registers held while
-// the copy is in flight); completion per thread with cp_async_wait<n>.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-    const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N_>
-__device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N_) : "memory");
-}
-
 // One particle's G2P inputs staged in shared memory: q0..q2 (x, F), then
 // (m, V0) and the material id.
 struct G2Stage {
@@ -2296,9 +2294,9 @@ cudaError_t launch_p2g(const View& V, const PhysFlags& pf, const Tuning& t, int 
         if (!V.pay) return cudaErrorInvalidValue;
         if (t.p2g_variant >= 4 && V.cell_range)  // without the sort's cell table: variant 3
             if (V.sp.cap)
-                k_p2g_runs<true><<<num_sms * t.pair_blocks_per_sm, P2GR_T, 0, st>>>(V);
+                k_p2g_slices<true><<<num_sms * min(P2GS_BLOCKS, t.pair_blocks_per_sm), P2GS_T, 0, st>>>(V);
             else
-                k_p2g_runs<false><<<num_sms * t.pair_blocks_per_sm, P2GR_T, 0, st>>>(V);
+                k_p2g_slices<false><<<num_sms * min(P2GS_BLOCKS, t.pair_blocks_per_sm), P2GS_T, 0, st>>>(V);
         else
             k_p2g_pairs<<<num_sms * t.pair_blocks_per_sm, P2GP_T, 0, st>>>(V);
         return cudaGetLastError();

@@ -81,3 +81,41 @@ def test_sorts_inside_a_call_equal_single_step_calls(gpu, N, n, boundary):
             assert np.array_equal(sk, np.sort(before))
     assert a.status() == b.status()
     _close(a.download(), b.download())
+
+
+@pytest.mark.parametrize("counts", [[1], [64], [1, 0, 3], [700], [5, 900, 2, 1, 40], [2000, 1]])
+@pytest.mark.parametrize("sparse", [False, True])
+def test_p2g_of_uneven_cells_equals_thread_per_cell(gpu, counts, sparse):
+    """Cells of very different counts, at tile corners and on the tiles' seams:
+    the grid of one step against the P2G with one thread per cell.  A node
+    sums at most n = all particles' terms, so two orders of summation differ
+    by at most n 2^-23 of the sum of the terms' sizes, bounded by n 2^-23
+    times the largest nodal mass (and momentum, whose terms are bounded by
+    m (|v| + |C| dx), 4 units of velocity here)."""
+    rng = np.random.default_rng(len(counts) + sum(counts))
+    n, dx = (23, 22, 21), 1.0 / 16
+    xs = []
+    for i, c in enumerate(counts):
+        # origins on a tile's first cell, its last cell, and in between
+        cell = np.array([[4, 4, 4], [7, 7, 7], [8, 7, 4], [11, 8, 8], [0, 0, 0], [19, 18, 17]])[i % 6]
+        xs.append((cell + 0.5 + rng.uniform(0.05, 0.95, (c, 3))) * dx)
+    x = np.concatenate(xs).astype(np.float32)
+    N = len(x)
+    V0 = np.full(N, (dx / 2) ** 3, np.float32)
+    scene = gpu.Scene(n, dx, 1e-4, (0.0, 0.0, 0.0), (0.0, 0.0, 0.0), 0, 0, 0)
+    v, Cm = rng.uniform(-1, 1, (N, 3)).astype(np.float32), rng.uniform(-5, 5, (N, 9)).astype(np.float32)
+    F = np.tile(np.eye(3, dtype=np.float32).ravel(), (N, 1))
+    grids = []
+    for variant in (4, 2):
+        sim = gpu.Simulator([scene], [N], [gpu.createElasticMaterial(1000.0, 0.0, 0.3)],
+                            sparse_tiles=512 if sparse and variant == 4 else None)
+        if variant != 4:
+            sim.set_variants(p2g_variant=variant)
+        sim.upload(x, v, Cm, F, (1000 * V0).astype(np.float32), V0)
+        sim.step(1)
+        m, gv = sim.grid()
+        grids.append((m, gv * m[:, None]))
+        assert sim.status() == 0
+    bound = N * 2.0 ** -23
+    assert np.abs(grids[0][0] - grids[1][0]).max() <= bound * grids[1][0].max()
+    assert np.abs(grids[0][1] - grids[1][1]).max() <= 4 * bound * grids[1][0].max() + 1e-12
