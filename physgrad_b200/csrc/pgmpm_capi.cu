@@ -650,30 +650,18 @@ int pgmpm_upload(pgmpm_solver s, const float* x, const float* v, const float* C,
     }
     if (N > 0) {
         View V = s->view();
-        // 1. identity pack (user order) to compute the keys
-        CK(cudaMemsetAsync(s->keys.p, 0, sizeof(uint32_t) * N, st));
-        // order = identity: use va as a temporary iota through the sort of all-zero keys
-        int w0 = 0;
-        CK(radix_sort_pairs(s->keys.as<uint32_t>(), nullptr, s->ka.as<uint32_t>(), s->va.as<uint32_t>(),
-                            s->kb.as<uint32_t>(), s->vb.as<uint32_t>(), s->sort_scratch.as<uint32_t>(), N, 1, &w0,
-                            st));
-        const uint32_t* iota = w0 ? s->vb.as<uint32_t>() : s->va.as<uint32_t>();
-        CK(launch_pack(V, dx_, dv, dC, dF, dm, dV0, dmat, iota, s->user_of_phys.as<uint32_t>(), s->phys_of_user.as<uint32_t>(), s->mV.as<float2>(),
-                       s->pf.multi_mat ? s->mat.as<int32_t>() : nullptr, st));
-        // 2. keys of the user-order positions, stable sort -> physical order
-        CK(launch_keys(V, s->pf, st));
+        // 1. keys of the positions in upload order, stable sort -> physical order
+        CK(launch_keys(V, dx_, s->pf, st));
         int which = 0;
         CK(radix_sort_pairs(s->keys.as<uint32_t>(), nullptr, s->ka.as<uint32_t>(), s->va.as<uint32_t>(),
                             s->kb.as<uint32_t>(), s->vb.as<uint32_t>(), s->sort_scratch.as<uint32_t>(), N,
                             s->key_bits, &which, st));
         const uint32_t* ord = which ? s->vb.as<uint32_t>() : s->va.as<uint32_t>();
         const uint32_t* sk = which ? s->kb.as<uint32_t>() : s->ka.as<uint32_t>();
-        // 3. pack in sorted order; the sorted keys are the keys of the physical order
-        CK(launch_pack(V, dx_, dv, dC, dF, dm, dV0, dmat, ord, s->user_of_phys.as<uint32_t>(), s->phys_of_user.as<uint32_t>(), s->mV.as<float2>(),
+        // 2. the state, its keys and its payload in sorted order
+        CK(launch_pack(V, dx_, dv, dC, dF, dm, dV0, dmat, ord, sk, s->user_of_phys.as<uint32_t>(),
+                       s->phys_of_user.as<uint32_t>(), s->mV.as<float2>(),
                        s->pf.multi_mat ? s->mat.as<int32_t>() : nullptr, st));
-        CK(cudaMemcpyAsync(s->keys.p, sk, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, st));
-        int rc = refresh_payload(s, st);
-        if (rc) return rc;
     }
     s->uploaded = true;
     return PGMPM_OK;

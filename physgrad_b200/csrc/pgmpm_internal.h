@@ -238,7 +238,8 @@ struct PhysFlags {
     bool has_fluid;  // some material uses the EOS model
     bool has_plastic;  // some material is ELASTOPLASTIC (von Mises)
 };
-cudaError_t launch_keys(const View& V, const PhysFlags& pf, cudaStream_t st);
+// x: the caller's positions, upload order; writes V.keys in that order
+cudaError_t launch_keys(const View& V, const float* x, const PhysFlags& pf, cudaStream_t st);
 cudaError_t launch_payload(const View& V, const PhysFlags& pf, cudaStream_t st);
 cudaError_t launch_mark(const View& V, cudaStream_t st);
 cudaError_t launch_p2g(const View& V, const PhysFlags& pf, const Tuning& t, int num_sms, cudaStream_t st);
@@ -250,8 +251,8 @@ cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int 
 cudaError_t launch_g2p2g(const View& V, const PhysFlags& pf, const Tuning& t, int num_sms, cudaStream_t st);
 cudaError_t launch_pack(const View& V, const float* x, const float* v, const float* C, const float* F,
                         const float* m, const float* V0, const int32_t* mat, const uint32_t* order,
-                        uint32_t* user_of_phys, uint32_t* phys_of_user, float2* mV_out, int32_t* mat_out,
-                        cudaStream_t st);
+                        const uint32_t* skeys, uint32_t* user_of_phys, uint32_t* phys_of_user, float2* mV_out,
+                        int32_t* mat_out, cudaStream_t st);
 // phys_of_user: upload index -> physical slot (written by launch_pack)
 cudaError_t launch_unpack(const View& V, const uint32_t* phys_of_user, float* x, float* v, float* C, float* F,
                           cudaStream_t st);

@@ -33,15 +33,14 @@ constexpr int TILE_NODES = TN * TN * TN;
 __device__ __forceinline__ const SceneDev& scene_ref(const View& V, int s) { return V.scenes[s]; }
 
 // ------------------------------------------------------------------ keys
+// Cell keys of the caller's positions, in upload order.
 template <int PHYS>
-__global__ void k_keys(View V) {
+__global__ void k_keys(View V, const float* __restrict__ pos) {
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     uint32_t flags = 0;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < V.N; p += stride) {
-        const int s = scene_of_particle(V, (int64_t)p);
-        const SceneDev& sc = scene_ref(V, s);
-        const float4 q0 = V.q[p];
-        const float x[3] = {q0.x, q0.y, q0.z};
+        const SceneDev& sc = scene_ref(V, scene_of_particle(V, p));
+        const float x[3] = {pos[3 * p], pos[3 * p + 1], pos[3 * p + 2]};
         int so[3];
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
@@ -77,28 +76,33 @@ __device__ __forceinline__ void tile_origin(const View& V, const SceneDev& sc, u
 }
 
 // --------------------------------------------------------------- payload
-// P2G payload of the current MLS state (after an upload, a material change,
-// or at the start of a replayed segment); G2P keeps it current afterwards.
+// P2G payload of one particle of the current MLS state.
+__device__ __forceinline__ void payload_of(const View& V, int64_t p, int mid, float2 mv, const float x[3],
+                                           const float F[9], const float v[3], const float C[9], uint32_t& flags) {
+    const int64_t N = V.N;
+    const SceneDev& sc = scene_ref(V, scene_of_particle(V, p));
+    Stencil st;
+    make_stencil<PHYS_MLS>(sc, x, st, flags);
+    float4 a0, a1, a2, a3;
+    mls_payload(sc, V.mats[mid], st.f, F, v, C, mv.x, mv.y, a0, a1, a2, a3);
+    V.pay[p] = a0;
+    V.pay[N + p] = a1;
+    V.pay[2 * N + p] = a2;
+    V.pay[3 * N + p] = a3;
+}
+
+// Payload of the whole state (after a material change, or at the start of a
+// replayed segment); the upload and G2P keep it current otherwise.
 template <bool MULTI>
 __global__ void k_payload(View V) {
     const int64_t N = V.N;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     uint32_t flags = 0;
     for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < N; p += stride) {
-        const int s = scene_of_particle(V, (int64_t)p);
-        const SceneDev& sc = scene_ref(V, s);
         float x[3], F[9], v[3], C[9];
         unpack_xF(V.q[p], V.q[N + p], V.q[2 * N + p], x, F);
         unpack_vC(V.q[3 * N + p], V.q[4 * N + p], V.q[5 * N + p], v, C);
-        Stencil st;
-        make_stencil<PHYS_MLS>(sc, x, st, flags);
-        const float2 mv = V.mV[p];
-        float4 a0, a1, a2, a3;
-        mls_payload(sc, V.mats[MULTI ? V.mat[p] : 0], st.f, F, v, C, mv.x, mv.y, a0, a1, a2, a3);
-        V.pay[p] = a0;
-        V.pay[N + p] = a1;
-        V.pay[2 * N + p] = a2;
-        V.pay[3 * N + p] = a3;
+        payload_of(V, p, MULTI ? V.mat[p] : 0, V.mV[p], x, F, v, C, flags);
     }
     if (flags) atomicOr(&V.counters[CNT_FLAGS], flags);
 }
@@ -2089,18 +2093,33 @@ __global__ void __launch_bounds__(G2_T, MINB) k_g2p2g(View V) {
 }
 
 // ------------------------------------------------------------ pack / unpack
-__global__ void k_pack(View V, const float* __restrict__ x, const float* __restrict__ v,
-                       const float* __restrict__ C, const float* __restrict__ F, const float* __restrict__ m,
-                       const float* __restrict__ V0, const int32_t* __restrict__ mat,
-                       const uint32_t* __restrict__ order, uint32_t* __restrict__ user_of_phys,
-                       uint32_t* __restrict__ phys_of_user, float2* __restrict__ mV_out,
-                       int32_t* __restrict__ mat_out) {
+// Packs the caller's particles into the state in sorted order (order: sorted
+// position -> upload index) with their keys, and forms the MLS payload where
+// the state is in registers.  Bound by the records' sectors, read in a random
+// order (10 sectors of 32 bytes for 112 bytes of a particle); loading the
+// records along their floats through shared memory, as k_unpack stores them,
+// was slower (304 against 280 us for 2 M particles: a gathered record's floats
+// come from L1 after its first one).  With the payload formed here and the
+// keys taken from the caller's positions, an upload makes one pass over the
+// particles where a first pack in upload order, a second one and a payload
+// kernel took 371 us (64 scenes, 3.9 M particles: 543 -> 361 us).
+template <bool PAY>
+__global__ void __launch_bounds__(PACK_T, 3) k_pack(View V, const float* __restrict__ x, const float* __restrict__ v,
+                                                    const float* __restrict__ C, const float* __restrict__ F,
+                                                    const float* __restrict__ m, const float* __restrict__ V0,
+                                                    const int32_t* __restrict__ mat,
+                                                    const uint32_t* __restrict__ order,
+                                                    const uint32_t* __restrict__ skeys,
+                                                    uint32_t* __restrict__ user_of_phys,
+                                                    uint32_t* __restrict__ phys_of_user, float2* __restrict__ mV_out,
+                                                    int32_t* __restrict__ mat_out) {
     const int64_t N = V.N;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    uint32_t flags = 0;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += stride) {
         const uint32_t u = order[i];
         if (u >= (uint32_t)N) {
-            atomicOr(&V.counters[CNT_FLAGS], FLAG_TILE_RANGE);
+            flags |= FLAG_TILE_RANGE;
             continue;
         }
         float xx[3], vv[3], CC[9], FF[9];
@@ -2114,6 +2133,7 @@ __global__ void k_pack(View V, const float* __restrict__ x, const float* __restr
             CC[a] = C ? C[9 * (int64_t)u + a] : 0.f;
             FF[a] = F ? F[9 * (int64_t)u + a] : ((a % 4 == 0) ? 1.f : 0.f);
         }
+        const float2 mv = make_float2(m[u], V0 ? V0[u] : 0.f);
         float4 o0, o1, o2, o3, o4, o5;
         pack_xF(xx, FF, o0, o1, o2);
         pack_vC(vv, CC, o3, o4, o5);
@@ -2123,43 +2143,31 @@ __global__ void k_pack(View V, const float* __restrict__ x, const float* __restr
         V.q[3 * N + i] = o3;
         V.q[4 * N + i] = o4;
         V.q[5 * N + i] = o5;
-        mV_out[i] = make_float2(m[u], V0 ? V0[u] : 0.f);
+        mV_out[i] = mv;
+        int32_t mid = 0;
         if (mat_out) {
-            int32_t mid = mat ? mat[u] : 0;
+            mid = mat ? mat[u] : 0;
             if (mid < 0 || mid >= V.M) {  // invalid material id: use 0 and report
-                atomicOr(&V.counters[CNT_FLAGS], FLAG_BAD_MATERIAL);
+                flags |= FLAG_BAD_MATERIAL;
                 mid = 0;
             }
             mat_out[i] = mid;
         }
         user_of_phys[i] = u;
         phys_of_user[u] = (uint32_t)i;
+        V.keys[i] = skeys[i];
+        if (PAY) payload_of(V, i, mid, mv, xx, FF, vv, CC, flags);
     }
+    if (flags) atomicOr(&V.counters[CNT_FLAGS], flags);
 }
 
 // Walks the upload order: the caller's records are written contiguously and
 // the state planes are gathered (scattered partial-sector writes cost more).
-__global__ void k_unpack(View V, const uint32_t* __restrict__ phys_of_user, float* __restrict__ x,
-                         float* __restrict__ v, float* __restrict__ C, float* __restrict__ F) {
-    const int64_t N = V.N;
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; u < N; u += stride) {
-        const int64_t i = phys_of_user[u];
-        if (i >= N) continue;
-        float xx[3], FF[9], vv[3], CC[9];
-        unpack_xF(V.q[i], V.q[N + i], V.q[2 * N + i], xx, FF);
-        unpack_vC(V.q[3 * N + i], V.q[4 * N + i], V.q[5 * N + i], vv, CC);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (x) x[3 * u + a] = xx[a];
-            if (v) v[3 * u + a] = vv[a];
-        }
-#pragma unroll
-        for (int a = 0; a < 9; ++a) {
-            if (C) C[9 * u + a] = CC[a];
-            if (F) F[9 * u + a] = FF[a];
-        }
-    }
+__global__ void __launch_bounds__(PACK_T) k_unpack(const float4* __restrict__ q, int64_t N,
+                                                   const uint32_t* __restrict__ phys_of_user, float* __restrict__ x,
+                                                   float* __restrict__ v, float* __restrict__ C,
+                                                   float* __restrict__ F) {
+    planes_to_records(q, N, phys_of_user, x, v, C, F);
 }
 
 __global__ void k_grid_download(View V, SceneDev sc, float* __restrict__ mass, float* __restrict__ vel) {
@@ -2214,12 +2222,12 @@ inline int grid_for(int64_t n, int block, int cap = 148 * 32) {
 
 }  // namespace
 
-cudaError_t launch_keys(const View& V, const PhysFlags& pf, cudaStream_t st) {
+cudaError_t launch_keys(const View& V, const float* x, const PhysFlags& pf, cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
     if (pf.physics == PHYS_MLS)
-        k_keys<PHYS_MLS><<<grid_for(V.N, 256), 256, 0, st>>>(V);
+        k_keys<PHYS_MLS><<<grid_for(V.N, 256), 256, 0, st>>>(V, x);
     else
-        k_keys<PHYS_REF><<<grid_for(V.N, 256), 256, 0, st>>>(V);
+        k_keys<PHYS_REF><<<grid_for(V.N, 256), 256, 0, st>>>(V, x);
     return cudaGetLastError();
 }
 
@@ -2474,18 +2482,23 @@ cudaError_t launch_g2p2g(const View& V, const PhysFlags& pf, const Tuning& t, in
 
 cudaError_t launch_pack(const View& V, const float* x, const float* v, const float* C, const float* F,
                         const float* m, const float* V0, const int32_t* mat, const uint32_t* order,
-                        uint32_t* user_of_phys, uint32_t* phys_of_user, float2* mV_out, int32_t* mat_out,
-                        cudaStream_t st) {
+                        const uint32_t* skeys, uint32_t* user_of_phys, uint32_t* phys_of_user, float2* mV_out,
+                        int32_t* mat_out, cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
-    k_pack<<<grid_for(V.N, 256), 256, 0, st>>>(V, x, v, C, F, m, V0, mat, order, user_of_phys, phys_of_user, mV_out,
-                                               mat_out);
+    const int nb = grid_for(V.N, PACK_T);
+    if (V.pay)
+        k_pack<true><<<nb, PACK_T, 0, st>>>(V, x, v, C, F, m, V0, mat, order, skeys, user_of_phys, phys_of_user,
+                                            mV_out, mat_out);
+    else
+        k_pack<false><<<nb, PACK_T, 0, st>>>(V, x, v, C, F, m, V0, mat, order, skeys, user_of_phys, phys_of_user,
+                                             mV_out, mat_out);
     return cudaGetLastError();
 }
 
 cudaError_t launch_unpack(const View& V, const uint32_t* phys_of_user, float* x, float* v, float* C, float* F,
                           cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
-    k_unpack<<<grid_for(V.N, 256), 256, 0, st>>>(V, phys_of_user, x, v, C, F);
+    k_unpack<<<grid_for(V.N, PACK_T), PACK_T, 0, st>>>(V.q, V.N, phys_of_user, x, v, C, F);
     return cudaGetLastError();
 }
 

@@ -119,3 +119,39 @@ def test_p2g_of_uneven_cells_equals_thread_per_cell(gpu, counts, sparse):
     bound = N * 2.0 ** -23
     assert np.abs(grids[0][0] - grids[1][0]).max() <= bound * grids[1][0].max()
     assert np.abs(grids[0][1] - grids[1][1]).max() <= 4 * bound * grids[1][0].max() + 1e-12
+
+
+@pytest.mark.parametrize("N", [1, 31, 32, 33, 255, 257, 1000])
+@pytest.mark.parametrize("device", [False, True])
+def test_upload_download_round_trip(gpu, N, device):
+    """The state comes back bit for bit in upload order, whatever is left out
+    on the way in (v, C zero, F identity) or asked for on the way out."""
+    import torch
+    rng = np.random.default_rng(N)
+    dx = 1.0 / 32
+    st = _scene_state(rng, N, (20, 24, 28), dx)
+    scene = gpu.Scene((20, 24, 28), dx, 1e-4)
+    sim = gpu.Simulator([scene], [N], [gpu.createElasticMaterial(1000.0, 1e4, 0.3)])
+    up = (lambda a: None if a is None else torch.tensor(a, device="cuda")) if device else (lambda a: a)
+
+    def down(names):
+        if not device:
+            return {k: a.reshape(N, -1) for k, a in sim.download().items() if k in names}
+        # records that are not 16-byte aligned, and words around them that must stay
+        bufs = {k: torch.full((N * w + 3,), 7.0, device="cuda") for k, w in (("x", 3), ("v", 3), ("C", 9), ("F", 9))}
+        out = {k: bufs[k][1:1 + N * (3 if k in "xv" else 9)] for k in names}
+        sim.download(out)
+        torch.cuda.synchronize()
+        for k in names:
+            assert bufs[k][0] == 7.0 and torch.all(bufs[k][-2:] == 7.0)
+        return {k: a.cpu().numpy().reshape(N, -1) for k, a in out.items()}
+
+    for given in (("x", "v", "C", "F"), ("x",), ("x", "F"), ("x", "v")):
+        sim.upload(*(up(st[k]) if k in given else None for k in ("x", "v", "C", "F")), up(st["m"]), up(st["V0"]))
+        want = {k: st[k] if k in given else np.zeros_like(st[k]) for k in ("x", "v", "C", "F")}
+        if "F" not in given:
+            want["F"] = np.tile(np.eye(3, dtype=np.float32).ravel(), (N, 1))
+        for names in (("x", "v", "C", "F"),) + ((("v",), ("F", "x"), ("C",)) if device else ()):
+            got = down(names)
+            for k in names:
+                assert np.array_equal(got[k], want[k].reshape(N, -1)), (given, names, k)
