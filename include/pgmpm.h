@@ -445,6 +445,21 @@ PGMPM_API void launch_mpm_timestep_backward(const float* grad_positions, const f
                                   float* grad_gravity, const float* saved_positions, const float* saved_velocities,
                                   int num_particles, int grid_resolution, float dt, void* stream);
 
+/* The two launchers for a caller that keeps the step's inputs itself: the
+ * forward writes new arrays (which may be the input ones), the backward takes
+ * that step's masses and gravity (may be NULL: the last forward's) instead of
+ * relying on the last forward call, and leaves them as the last call's.  A
+ * first forward call with the device, particle count and resolution must have
+ * been made. */
+PGMPM_API void pgmpm_mpm_timestep_forward(const float* positions, const float* velocities, const float* masses,
+                                float* positions_out, float* velocities_out, int num_particles, int grid_resolution,
+                                float dt, const float* gravity, void* stream);
+PGMPM_API void pgmpm_mpm_timestep_backward(const float* grad_positions, const float* grad_velocities,
+                                 float* grad_input_positions, float* grad_input_velocities, float* grad_masses,
+                                 float* grad_gravity, const float* saved_positions, const float* saved_velocities,
+                                 const float* masses, const float* gravity, int num_particles, int grid_resolution,
+                                 float dt, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -204,6 +204,10 @@ SIGNATURES = {
     "launch_mpm_timestep_forward": (None, [_vp, _vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_float, _vp, _vp]),
     "launch_mpm_timestep_backward": (None, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_int, ctypes.c_int,
                                             ctypes.c_float, _vp]),
+    "pgmpm_mpm_timestep_forward": (None, [_vp, _vp, _vp, _vp, _vp, ctypes.c_int, ctypes.c_int, ctypes.c_float, _vp,
+                                          _vp]),
+    "pgmpm_mpm_timestep_backward": (None, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, ctypes.c_int,
+                                           ctypes.c_int, ctypes.c_float, _vp]),
 }
 
 _lib = None

@@ -83,13 +83,18 @@ def simulate(sim: Simulator, x0, v0, E, m, V0, n_steps: int, checkpoint_every: i
 
 
 def _launch(name: str, *args):
-    """Calls a void launch_* entry point; raises if it reported an error."""
+    """Calls a void launch entry point; raises if it reported an error."""
     L = lib()
     L.pgmpm_clear_error()
     getattr(L, name)(*args)
     msg = L.pgmpm_last_error()
     if msg:
         raise PGMPMError(-1, msg.decode())
+
+
+def _f32(t):
+    t = t.detach()
+    return t if t.dtype == torch.float32 and t.is_contiguous() else t.to(torch.float32).contiguous()
 
 
 class MPMTimestep(torch.autograd.Function):
@@ -104,12 +109,11 @@ class MPMTimestep(torch.autograd.Function):
     def forward(ctx, positions, velocities, masses, gravity, grid_resolution: int, dt: float):
         if not positions.is_cuda:
             raise ValueError("MPMTimestep expects CUDA tensors")
-        f32 = lambda t: t.detach().to(torch.float32).contiguous()
-        x0, v0, m, g = f32(positions), f32(velocities), f32(masses), f32(gravity)
-        x, v = x0.clone(), v0.clone()
+        x0, v0, m, g = _f32(positions), _f32(velocities), _f32(masses), _f32(gravity)
+        x, v = torch.empty_like(x0), torch.empty_like(v0)
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        _launch("launch_mpm_timestep_forward", x.data_ptr(), v.data_ptr(), m.data_ptr(), x.shape[0],
-                int(grid_resolution), float(dt), g.data_ptr(), stream)
+        _launch("pgmpm_mpm_timestep_forward", x0.data_ptr(), v0.data_ptr(), m.data_ptr(), x.data_ptr(), v.data_ptr(),
+                x.shape[0], int(grid_resolution), float(dt), g.data_ptr(), stream)
         ctx.save_for_backward(x0, v0, m, g)
         ctx.res, ctx.dt = int(grid_resolution), float(dt)
         return x, v
@@ -118,16 +122,12 @@ class MPMTimestep(torch.autograd.Function):
     def backward(ctx, gx, gv):
         x0, v0, m, g = ctx.saved_tensors
         N = x0.shape[0]
-        z = lambda t: torch.zeros_like(x0) if t is None else t.detach().to(torch.float32).contiguous()
+        z = lambda t: torch.zeros_like(x0) if t is None else _f32(t)
         gx, gv = z(gx), z(gv)
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        # the backward launcher uses the masses and gravity of the last forward
-        # call with this particle count and resolution: make that this step's
-        xs, vs = x0.clone(), v0.clone()
-        _launch("launch_mpm_timestep_forward", xs.data_ptr(), vs.data_ptr(), m.data_ptr(), N, ctx.res, ctx.dt,
-                g.data_ptr(), stream)
         gix, giv = torch.empty_like(x0), torch.empty_like(v0)
         gim, gg = torch.empty_like(m), torch.zeros_like(g)
-        _launch("launch_mpm_timestep_backward", gx.data_ptr(), gv.data_ptr(), gix.data_ptr(), giv.data_ptr(),
-                gim.data_ptr(), gg.data_ptr(), x0.data_ptr(), v0.data_ptr(), N, ctx.res, ctx.dt, stream)
+        _launch("pgmpm_mpm_timestep_backward", gx.data_ptr(), gv.data_ptr(), gix.data_ptr(), giv.data_ptr(),
+                gim.data_ptr(), gg.data_ptr(), x0.data_ptr(), v0.data_ptr(), m.data_ptr(), g.data_ptr(), N, ctx.res,
+                ctx.dt, stream)
         return gix, giv, gim, gg, None, None

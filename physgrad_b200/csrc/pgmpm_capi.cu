@@ -176,15 +176,7 @@ int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, 
     }
     if (timed) CK(cudaEventRecord(s->ev[0], st));
     if (s->tune.step_sort == 0) {
-        BinSortBufs B;
-        B.keys_in = b.keys_in;
-        B.cnt = s->sort_counts();
-        B.out_k = b.which ? b.kb : b.ka;  // where the step's readers look (View::skeys / order)
-        B.out_v = b.which ? b.vb : b.va;
-        B.cell_range = b.cell_range;
-        B.ptile = b.ptile;
-        B.tile_info = s->tile_info.as<uint4>();
-        B.gsum = s->bs_gsum.as<uint32_t>();
+        const BinSortBufs B = s->bin_sort_bufs(b);
         if (b.sort_mode == 0) {
             CK(bin_sort_step(V, B, s->num_sms, counted, st));
         } else if (b.sort_mode == 2) {

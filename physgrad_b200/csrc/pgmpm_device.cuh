@@ -632,6 +632,42 @@ __device__ __forceinline__ void unpack_payload(const float4& p0, const float4& p
     f[2] = p3.w;
 }
 
+// ------------------------------------------------ node sums of a cell tile
+constexpr int TN = 6;              // edge of the node block a 4^3 cell tile touches (4 cells + 2)
+constexpr int TILE_NODES = TN * TN * TN;
+// Kernels with three threads per cell (thread 3 c + k: the nodes at z-offset k
+// of cell c's stencil): block size, and float4s per z-offset of the table that
+// the threads store their 9 nodes to (3 more than 9 per cell, so that a cell's
+// three threads store to different banks)
+constexpr int P2GS_T = 192;
+constexpr int P2GS_PLANE = 9 * 64 + 3;
+
+// Sum of the contributions to node (nx, ny, nz) of the 6^3 node block of a
+// 4^3 cell tile, from T4[z-offset][x-offset + 3 y-offset][cell].  Offsets
+// whose cell falls outside the tile are skipped: z-offsets by the whole warp
+// where it can (its lanes mostly share nz), the others by predicate.
+__device__ __forceinline__ float4 slices_node_sum(const float4* T4, int nx, int ny, int nz) {
+    const uint32_t vx = (nx <= 3 ? 1u : 0u) | (nx >= 1 && nx <= 4 ? 2u : 0u) | (nx >= 2 ? 4u : 0u);
+    const uint32_t vy = (ny <= 3 ? 1u : 0u) | (ny >= 1 && ny <= 4 ? 2u : 0u) | (ny >= 2 ? 4u : 0u);
+    const int cn = nx + 4 * ny + 16 * nz;
+    float2 a = f2(0.f), b = f2(0.f);
+#pragma unroll
+    for (int zz = 0; zz < 3; ++zz) {
+        if ((unsigned)(nz - zz) > 3u) continue;
+        const float4* plane = T4 + zz * (P2GS_PLANE - 16) + cn;
+#pragma unroll
+        for (int yy = 0; yy < 3; ++yy)
+#pragma unroll
+            for (int xx = 0; xx < 3; ++xx)
+                if ((vx >> xx) & (vy >> yy) & 1u) {
+                    const float4 t = plane[(xx + 3 * yy) * 64 - (xx + 4 * yy)];
+                    a = f2_add(a, make_float2(t.x, t.y));
+                    b = f2_add(b, make_float2(t.z, t.w));
+                }
+    }
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
 // ----------------------------------------------------------- grid update
 __device__ __forceinline__ bool in_wall(const SceneDev& sc, int a, int idx, int& side) {
     if (idx < sc.bthick) { side = -1; return true; }

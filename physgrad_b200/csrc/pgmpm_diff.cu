@@ -581,6 +581,26 @@ struct LaunchEntry {
 std::mutex g_launch_mu;
 std::map<std::tuple<int, int, int>, LaunchEntry> g_launch_solvers;
 
+// Node arrays of the reverse, the accumulator cleared once (every call leaves
+// it zero).
+bool launch_adj_grids(pgmpm_solver s, cudaStream_t st) {
+    const size_t bytes = sizeof(float4) * nodes_of(s);
+    if (s->adj_grid_gv.bytes < bytes &&
+        (s->adj_grid_gv.alloc(bytes) != cudaSuccess || cudaMemsetAsync(s->adj_grid_gv.p, 0, bytes, st) != cudaSuccess ||
+         cudaStreamSynchronize(st) != cudaSuccess))
+        return false;
+    return s->adj_grid_gpm.ensure(bytes) == cudaSuccess;
+}
+
+// One step on the caller's arrays (launch_ref_step).
+void launch_ref(pgmpm_solver s, const RefStep& R, cudaStream_t st, const char* who) {
+    const StepBufs b = s->live_bufs();
+    if (launch_ref_step(s->view_for(b), s->bin_sort_bufs(b), R, s->pf, s->tune, s->num_sms, st) != cudaSuccess)
+        fail(PGMPM_ERR_CUDA, "%s: %s", who, cudaGetErrorString(cudaGetLastError()));
+    else if (!R.gx)
+        s->met.total_steps++;
+}
+
 // per-call dt into the scene table (the dt word only: gravity arrives as a
 // device pointer and is copied there by the forward)
 bool launch_set_dt(pgmpm_solver s, float dt, cudaStream_t st, const char* who) {
@@ -596,11 +616,13 @@ bool launch_set_dt(pgmpm_solver s, float dt, cudaStream_t st, const char* who) {
 }
 }  // namespace
 
-extern "C" void launch_mpm_timestep_forward(float* positions, float* velocities, const float* masses,
-                                            int num_particles, int grid_resolution, float dt, const float* gravity,
-                                            void* stream) {
-    if (num_particles < 0 || grid_resolution < 4 || !(dt > 0.f) || (num_particles > 0 && (!positions || !velocities || !masses))) {
-        fail(PGMPM_ERR_ARG, "launch_mpm_timestep_forward: invalid arguments");
+namespace {
+void timestep_forward(const char* who, const float* positions, const float* velocities, const float* masses,
+                      float* positions_out, float* velocities_out, int num_particles, int grid_resolution, float dt,
+                      const float* gravity, void* stream) {
+    if (num_particles < 0 || grid_resolution < 4 || !(dt > 0.f) ||
+        (num_particles > 0 && (!positions || !velocities || !masses || !positions_out || !velocities_out))) {
+        fail(PGMPM_ERR_ARG, "%s: invalid arguments", who);
         return;
     }
     if (num_particles == 0) return;
@@ -630,25 +652,54 @@ extern "C" void launch_mpm_timestep_forward(float* positions, float* velocities,
             s = entry->s;
         }
     }
-    // per-call dt and gravity (device pointer) into the scene table
-    if (!launch_set_dt(s, dt, st, "launch_mpm_timestep_forward")) return;
+    if (!launch_set_dt(s, dt, st, who)) return;
+    // the masses (and the gravity, in the scene table) are kept for
+    // launch_mpm_timestep_backward
+    if (entry->masses.ensure(sizeof(float) * (size_t)num_particles) != cudaSuccess) {
+        fail(PGMPM_ERR_CUDA, "%s: keeping the masses failed", who);
+        return;
+    }
+    if (s->tune.step_sort == 0) {  // on the caller's arrays
+        RefStep R{};
+        R.x = positions;
+        R.v = velocities;
+        R.xo = positions_out;
+        R.vo = velocities_out;
+        R.m = masses;
+        R.gravity = gravity;
+        R.keep_m = entry->masses.as<float>();
+        launch_ref(s, R, st, who);
+        return;
+    }
     if (gravity) {
         if (cudaMemcpyAsync(&s->d_scenes.as<SceneDev>()[0].gravity[0], gravity, 3 * sizeof(float),
                             cudaMemcpyDeviceToDevice, st) != cudaSuccess) {
-            fail(PGMPM_ERR_CUDA, "launch_mpm_timestep_forward: gravity copy failed");
+            fail(PGMPM_ERR_CUDA, "%s: gravity copy failed", who);
             return;
         }
     }
-    std::vector<float> ones;  // volumes are not used by the REF_COMPAT physics
     if (pgmpm_upload(s, positions, velocities, nullptr, nullptr, masses, nullptr, nullptr, PGMPM_PTR_DEVICE, stream))
         return;
     if (pgmpm_step(s, 1, stream)) return;
-    if (pgmpm_download(s, positions, velocities, nullptr, nullptr, PGMPM_PTR_DEVICE, stream)) return;
-    // kept for launch_mpm_timestep_backward
-    if (entry->masses.ensure(sizeof(float) * (size_t)num_particles) != cudaSuccess ||
-        cudaMemcpyAsync(entry->masses.p, masses, sizeof(float) * (size_t)num_particles, cudaMemcpyDeviceToDevice,
+    if (pgmpm_download(s, positions_out, velocities_out, nullptr, nullptr, PGMPM_PTR_DEVICE, stream)) return;
+    if (cudaMemcpyAsync(entry->masses.p, masses, sizeof(float) * (size_t)num_particles, cudaMemcpyDeviceToDevice,
                         st) != cudaSuccess)
-        fail(PGMPM_ERR_CUDA, "launch_mpm_timestep_forward: keeping the masses failed");
+        fail(PGMPM_ERR_CUDA, "%s: keeping the masses failed", who);
+}
+}  // namespace
+
+extern "C" void launch_mpm_timestep_forward(float* positions, float* velocities, const float* masses,
+                                            int num_particles, int grid_resolution, float dt, const float* gravity,
+                                            void* stream) {
+    timestep_forward("launch_mpm_timestep_forward", positions, velocities, masses, positions, velocities,
+                     num_particles, grid_resolution, dt, gravity, stream);
+}
+
+extern "C" void pgmpm_mpm_timestep_forward(const float* positions, const float* velocities, const float* masses,
+                                           float* positions_out, float* velocities_out, int num_particles,
+                                           int grid_resolution, float dt, const float* gravity, void* stream) {
+    timestep_forward("pgmpm_mpm_timestep_forward", positions, velocities, masses, positions_out, velocities_out,
+                     num_particles, grid_resolution, dt, gravity, stream);
 }
 
 // launch_mpm_timestep_backward: src/pytorch_autograd.cu:384-402 shape.  The
@@ -659,15 +710,18 @@ extern "C" void launch_mpm_timestep_forward(float* positions, float* velocities,
 // the three reverse kernels of pgmpm_ref_adjoint.cu run.  grad_gravity is
 // added to, as the reference's kernel does (zero it first); grad_masses may
 // be NULL.
-extern "C" void launch_mpm_timestep_backward(const float* grad_positions, const float* grad_velocities,
-                                             float* grad_input_positions, float* grad_input_velocities,
-                                             float* grad_masses, float* grad_gravity, const float* saved_positions,
-                                             const float* saved_velocities, int num_particles, int grid_resolution,
-                                             float dt, void* stream) {
+namespace {
+// masses null: those (and the gravity) of the last forward call with this
+// device, particle count and resolution; else masses and gravity replace them.
+void timestep_backward(const char* who, const float* grad_positions, const float* grad_velocities,
+                       float* grad_input_positions, float* grad_input_velocities, float* grad_masses,
+                       float* grad_gravity, const float* saved_positions, const float* saved_velocities,
+                       const float* masses, const float* gravity, int num_particles, int grid_resolution, float dt,
+                       void* stream) {
     if (num_particles < 0 || grid_resolution < 4 || !(dt > 0.f) ||
         (num_particles > 0 && (!grad_positions || !grad_velocities || !grad_input_positions ||
                                !grad_input_velocities || !saved_positions || !saved_velocities))) {
-        fail(PGMPM_ERR_ARG, "launch_mpm_timestep_backward: invalid arguments");
+        fail(PGMPM_ERR_ARG, "%s: invalid arguments", who);
         return;
     }
     if (num_particles == 0) return;
@@ -675,31 +729,84 @@ extern "C" void launch_mpm_timestep_backward(const float* grad_positions, const 
     cudaGetDevice(&dev);
     cudaStream_t st = ST(stream);
     pgmpm_solver s = nullptr;
-    const float* masses = nullptr;
+    float* kept = nullptr;
     {
         std::lock_guard<std::mutex> lk(g_launch_mu);
         auto it = g_launch_solvers.find(std::make_tuple(dev, num_particles, grid_resolution));
         if (it == g_launch_solvers.end() || !it->second.masses.p) {
             fail(PGMPM_ERR_STATE,
-                 "launch_mpm_timestep_backward: no launch_mpm_timestep_forward call with this device, particle "
-                 "count and resolution");
+                 "%s: no launch_mpm_timestep_forward call with this device, particle count and resolution", who);
             return;
         }
         s = it->second.s;
-        masses = it->second.masses.as<float>();
+        kept = it->second.masses.as<float>();
     }
-    if (!launch_set_dt(s, dt, st, "launch_mpm_timestep_backward")) return;
-    if (pgmpm_upload(s, saved_positions, saved_velocities, nullptr, nullptr, masses, nullptr, nullptr,
-                     PGMPM_PTR_DEVICE, stream))
+    if (!launch_set_dt(s, dt, st, who)) return;
+    if (s->tune.step_sort == 0) {  // on the caller's arrays
+        if (!launch_adj_grids(s, st)) {
+            fail(PGMPM_ERR_CUDA, "%s: grid adjoint buffer", who);
+            return;
+        }
+        RefStep R{};
+        R.x = saved_positions;
+        R.v = saved_velocities;
+        R.m = masses ? masses : kept;
+        R.gravity = gravity;
+        R.keep_m = kept;
+        R.gx = grad_positions;
+        R.gv = grad_velocities;
+        R.gx_in = grad_input_positions;
+        R.gv_in = grad_input_velocities;
+        R.gm_in = grad_masses;
+        R.ggrav = grad_gravity;
+        R.acc = s->adj_grid_gv.as<float4>();
+        R.gpm = s->adj_grid_gpm.as<float4>();
+        launch_ref(s, R, st, who);
+        return;
+    }
+    if ((masses && cudaMemcpyAsync(kept, masses, sizeof(float) * (size_t)num_particles, cudaMemcpyDeviceToDevice,
+                                   st) != cudaSuccess) ||
+        (gravity && cudaMemcpyAsync(&s->d_scenes.as<SceneDev>()[0].gravity[0], gravity, 3 * sizeof(float),
+                                    cudaMemcpyDeviceToDevice, st) != cudaSuccess)) {
+        fail(PGMPM_ERR_CUDA, "%s: mass or gravity copy failed", who);
+        return;
+    }
+    if (pgmpm_upload(s, saved_positions, saved_velocities, nullptr, nullptr, kept, nullptr, nullptr, PGMPM_PTR_DEVICE,
+                     stream))
         return;
     if (pgmpm_step(s, 1, stream)) return;
     const size_t gbytes = sizeof(float4) * nodes_of(s);
     if (s->adj_grid_gv.ensure(gbytes) != cudaSuccess || cudaMemsetAsync(s->adj_grid_gv.p, 0, gbytes, st) != cudaSuccess) {
-        fail(PGMPM_ERR_CUDA, "launch_mpm_timestep_backward: grid adjoint buffer");
+        fail(PGMPM_ERR_CUDA, "%s: grid adjoint buffer", who);
         return;
     }
-    if (launch_ref_adjoint(s->view(), saved_positions, saved_velocities, masses, grad_positions, grad_velocities,
+    if (launch_ref_adjoint(s->view(), saved_positions, saved_velocities, kept, grad_positions, grad_velocities,
                            s->adj_grid_gv.as<float4>(), grad_input_positions, grad_input_velocities, grad_masses,
                            grad_gravity, s->num_sms, st) != cudaSuccess)
-        fail(PGMPM_ERR_CUDA, "launch_mpm_timestep_backward: %s", cudaGetErrorString(cudaGetLastError()));
+        fail(PGMPM_ERR_CUDA, "%s: %s", who, cudaGetErrorString(cudaGetLastError()));
+}
+}  // namespace
+
+extern "C" void launch_mpm_timestep_backward(const float* grad_positions, const float* grad_velocities,
+                                             float* grad_input_positions, float* grad_input_velocities,
+                                             float* grad_masses, float* grad_gravity, const float* saved_positions,
+                                             const float* saved_velocities, int num_particles, int grid_resolution,
+                                             float dt, void* stream) {
+    timestep_backward("launch_mpm_timestep_backward", grad_positions, grad_velocities, grad_input_positions,
+                      grad_input_velocities, grad_masses, grad_gravity, saved_positions, saved_velocities, nullptr,
+                      nullptr, num_particles, grid_resolution, dt, stream);
+}
+
+extern "C" void pgmpm_mpm_timestep_backward(const float* grad_positions, const float* grad_velocities,
+                                            float* grad_input_positions, float* grad_input_velocities,
+                                            float* grad_masses, float* grad_gravity, const float* saved_positions,
+                                            const float* saved_velocities, const float* masses, const float* gravity,
+                                            int num_particles, int grid_resolution, float dt, void* stream) {
+    if (num_particles > 0 && !masses) {
+        fail(PGMPM_ERR_ARG, "pgmpm_mpm_timestep_backward: invalid arguments");
+        return;
+    }
+    timestep_backward("pgmpm_mpm_timestep_backward", grad_positions, grad_velocities, grad_input_positions,
+                      grad_input_velocities, grad_masses, grad_gravity, saved_positions, saved_velocities, masses,
+                      gravity, num_particles, grid_resolution, dt, stream);
 }

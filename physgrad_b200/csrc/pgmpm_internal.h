@@ -212,6 +212,20 @@ cudaError_t radix_sort_pairs(const uint32_t* kin, const uint32_t* vin, uint32_t*
                              uint32_t* vb, uint32_t* scratch, int64_t n, int key_bits, int* which,
                              cudaStream_t st);
 
+// One REF_COMPAT step on the caller's arrays (bin sort): the forward (gx null:
+// new positions and velocities to xo, vo, which may be x and v) or the reverse
+// of the step from x, v, m (gx_in, gv_in, gm_in (may be null), ggrav added to).
+struct RefStep {
+    const float *x, *v, *m;  // [N][3], [N][3], [N]
+    const float* gravity;    // device [3], copied into the scene; null: the scene's
+    float* keep_m;           // copy of m (or m itself)
+    float *xo, *vo;
+    const float *gx, *gv;
+    float *gx_in, *gv_in, *gm_in, *ggrav;
+    float4* acc;             // per node, zero between calls
+    float4* gpm;             // per node
+};
+
 // Per-step bin sort (pgmpm_sort.cu): keys_in (physical order) -> out_k /
 // out_v sorted by key, plus the occupied cell tiles with their ranges
 // (largest first), every cell's [begin, end) in the sorted order of the
@@ -229,7 +243,9 @@ struct BinSortBufs {
     uint32_t* gsum;        // bin_sort_groups(total_ct) words (scratch)
 };
 int64_t bin_sort_groups(int64_t total_ct);
-cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool counted, cudaStream_t st);
+// rec: write the particles' records to the state planes instead of out_k, out_v
+cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool counted, cudaStream_t st,
+                          const RefStep* rec = nullptr);
 
 // pgmpm_kernels.cu
 struct PhysFlags {
@@ -287,6 +303,8 @@ cudaError_t launch_state_to_planes(const float* x, const float* v, const float* 
 cudaError_t launch_ref_adjoint(const View& V, const float* x, const float* v, const float* m, const float* gx,
                                const float* gv, float4* G, float* gx_in, float* gv_in, float* gm_in, float* ggrav,
                                int num_sms, cudaStream_t st);
+cudaError_t launch_ref_step(const View& V, const BinSortBufs& B, const RefStep& R, const PhysFlags& pf,
+                            const Tuning& t, int num_sms, cudaStream_t st);
 cudaError_t launch_planes_to_state(const float4* g, const uint32_t* phys_of_user, float* x, float* v, float* C,
                                    float* F, int64_t N, cudaStream_t st);
 

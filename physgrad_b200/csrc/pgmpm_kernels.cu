@@ -27,8 +27,6 @@ namespace pgmpm {
 
 namespace {
 
-constexpr int TN = 6;              // smem tile edge in nodes (4 cells + 2)
-constexpr int TILE_NODES = TN * TN * TN;
 
 __device__ __forceinline__ const SceneDev& scene_ref(const View& V, int s) { return V.scenes[s]; }
 
@@ -971,35 +969,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // count (102: the ranking's barriers, and neighbouring lanes no longer share
 // sectors), the next payload prefetched into registers (115), the sums on
 // packed FP32 pairs (91.6: the doubled weights cost moves).
-constexpr int P2GS_T = 192;
-constexpr int P2GS_BLOCKS = 4;          // resident blocks per SM
-constexpr int P2GS_PLANE = 9 * 64 + 3;  // float4s per z-offset of the flush table (3 more: see the stores)
-
-// Sum of the contributions to node (nx, ny, nz) of the 6^3 node block of a
-// 4^3 cell tile, from T4[z-offset][x-offset + 3 y-offset][cell].  Offsets
-// whose cell falls outside the tile are skipped: z-offsets by the whole warp
-// where it can (its lanes mostly share nz), the others by predicate.
-__device__ __forceinline__ float4 slices_node_sum(const float4* T4, int nx, int ny, int nz) {
-    const uint32_t vx = (nx <= 3 ? 1u : 0u) | (nx >= 1 && nx <= 4 ? 2u : 0u) | (nx >= 2 ? 4u : 0u);
-    const uint32_t vy = (ny <= 3 ? 1u : 0u) | (ny >= 1 && ny <= 4 ? 2u : 0u) | (ny >= 2 ? 4u : 0u);
-    const int cn = nx + 4 * ny + 16 * nz;
-    float2 a = f2(0.f), b = f2(0.f);
-#pragma unroll
-    for (int zz = 0; zz < 3; ++zz) {
-        if ((unsigned)(nz - zz) > 3u) continue;
-        const float4* plane = T4 + zz * (P2GS_PLANE - 16) + cn;
-#pragma unroll
-        for (int yy = 0; yy < 3; ++yy)
-#pragma unroll
-            for (int xx = 0; xx < 3; ++xx)
-                if ((vx >> xx) & (vy >> yy) & 1u) {
-                    const float4 t = plane[(xx + 3 * yy) * 64 - (xx + 4 * yy)];
-                    a = f2_add(a, make_float2(t.x, t.y));
-                    b = f2_add(b, make_float2(t.z, t.w));
-                }
-    }
-    return make_float4(a.x, a.y, b.x, b.y);
-}
+constexpr int P2GS_BLOCKS = 4;  // resident blocks per SM
 
 template <bool SPARSE>
 __global__ void __launch_bounds__(P2GS_T, P2GS_BLOCKS) k_p2g_slices(View V) {

@@ -292,6 +292,19 @@ struct pgmpm_solver_s {
         return c;
     }
 
+    pgmpm::BinSortBufs bin_sort_bufs(const pgmpm::StepBufs& b) const {
+        pgmpm::BinSortBufs B;
+        B.keys_in = b.keys_in;
+        B.cnt = sort_counts();
+        B.out_k = b.which ? b.kb : b.ka;  // where the step's readers look (View::skeys / order)
+        B.out_v = b.which ? b.vb : b.va;
+        B.cell_range = b.cell_range;
+        B.ptile = b.ptile;
+        B.tile_info = tile_info.as<uint4>();
+        B.gsum = bs_gsum.as<uint32_t>();
+        return B;
+    }
+
     // split steps whose G2P counts its new keys for the sort of the step
     // that follows in the same call.  Up to this many particles it saves more
     // than it costs; with more, whose state outgrows L2, its atomics hold the

@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint32_t* __restr
 constexpr int BS_T = 256;
 constexpr int BS_ITEMS = 8;                 // keys per thread in bs_count / bs_scatter
 constexpr int BS_TILE = BS_T * BS_ITEMS;    // keys per block
+constexpr int BS_REC_ITEMS = 1;             // particles per thread of bs_scatter when it moves their records
 // cell tiles per warp of bs_tiles: a warp takes its occupied tiles in turn
 // (~1 us each: a sparse grid's claims are chains of L2 reads), so few per warp
 // are better until the blocks' reads of the counts before them (tiles^2 / 2
@@ -471,12 +472,16 @@ __global__ void __launch_bounds__(BS_T) bs_tiles(View V, SortCounts c, const uin
 }
 
 // Blocks [0, tile_blocks): the work list and the counters, the rest: the
-// particles.
+// particles, whose sorted keys and indices go to ok_ and ov -- or (REC), from
+// the caller's arrays of R, as records to the state planes: (u - s - 1, m)
+// with u the grid coordinates and s the cell's lowest node, (v, index) and for
+// the reverse (gv + dt gx, 0).
+template <bool REC>
 __global__ void __launch_bounds__(BS_T) bs_scatter(View V, const uint32_t* __restrict__ keys, SortCounts c,
                                                    const uint2* __restrict__ cell_range,
                                                    const uint4* __restrict__ tile_info, uint4* __restrict__ ptile,
                                                    uint32_t* __restrict__ ok_, uint32_t* __restrict__ ov,
-                                                   int tile_blocks) {
+                                                   int tile_blocks, RefStep R) {
     const int64_t n = V.N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if ((int)blockIdx.x < tile_blocks) {
@@ -503,23 +508,43 @@ __global__ void __launch_bounds__(BS_T) bs_scatter(View V, const uint32_t* __res
         }
         return;
     }
-    const int64_t base = (int64_t)(blockIdx.x - tile_blocks) * BS_TILE + warp * (32 * BS_ITEMS);
-    uint32_t k[BS_ITEMS], sl[BS_ITEMS], pos[BS_ITEMS];
+    constexpr int ITEMS = REC ? BS_REC_ITEMS : BS_ITEMS;
+    const int64_t base = (int64_t)(blockIdx.x - tile_blocks) * (BS_T * ITEMS) + warp * (32 * ITEMS);
+    uint32_t k[ITEMS], sl[ITEMS], pos[ITEMS];
 #pragma unroll
-    for (int r = 0; r < BS_ITEMS; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const int64_t i = base + r * 32 + lane;
         k[r] = i < n ? keys[i] : 0u;
         sl[r] = i < n ? c.slot[i] : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < BS_ITEMS; ++r)
+    for (int r = 0; r < ITEMS; ++r)
         pos[r] = (k[r] < c.ncells ? cell_range[k[r]].x : V.sort_work[SW_VALID]) + sl[r];
 #pragma unroll
-    for (int r = 0; r < BS_ITEMS; ++r) {
+    for (int r = 0; r < ITEMS; ++r) {
         const int64_t i = base + r * 32 + lane;
         if (i < n && (int64_t)pos[r] < n) {
-            ok_[pos[r]] = k[r];
-            ov[pos[r]] = (uint32_t)i;
+            if (REC) {
+                const SceneDev& sc = V.scenes[0];
+                float g[3];
+                uint32_t f = 0;
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    float u;
+                    const int s = stencil_origin(R.x[3 * i + a], sc.origin[a], sc.dx, sc.inv_dx, sc.n[a], PHYS_REF, u, f);
+                    g[a] = __fsub_rn(u, (float)(s + 1));
+                }
+                V.q[pos[r]] = make_float4(g[0], g[1], g[2], R.m[i]);
+                V.q[n + pos[r]] = make_float4(R.v[3 * i], R.v[3 * i + 1], R.v[3 * i + 2], __uint_as_float((uint32_t)i));
+                if (R.gx) {
+                    const float dt = sc.dt;
+                    V.q[2 * n + pos[r]] = make_float4(R.gv[3 * i] + dt * R.gx[3 * i], R.gv[3 * i + 1] + dt * R.gx[3 * i + 1],
+                                                      R.gv[3 * i + 2] + dt * R.gx[3 * i + 2], 0.f);
+                }
+            } else {
+                ok_[pos[r]] = k[r];
+                ov[pos[r]] = (uint32_t)i;
+            }
         }
     }
 }
@@ -527,7 +552,8 @@ __global__ void __launch_bounds__(BS_T) bs_scatter(View V, const uint32_t* __res
 
 int64_t bin_sort_groups(int64_t total_ct) { return (total_ct + BS_GROUP) / BS_GROUP; }
 
-cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool counted, cudaStream_t st) {
+cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool counted, cudaStream_t st,
+                          const RefStep* rec) {
     const int64_t n = V.N;
     if (n <= 0) return cudaSuccess;
     if (!B.cell_range || !B.ptile || !V.sort_work) return cudaErrorInvalidValue;
@@ -547,8 +573,12 @@ cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool
         bs_tiles<BT_MANY><<<cell_blocks + node_blocks, BS_T, 0, st>>>(V, B.cnt, gsum, B.cell_range, B.tile_info,
                                                                      cell_blocks);
     const int tile_blocks = (int)std::min<int64_t>(num_sms, (nct + BS_T - 1) / BS_T);
-    bs_scatter<<<tile_blocks + gk, BS_T, 0, st>>>(V, B.keys_in, B.cnt, B.cell_range, B.tile_info, B.ptile, B.out_k,
-                                                 B.out_v, tile_blocks);
+    if (rec)
+        bs_scatter<true><<<tile_blocks + (int)((n + BS_T * BS_REC_ITEMS - 1) / (BS_T * BS_REC_ITEMS)), BS_T, 0, st>>>(V, B.keys_in, B.cnt, B.cell_range, B.tile_info, B.ptile,
+                                                           nullptr, nullptr, tile_blocks, *rec);
+    else
+        bs_scatter<false><<<tile_blocks + gk, BS_T, 0, st>>>(V, B.keys_in, B.cnt, B.cell_range, B.tile_info, B.ptile,
+                                                            B.out_k, B.out_v, tile_blocks, RefStep{});
     return cudaGetLastError();
 }
 

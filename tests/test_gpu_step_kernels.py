@@ -155,3 +155,35 @@ def test_upload_download_round_trip(gpu, N, device):
             got = down(names)
             for k in names:
                 assert np.array_equal(got[k], want[k].reshape(N, -1)), (given, names, k)
+
+
+@pytest.mark.parametrize("n_near", [1, 40, 193, 700])
+def test_pic_step_routes_agree(gpu, n_near):
+    """launch_mpm_timestep_* sort by bins from ~8 cells per particle on and by
+    radix below.  The same particles (partly on and outside the grid's faces)
+    with few and with many others far away take the two routes; results and
+    gradients agree to FP32 rounding: 1e-6 of the largest value of a field,
+    times 8 for the terms of a node's sums (<= 700 / 27 per cell on average)."""
+    import torch
+    from physgrad_b200 import autograd
+    rng = np.random.default_rng(n_near)
+    res, dx = 108, 1.0 / 108
+    near = rng.uniform(0.0, 9.0, (n_near, 3)) * dx
+    near[: n_near // 8 + 1] = rng.uniform(-3.0, 1.0, (n_near // 8 + 1, 3)) * dx  # outside and at the lowest nodes
+    outs = []
+    for n_far in (50, 40000):  # 27^3 tiles: radix up to ~26 K particles
+        far = 0.4 + rng.uniform(0.0, 0.5, (n_far, 3))
+        x = np.concatenate([near, far]).astype(np.float32)
+        r2 = np.random.default_rng(7)
+        vals = r2.normal(0, 1, (n_near, 10)).astype(np.float32)
+        pad = lambda a, w: np.concatenate([a.reshape(n_near, w), np.ones((n_far, w), np.float32)])
+        t = lambda a: torch.tensor(a, device="cuda")
+        xs, vs = t(x).requires_grad_(True), t(pad(vals[:, :3], 3)).requires_grad_(True)
+        m = t(pad(0.5 + np.abs(vals[:, 3]), 1)[:, 0].copy()).requires_grad_(True)
+        g = torch.tensor([0.1, -9.8, 0.3], device="cuda", requires_grad=True)
+        xo, vo = autograd.MPMTimestep.apply(xs, vs, m, g, res, 1e-3)
+        grads = torch.autograd.grad([xo, vo], [xs, vs, m], [t(pad(vals[:, 4:7], 3)), t(pad(vals[:, 7:10], 3))])
+        outs.append([a.detach()[:n_near].cpu().numpy() for a in (xo, vo, *grads)])
+    for a, b in zip(*outs):
+        assert np.isfinite(b).all()
+        assert np.abs(a - b).max() <= 8e-6 * np.abs(b).max() + 1e-9
