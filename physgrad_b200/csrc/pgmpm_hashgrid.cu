@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "pgmpm_hashgrid.cuh"
 #include "pgmpm_solver_impl.h"
 
 using namespace pgmpm;
@@ -44,41 +45,21 @@ struct pgmpm_hashgrid_s {
     DevBuf cell_ids;                // per particle: cell id (particle order)
     DevBuf ka, va, kb, vb, scratch, pos_stage;  // sort buffers; va keeps the sorted particle indices
     DevBuf qcount, qstage, qout_stage, scan_tmp, stats;  // query scratch, kept between calls
+    // dense queries (cells in grid order, x outer, z inner): z stretches and
+    // block sums for the last half width and first[] of the cells' buckets (one
+    // allocation), and the buckets themselves
+    DevBuf grid_tables, grid_index;
+    uint2* grid_rows() const { return grid_tables.as<uint2>(); }
+    uint32_t* grid_sum() const { return reinterpret_cast<uint32_t*>(grid_rows() + total); }
+    uint32_t* grid_first() const { return grid_sum() + total; }
+    uint32_t mult_max = 0;    // most cells that hash to one bucket (0: not counted yet)
+    bool grid_ready = false;  // grid_first and grid_index hold the last build's
+    int64_t sum_src = -1;     // grid_rows and grid_sum hold the last build's for this half width
 };
 
 namespace {
 
 constexpr int HG_T = 256;
-
-struct HGDev {
-    float cell, dmin[3];
-    uint32_t res[3], total;
-    unsigned long long total_m;  // 2^64 / total + 1 (mod 2^64), for hg_mod
-};
-
-// a % total by direct computation of the remainder (Lemire, Kaser and Kurz,
-// "Faster remainder by direct computation", 2019): for 32-bit a and d and
-// M = floor(2^64 / d) + 1, a mod d = floor(((M a) mod 2^64) d / 2^64).
-__device__ __forceinline__ uint32_t hg_mod(uint32_t a, const HGDev& G) {
-    return (uint32_t)__umul64hi(G.total_m * (unsigned long long)a, (unsigned long long)G.total);
-}
-
-// src/sparse_data_structures.h:121-128: bit interleave in uint32 arithmetic
-__device__ __forceinline__ uint32_t hg_expand(uint32_t v) {
-    v = (v * 0x00010001u) & 0xFF0000FFu;
-    v = (v * 0x00000101u) & 0x0F00F00Fu;
-    v = (v * 0x00000011u) & 0xC30C30C3u;
-    v = (v * 0x00000005u) & 0x49249249u;
-    return v;
-}
-__device__ __forceinline__ uint32_t hg_morton(uint32_t x, uint32_t y, uint32_t z) {
-    return hg_expand(x) | (hg_expand(y) << 1) | (hg_expand(z) << 2);
-}
-// (x - min) / cell in IEEE single, truncated toward zero to a 64-bit integer
-// and reduced mod 2^32: the host's float -> uint32 conversion
-__device__ __forceinline__ uint32_t hg_coord(float x, float mn, float cell) {
-    return (uint32_t)(unsigned long long)__float2ll_rz(__fdiv_rn(__fsub_rn(x, mn), cell));
-}
 
 // cell id per particle, and the per-cell counts (one atomic per particle:
 // input order is arbitrary, so a warp's particles rarely share a cell and
@@ -100,27 +81,6 @@ __global__ void k_hg_cells(HGDev G, const float* __restrict__ pos, int64_t n, ui
 // a time, give each cell its place by a scan over the lanes and copy the
 // cell's particles, so a query's list is written into one contiguous stretch
 // by its lanes together.
-// (dx, dy, dz) of cell t of the block, packed 10 bits each, for the block's
-// cells in shared memory when there are at most HG_TAB of them
-constexpr int HG_TAB = 1024;
-__device__ __forceinline__ uint32_t hg_offsets(uint32_t t, uint32_t w) {
-    return (t % w) << 20 | ((t / w) % w) << 10 | (t / (w * w));
-}
-__device__ __forceinline__ void hg_fill_table(uint32_t* tab, uint32_t ncell, uint32_t w) {
-    if (ncell <= (uint32_t)HG_TAB)
-        for (uint32_t t = threadIdx.x; t < ncell; t += blockDim.x) tab[t] = hg_offsets(t, w);
-    __syncthreads();
-}
-__device__ __forceinline__ bool hg_cell_of(const HGDev& G, const uint32_t c[3], uint32_t src, uint32_t w,
-                                           uint32_t ncell, const uint32_t* tab, uint32_t t, uint32_t& id) {
-    const uint32_t o = ncell <= (uint32_t)HG_TAB ? tab[t] : hg_offsets(t, w);
-    const uint32_t dx = o & 1023u, dy = (o >> 10) & 1023u, dz = o >> 20;
-    const uint32_t gx = c[0] + dx - src, gy = c[1] + dy - src, gz = c[2] + dz - src;  // wrap: below 0 fails
-    if (gx >= G.res[0] || gy >= G.res[1] || gz >= G.res[2]) return false;
-    id = hg_mod(hg_morton(gx, gy, gz), G);
-    return true;
-}
-
 // Count pass, one thread per query: the block's cells in nested loops (the
 // reference's order does not matter for a sum)
 __global__ void k_hg_qcount(HGDev G, const float* __restrict__ q, int64_t nq, uint32_t src,
@@ -196,28 +156,28 @@ __global__ void k_hg_qfill(HGDev G, const float* __restrict__ q, int64_t nq, uin
     }
 }
 
-// Exclusive scan of n uint32 counts into int64 offsets[0..n] (offsets[n] =
-// total): per-block sums, one block scanning the sums, then each block's
-// scan plus its carry.
+// Exclusive scan of n uint32 counts into out[0..n] (out[n] = total, where
+// asked for): per-block sums, one block scanning the sums, then each block's
+// scan plus its carry.  A warp takes SCAN_ROWS rows of 32 counts, so that every
+// access is a full line (2 M counts: sums 10 -> 3.9 us, apply 11.4 -> 7.7 us
+// against one count per thread).
 constexpr int SCAN_T = 1024;
-__device__ __forceinline__ int64_t block_incl_scan(int64_t x, int64_t* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+constexpr int SCAN_ROWS = 4;
+constexpr int SCAN_TILE = SCAN_T * SCAN_ROWS;  // counts per block
+__device__ __forceinline__ int64_t warp_incl_scan(int64_t x, int lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int64_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
         if (lane >= o) x += y;
     }
+    return x;
+}
+__device__ __forceinline__ int64_t block_incl_scan(int64_t x, int64_t* sh) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    x = warp_incl_scan(x, lane);
     if (lane == 31) sh[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-        int64_t w = lane < SCAN_T / 32 ? sh[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int64_t y = __shfl_up_sync(0xFFFFFFFFu, w, o);
-            if (lane >= o) w += y;
-        }
-        sh[lane] = w;
-    }
+    if (warp == 0) sh[lane] = warp_incl_scan(lane < SCAN_T / 32 ? sh[lane] : 0, lane);
     __syncthreads();
     const int64_t r = x + (warp ? sh[warp - 1] : 0);
     __syncthreads();
@@ -226,9 +186,23 @@ __device__ __forceinline__ int64_t block_incl_scan(int64_t x, int64_t* sh) {
 __global__ void __launch_bounds__(SCAN_T) k_scan_sums(const uint32_t* __restrict__ in, int64_t n,
                                                       int64_t* __restrict__ bsum) {
     __shared__ int64_t sh[32];
-    const int64_t i = (int64_t)blockIdx.x * SCAN_T + threadIdx.x;
-    const int64_t r = block_incl_scan(i < n ? in[i] : 0, sh);
-    if (threadIdx.x == SCAN_T - 1) bsum[blockIdx.x] = r;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int64_t s = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ROWS; ++k) {
+        const int64_t i = (int64_t)blockIdx.x * SCAN_TILE + k * SCAN_T + threadIdx.x;
+        s += i < n ? in[i] : 0u;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, o);
+    if (lane == 0) sh[warp] = s;
+    __syncthreads();
+    if (warp == 0) {
+        s = sh[lane];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xFFFFFFFFu, s, o);
+        if (lane == 0) bsum[blockIdx.x] = s;
+    }
 }
 __global__ void __launch_bounds__(SCAN_T) k_scan_carry(int64_t* __restrict__ bsum, int64_t nb) {
     __shared__ int64_t sh[32];
@@ -245,16 +219,172 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_carry(int64_t* __restrict__ bsu
         __syncthreads();
     }
 }
-// OutT: int64 query offsets (with the total in out[n]) or uint32 cell starts
+// OutT: int64 query offsets or uint32 cell starts
 template <class OutT, bool TOTAL>
 __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const uint32_t* __restrict__ in, int64_t n,
                                                        const int64_t* __restrict__ bsum, OutT* __restrict__ out) {
     __shared__ int64_t sh[32];
-    const int64_t i = (int64_t)blockIdx.x * SCAN_T + threadIdx.x;
-    const int64_t v = i < n ? in[i] : 0;
-    const int64_t r = block_incl_scan(v, sh);
-    if (i < n) out[i] = (OutT)(bsum[blockIdx.x] + r - v);
-    if (TOTAL && i == n - 1) out[n] = (OutT)(bsum[blockIdx.x] + r);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + warp * (32 * SCAN_ROWS) + lane;
+    int64_t v[SCAN_ROWS], x[SCAN_ROWS], run = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_ROWS; ++k) v[k] = base + 32 * k < n ? in[base + 32 * k] : 0u;
+#pragma unroll
+    for (int k = 0; k < SCAN_ROWS; ++k) {  // inclusive over the warp's rows so far
+        x[k] = run + warp_incl_scan(v[k], lane);
+        run = __shfl_sync(0xFFFFFFFFu, x[k], 31);
+    }
+    if (lane == 0) sh[warp] = run;
+    __syncthreads();
+    if (warp == 0) sh[lane] = warp_incl_scan(sh[lane], lane);
+    __syncthreads();
+    const int64_t before = bsum[blockIdx.x] + (warp ? sh[warp - 1] : 0);
+#pragma unroll
+    for (int k = 0; k < SCAN_ROWS; ++k) {
+        const int64_t i = base + 32 * k;
+        if (i < n) out[i] = (OutT)(before + x[k] - v[k]);
+        if (TOTAL && i == n - 1) out[n] = (OutT)(before + x[k]);
+    }
+}
+
+// ------------------------------------------------------ dense query sets
+// When the queries are at least 1/4 of the cells (HG_DENSE_CELLS), the index is first laid out
+// again in grid order (x outer, z inner): every cell's bucket, one after the
+// other, so that the 2s+1 cells of a query's block along z are one stretch of
+// it and no query hashes anything:
+//   k_hg_grid    (start, count) of every cell, scanned into the stretches
+//   k_hg_expand  the buckets in grid order (buckets that several cells hash to
+//                are repeated: at most mult_max times the particles)
+//   k_hg_rows    each cell's stretch of 2s+1 cells along z
+//   k_hg_blocks  and the particles of its whole block, once per cell instead of
+//                once per query
+//   k_hg_dcount  per query: its cell's block sum
+//   k_hg_dfill   27 lanes for three queries (or a warp per query): a lane reads
+//                one stretch, the lanes then take the lists' entries in turn
+//                (hg_walk), so that lists are written in full lines
+// Bound by scattered L1/L2 accesses.  2 M queries over 2 M cells of one
+// particle each (27 cells per query): count and fill 168 + 496 us with the
+// hashed kernels (27 scattered 4-byte reads a query and pass, entries copied
+// cell by cell), 15 + 228 us here and 64 us for the layout (380 us for the fill
+// with one query per warp and a lane per cell).
+constexpr uint32_t HG_OUTSIDE = 0xFFFFFFFFu;  // qcell: the query is outside the grid
+
+__global__ void k_hg_mult(HGDev G, uint32_t* __restrict__ mult) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= G.total) return;
+    const uint32_t z = c % G.res[2], xy = c / G.res[2], y = xy % G.res[1], x = xy / G.res[1];
+    atomicAdd(&mult[hg_mod(hg_morton(x, y, z), G)], 1u);
+}
+__global__ void k_hg_max(const uint32_t* __restrict__ v, uint32_t n, uint32_t* __restrict__ out) {
+    uint32_t m = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, v[i]);
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
+}
+__global__ void k_hg_grid(HGDev G, const uint32_t* __restrict__ counts, const uint32_t* __restrict__ starts,
+                          uint32_t* __restrict__ ccount, uint32_t* __restrict__ cstart) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= G.total) return;
+    const uint32_t z = c % G.res[2], xy = c / G.res[2], y = xy % G.res[1], x = xy / G.res[1];
+    const uint32_t id = hg_mod(hg_morton(x, y, z), G);
+    ccount[c] = counts[id];
+    cstart[c] = starts[id];
+}
+// first[c] .. first[c + 1]: cell c's bucket in grid order
+__global__ void k_hg_expand(uint32_t total, const uint32_t* __restrict__ first, const uint32_t* __restrict__ cstart,
+                            const uint32_t* __restrict__ sorted_index, uint32_t* __restrict__ out) {
+    // warps copy their 32 cells' buckets together: one stretch of out
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t f = c < total ? first[c] : 0u, k = c < total ? first[c + 1] - f : 0u;
+    const int lane = threadIdx.x & 31;
+    uint32_t* dst = out + __shfl_sync(0xFFFFFFFFu, f, 0);
+    hg_walk(c < total ? cstart[c] : 0u, k, lane, [&](bool valid, uint32_t e, uint32_t pos) {
+        if (valid) dst[e] = __ldg(&sorted_index[pos]);
+    });
+}
+__global__ void k_hg_rows(HGDev G, uint32_t src, const uint32_t* __restrict__ first, uint2* __restrict__ rows) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= G.total) return;
+    const uint32_t z = c % G.res[2], row = c - z;
+    const uint32_t f = first[row + (z > src ? z - src : 0u)];
+    rows[c] = make_uint2(f, first[row + min(z + src, G.res[2] - 1u) + 1u] - f);
+}
+__global__ void k_hg_blocks(HGDev G, uint32_t src, const uint2* __restrict__ rows, uint32_t* __restrict__ sums) {
+    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= G.total) return;
+    const uint32_t z = c % G.res[2], xy = c / G.res[2], y = xy % G.res[1], x = xy / G.res[1];
+    const uint32_t x0 = x > src ? x - src : 0u, x1 = min(x + src, G.res[0] - 1u);
+    const uint32_t y0 = y > src ? y - src : 0u, y1 = min(y + src, G.res[1] - 1u);
+    uint32_t k = 0;
+    for (uint32_t i = x0; i <= x1; ++i)
+        for (uint32_t j = y0; j <= y1; ++j) k += rows[(i * G.res[1] + j) * G.res[2] + z].y;
+    sums[c] = k;
+}
+__global__ void k_hg_dcount(HGDev G, const float* __restrict__ q, int64_t nq, uint32_t src,
+                            const uint32_t* __restrict__ first, const uint32_t* __restrict__ sums,
+                            uint32_t* __restrict__ qcount, uint32_t* __restrict__ qcell) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nq) return;
+    uint32_t c[3];
+    bool in = true;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        c[a] = hg_coord(q[3 * i + a], G.dmin[a], G.cell);
+        in = in && c[a] < G.res[a];
+    }
+    const uint32_t lin = (c[0] * G.res[1] + c[1]) * G.res[2] + c[2];
+    uint32_t k = 0;
+    if (in)
+        k = sums[lin];
+    else
+        for (uint32_t dx = 0; dx <= 2 * src; ++dx)
+            for (uint32_t dy = 0; dy <= 2 * src; ++dy) k += hg_row(G, c, src, dx, dy, first).y;
+    qcount[i] = k;
+    qcell[i] = in ? lin : HG_OUTSIDE;
+}
+// Nothing is written when the lists (offsets[nq] entries) exceed capacity.
+// QW: queries a warp takes together; their lists are one stretch of out, and
+// (2 src + 1)^2 QW <= 32 stretches come from one read per lane.  QW = 1 also
+// takes wider blocks, 32 stretches at a time.
+template <int QW>
+__global__ void __launch_bounds__(HG_T) k_hg_dfill(HGDev G, const float* __restrict__ q, int64_t nq, uint32_t src,
+                                                   const uint32_t* __restrict__ first, const uint2* __restrict__ rows,
+                                                   const uint32_t* __restrict__ index,
+                                                   const uint32_t* __restrict__ qcell,
+                                                   const int64_t* __restrict__ offsets, int64_t capacity,
+                                                   uint32_t* __restrict__ out) {
+    if (offsets[nq] > capacity) return;
+    const uint32_t w = 2 * src + 1, nrow = w * w;
+    const int lane = threadIdx.x & 31;
+    const uint32_t mine = QW > 1 ? lane / nrow : 0u;  // this lane's query of the warp's, and its row of it
+    const uint32_t r1 = QW > 1 ? lane % nrow : (uint32_t)lane;
+    const int64_t step = (int64_t)gridDim.x * (HG_T / 32) * QW;
+    for (int64_t i0 = ((int64_t)blockIdx.x * (HG_T / 32) + (threadIdx.x >> 5)) * QW; i0 < nq; i0 += step) {
+        uint32_t* dst = out + offsets[i0];
+        const int64_t i = i0 + mine;
+        const uint32_t lin = mine < (uint32_t)QW && i < nq ? qcell[i] : HG_OUTSIDE;
+        for (uint32_t r0 = 0; r0 < nrow; r0 += 32) {
+            const uint32_t r = r0 + r1;
+            uint2 seg = make_uint2(0u, 0u);
+            if (r < nrow && mine < (uint32_t)QW && i < nq) {
+                const uint32_t dx = r / w, dy = r % w;
+                if (lin != HG_OUTSIDE) {
+                    const uint32_t xy = lin / G.res[2], y = xy % G.res[1] + dy - src, x = xy / G.res[1] + dx - src;
+                    if (x < G.res[0] && y < G.res[1])
+                        seg = __ldg(&rows[lin + ((dx - src) * G.res[1] + (dy - src)) * G.res[2]]);
+                } else {
+                    uint32_t c[3];
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) c[a] = hg_coord(q[3 * i + a], G.dmin[a], G.cell);
+                    seg = hg_row(G, c, src, dx, dy, first);
+                }
+            }
+            dst += hg_walk(seg.x, seg.y, lane, [&](bool valid, uint32_t e, uint32_t pos) {
+                if (valid) dst[e] = __ldg(&index[pos]);
+            });
+            if (QW > 1) break;
+        }
+    }
 }
 
 __global__ void k_hg_stats(const uint32_t* __restrict__ counts, uint32_t total,
@@ -309,7 +439,72 @@ const float* staged(DevBuf& stage, const float* p, int64_t nfloat, int32_t kind,
     return stage.as<float>();
 }
 
+// Cells per query up to which the dense tables pay: laying them out costs 30 ps
+// per cell (2 M cells), and a hashed query of 27 cells 0.2 ns more than a dense
+// one.
+constexpr int64_t HG_DENSE_CELLS = 4;
+constexpr uint32_t HG_DENSE_MULT = 8;  // most cells per bucket (grid_index is that many times the particles)
+
+// The grid-order tables of the last build for blocks of half width src (kept
+// until the next build).  1: ready; 0: too many cells share a bucket, or their
+// memory is not to be had (the hashed queries need none); < 0: an error.
+int dense_tables(pgmpm_hashgrid_s* g, const HGDev& G, uint32_t src, cudaStream_t st) {
+    const size_t cells = g->total;
+    const int nb = blocks_of((int64_t)cells, HG_T);
+    const int64_t sb = ((int64_t)cells + SCAN_TILE - 1) / SCAN_TILE;
+    auto have = [](cudaError_t e) {
+        if (e != cudaSuccess) cudaGetLastError();  // clear the failed allocation
+        return e == cudaSuccess;
+    };
+    if (!have(g->grid_tables.ensure((sizeof(uint2) + 2 * sizeof(uint32_t)) * cells + sizeof(uint32_t))) ||
+        !have(g->scan_tmp.ensure(sizeof(int64_t) * sb)))
+        return 0;
+    uint32_t* sum = g->grid_sum();
+    // a cube of 2^k cells an axis has no two cells in a bucket; otherwise count
+    // once per grid, since it is a property of the resolution
+    if (g->res[0] == g->res[1] && g->res[1] == g->res[2] && (g->res[0] & (g->res[0] - 1u)) == 0u) g->mult_max = 1;
+    if (g->mult_max == 0) {
+        CK(cudaMemsetAsync(sum, 0, sizeof(uint32_t) * cells, st));
+        CK(cudaMemsetAsync(g->stats.p, 0, sizeof(uint32_t), st));
+        k_hg_mult<<<nb, HG_T, 0, st>>>(G, sum);
+        k_hg_max<<<std::min(nb, 148 * 8), HG_T, 0, st>>>(sum, g->total, g->stats.as<uint32_t>());
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(&g->mult_max, g->stats.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+    }
+    if (g->mult_max > HG_DENSE_MULT || g->n * g->mult_max > 0xFFFFFFFFll ||
+        !have(g->grid_index.ensure(sizeof(uint32_t) * std::max<size_t>((size_t)g->n * g->mult_max, 1))))
+        return 0;
+    uint32_t* first = g->grid_first();
+    if (!g->grid_ready) {
+        uint32_t* cstart = reinterpret_cast<uint32_t*>(g->grid_rows());  // until k_hg_rows writes it
+        int64_t* bsum = g->scan_tmp.as<int64_t>();
+        k_hg_grid<<<nb, HG_T, 0, st>>>(G, g->counts.as<uint32_t>(), g->starts.as<uint32_t>(), sum, cstart);
+        CK(exclusive_scan(sum, (int64_t)cells, bsum, first, st));
+        k_hg_expand<<<nb, HG_T, 0, st>>>(g->total, first, cstart, g->va.as<uint32_t>(), g->grid_index.as<uint32_t>());
+    }
+    if (!g->grid_ready || g->sum_src != (int64_t)src) {
+        k_hg_rows<<<nb, HG_T, 0, st>>>(G, src, first, g->grid_rows());
+        k_hg_blocks<<<nb, HG_T, 0, st>>>(G, src, g->grid_rows(), sum);
+    }
+    CK(cudaGetLastError());
+    g->grid_ready = true;
+    g->sum_src = src;
+    return 1;
+}
+
 }  // namespace
+
+namespace pgmpm {
+size_t exclusive_scan_bytes(int64_t n) { return sizeof(int64_t) * (size_t)((n + SCAN_TILE - 1) / SCAN_TILE); }
+cudaError_t exclusive_scan(const uint32_t* in, int64_t n, int64_t* scratch, uint32_t* out, cudaStream_t st) {
+    const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
+    k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(in, n, scratch);
+    k_scan_carry<<<1, SCAN_T, 0, st>>>(scratch, nb);
+    k_scan_apply<uint32_t, true><<<(int)nb, SCAN_T, 0, st>>>(in, n, scratch, out);
+    return cudaGetLastError();
+}
+}  // namespace pgmpm
 
 extern "C" {
 
@@ -386,7 +581,7 @@ int pgmpm_hashgrid_build(pgmpm_hashgrid g, const float* positions, int64_t n, in
         k_hg_cells<<<blocks_of(n, HG_T), HG_T, 0, st>>>(G, pos, n, ids, counts);
         CK(cudaGetLastError());
     }
-    const int64_t nb = ((int64_t)g->total + SCAN_T - 1) / SCAN_T;
+    const int64_t nb = ((int64_t)g->total + SCAN_TILE - 1) / SCAN_TILE;
     CK(g->scan_tmp.ensure(sizeof(int64_t) * nb));
     int64_t* bsum = g->scan_tmp.as<int64_t>();
     k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(counts, g->total, bsum);
@@ -405,6 +600,8 @@ int pgmpm_hashgrid_build(pgmpm_hashgrid g, const float* positions, int64_t n, in
         CK(cudaMemcpyAsync(g->va.p, sorted_index, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
     g->n = n;
     g->built = true;
+    g->grid_ready = false;
+    g->sum_src = -1;
     return PGMPM_OK;
 }
 
@@ -440,37 +637,68 @@ int pgmpm_hashgrid_neighbors(pgmpm_hashgrid g, const float* queries, int64_t nq,
     const float* q = staged(g->qstage, queries, 3 * nq, ptr_kind, st, rc);
     if (rc) return rc;
     const HGDev G = dev_of(g);
-    CK(g->qcount.ensure(sizeof(uint32_t) * std::max<int64_t>(nq, 1)));
-    const int64_t nb = std::max<int64_t>(1, (nq + SCAN_T - 1) / SCAN_T);
-    // scan_tmp: block sums, then the offsets when the caller's are on the host
+    CK(g->qcount.ensure(2 * sizeof(uint32_t) * std::max<int64_t>(nq, 1)));  // counts, then the queries' cells
+    const int64_t nb = std::max<int64_t>(1, (nq + SCAN_TILE - 1) / SCAN_TILE);
     const size_t off_bytes = sizeof(int64_t) * (size_t)(nq + 1);
+    uint32_t *qcount = g->qcount.as<uint32_t>(), *qcell = qcount + nq;
+    bool dense = false;
+    if (nq > 0 && (int64_t)g->total <= HG_DENSE_CELLS * nq && g->total < 0x80000000u) {
+        rc = dense_tables(g, G, src, st);
+        if (rc < 0) return rc;
+        dense = rc == 1;
+    }
+    // scan_tmp: block sums, then the offsets when the caller's are on the host
     CK(g->scan_tmp.ensure(sizeof(int64_t) * nb + (ptr_kind == PGMPM_PTR_HOST ? off_bytes : 0)));
     int64_t* bsum = g->scan_tmp.as<int64_t>();
     int64_t* doff = ptr_kind == PGMPM_PTR_HOST ? bsum + nb : offsets;
+    const uint32_t* first = dense ? g->grid_first() : nullptr;
     if (nq > 0) {
-        k_hg_qcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts.as<uint32_t>(),
-                                                          g->qcount.as<uint32_t>());
-        k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(g->qcount.as<uint32_t>(), nq, bsum);
+        if (dense)
+            k_hg_dcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, first, g->grid_sum(), qcount,
+                                                              qcell);
+        else
+            k_hg_qcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts.as<uint32_t>(), qcount);
+        k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum);
         k_scan_carry<<<1, SCAN_T, 0, st>>>(bsum, nb);
-        k_scan_apply<int64_t, true><<<(int)nb, SCAN_T, 0, st>>>(g->qcount.as<uint32_t>(), nq, bsum, doff);
+        k_scan_apply<int64_t, true><<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum, doff);
         CK(cudaGetLastError());
     } else {
         CK(cudaMemsetAsync(doff, 0, sizeof(int64_t), st));
+    }
+    auto fill = [&](uint32_t* dout, int64_t cap) {
+        auto dfill = [&](auto kernel, int qw) {
+            kernel<<<(int)std::min<int64_t>(blocks_of(nq, qw * (HG_T / 32)), 148 * 64), HG_T, 0, st>>>(
+                G, q, nq, src, first, g->grid_rows(), g->grid_index.as<uint32_t>(), qcell,
+                doff, cap, dout);
+        };
+        if (dense && src <= 1)  // 1 or 9 stretches per query
+            src == 0 ? dfill(k_hg_dfill<32>, 32) : dfill(k_hg_dfill<3>, 3);
+        else if (dense)
+            dfill(k_hg_dfill<1>, 1);
+        else
+            k_hg_qfill<<<blocks_of(nq * HG_FG, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts.as<uint32_t>(),
+                                                                     g->starts.as<uint32_t>(), g->va.as<uint32_t>(),
+                                                                     doff, dout);
+    };
+    // into a device buffer the dense fill follows at once (it checks the
+    // capacity itself); otherwise the host learns the total first
+    const bool early = dense && indices && capacity > 0 && ptr_kind == PGMPM_PTR_DEVICE;
+    if (early) {
+        fill(indices, capacity);
+        CK(cudaGetLastError());
     }
     int64_t tot = 0;
     CK(cudaMemcpyAsync(&tot, doff + nq, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
     *total = tot;
     if (ptr_kind == PGMPM_PTR_HOST) CK(cudaMemcpyAsync(offsets, doff, off_bytes, cudaMemcpyDeviceToHost, st));
-    if (indices && tot <= capacity && tot > 0) {
+    if (!early && indices && tot <= capacity && tot > 0) {
         uint32_t* dout = indices;
         if (ptr_kind == PGMPM_PTR_HOST) {
             CK(g->qout_stage.ensure(sizeof(uint32_t) * tot));
             dout = g->qout_stage.as<uint32_t>();
         }
-        k_hg_qfill<<<blocks_of(nq * HG_FG, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts.as<uint32_t>(),
-                                                              g->starts.as<uint32_t>(), g->va.as<uint32_t>(), doff,
-                                                              dout);
+        fill(dout, tot);
         CK(cudaGetLastError());
         if (ptr_kind == PGMPM_PTR_HOST)
             CK(cudaMemcpyAsync(indices, dout, sizeof(uint32_t) * tot, cudaMemcpyDeviceToHost, st));
