@@ -962,7 +962,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // 1/64 of a tile, partial sums of split cells joined by a segmented scan), the
 // former variant 4, kept every lane busy but spent two thirds of their
 // instructions on the flush.  P2G per step, runs -> slices: 4,096 particles
-// 9.7 -> 5.1 us, 32,768: 13.4 -> 8.2, 150 K: 18.3 -> 15.4, 262 K sparse: 22.0
+// 9.7 -> 4.7 us, 32,768: 13.4 -> 6.8, 150 K: 18.3 -> 15.4, 262 K sparse: 22.0
 // -> 17.7, 2 M (two densities): 98.0 -> 89.9, 64 scenes of 3.9 M (2 per cell):
 // 268 -> 237.  Slower: 5 blocks per SM (64 registers, spills: 109 us at 2 M),
 // half tiles in 96-thread blocks (104), cells dealt to the warps by particle
@@ -983,9 +983,11 @@ __global__ void __launch_bounds__(P2GS_T, P2GS_BLOCKS) k_p2g_slices(View V) {
     const float wo = k == 0 ? 1.5f : k == 1 ? 1.0f : 0.5f;  // w_k(f) is a quadratic in f - wo
     const int64_t N = V.N;
     const uint32_t ntiles = V.counters[CNT_CTILES];
-    // slices of a cell's particles when tiles are few: one work item per
-    // (tile, slice)
-    const uint32_t S = ntiles ? min(4u, max(1u, (gridDim.x + ntiles - 1) / ntiles)) : 1u;
+    // slices of a cell's particles when tiles are few, one work item per (tile,
+    // slice): as many as still fit the resident blocks at once (rounded up, a
+    // few blocks took a second item: 216 tiles of 5 particles per cell 8.3 ->
+    // 6.8 us; at most 4 instead of 8: 4,096 particles 4.65 -> 5.1 us)
+    const uint32_t S = ntiles ? min(8u, max(1u, gridDim.x / ntiles)) : 1u;
     const uint32_t nwork = ntiles * S;
     // items [0, gridDim.x) are the blocks' first; further ones are claimed,
     // one ahead when there are enough of them that no block holds a claim
