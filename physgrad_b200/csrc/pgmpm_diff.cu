@@ -478,6 +478,7 @@ int pgmpm_backward(pgmpm_solver s, const float* gx_out, const float* gv_out, con
     rc = unprime(s, st);
     if (rc) return rc;
     CK(s->adj_g.ensure(sizeof(float4) * 6 * Nz));
+    CK(s->adj_pay.ensure(sizeof(float4) * 4 * Nz));
     CK(s->adj_grid_gv.ensure(sizeof(float4) * nodes_of(s)));
     CK(s->adj_grid_gpm.ensure(sizeof(float4) * nodes_of(s)));
     CK(s->adj_gE.ensure(sizeof(float) * M));
@@ -501,6 +502,7 @@ int pgmpm_backward(pgmpm_solver s, const float* gx_out, const float* gv_out, con
     CK(launch_state_to_planes(dx, dv, dC, dF, s->user_of_phys.as<uint32_t>(), s->adj_g.as<float4>(), N, st));
     AdjView A;
     A.g = s->adj_g.as<float4>();
+    A.pay = s->adj_pay.as<float4>();
     A.grid_gv = s->adj_grid_gv.as<float4>();
     A.grid_gpm = s->adj_grid_gpm.as<float4>();
     A.gE = s->adj_gE.as<float>();

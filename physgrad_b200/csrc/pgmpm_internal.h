@@ -287,6 +287,7 @@ struct AdjView {
     // adjoint of the state before it (physical order, same plane packing)
     float4* g;                 // 6 planes
     const float4* q_next;      // state after the step (C' for the F update and the fluid reset)
+    float4* pay;               // the scatter's payload (4 planes of N float4)
     float4* grid_gv;           // (0, dL/dv_i) scatter target, zeroed by the grid adjoint
     float4* grid_gpm;          // (dL/dp_i, dL/dm_i) per node
     float* gE;                 // [M] dL/dE accumulators

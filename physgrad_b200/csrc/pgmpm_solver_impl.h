@@ -188,7 +188,7 @@ struct pgmpm_solver_s {
     cudaStream_t side_stream = nullptr;  // the replay that overlaps a segment's reverse
     cudaStream_t body_stream = nullptr;  // captures the bodies of conditional graph nodes
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-    pgmpm::DevBuf adj_g, adj_grid_gv, adj_grid_gpm, adj_gE, adj_stage;
+    pgmpm::DevBuf adj_g, adj_pay, adj_grid_gv, adj_grid_gpm, adj_gE, adj_stage;
 
     pgmpm::StepBufs live_bufs() const {
         pgmpm::StepBufs b;

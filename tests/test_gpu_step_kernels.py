@@ -121,6 +121,44 @@ def test_p2g_of_uneven_cells_equals_thread_per_cell(gpu, counts, sparse):
     assert np.abs(grids[0][1] - grids[1][1]).max() <= 4 * bound * grids[1][0].max() + 1e-12
 
 
+@pytest.mark.parametrize("counts", [[1], [64], [1, 0, 3], [700], [5, 900, 2, 1, 40], [2000, 1]])
+@pytest.mark.parametrize("mats", ["elastic", "mixed"])
+def test_adjoint_scatter_of_uneven_cells_equals_thread_per_cell(gpu, counts, mats):
+    """The reverse step from cells of very different counts, through the
+    scatter over a stored payload and the one with a thread per cell.  The
+    gradients are sums over at most n particles' terms, so the two orders
+    differ by a few times n 2^-23 of the largest gradient (3 stages: scatter,
+    grid, gather), and 1e-5 for the arithmetic of the stress adjoint."""
+    rng = np.random.default_rng(len(counts) + sum(counts))
+    n, dx = (23, 22, 21), 1.0 / 16
+    xs = []
+    for i, c in enumerate(counts):
+        cell = np.array([[4, 4, 4], [7, 7, 7], [8, 7, 4], [11, 8, 8], [0, 0, 0], [19, 18, 17]])[i % 6]
+        xs.append((cell + 0.5 + rng.uniform(0.1, 0.9, (c, 3))) * dx)
+    x = np.concatenate(xs).astype(np.float32)
+    N = len(x)
+    V0 = np.full(N, (dx / 2) ** 3, np.float32)
+    scene = gpu.Scene(n, dx, 1e-4, (0.0, -9.8, 0.0), (0.0, 0.0, 0.0), 0, 0, 0)
+    v, Cm = rng.uniform(-1, 1, (N, 3)).astype(np.float32), rng.uniform(-5, 5, (N, 9)).astype(np.float32)
+    F = (np.eye(3).ravel() + rng.normal(0, 0.02, (N, 9))).astype(np.float32)
+    ms = [gpu.createElasticMaterial(1000.0, 1e4, 0.3)]
+    if mats == "mixed":
+        ms.append(gpu.createFluidMaterial(1000, 5.0, 1e4))
+    go = {k: rng.normal(0, 1, (N, d)).astype(np.float32) for k, d in (("x", 3), ("v", 3), ("C", 9), ("F", 9))}
+    res = []
+    for variant in (4, 2):
+        sim = gpu.Simulator([scene], [N], ms)
+        if variant != 4:
+            sim.set_variants(p2g_variant=variant)
+        sim.upload(x, v, Cm, F, (1000 * V0).astype(np.float32), V0, (np.arange(N) % len(ms)).astype(np.int32))
+        sim.forward_checkpointed(1, 1)
+        res.append(sim.backward(go))
+        assert sim.status() == 0
+    for key in ("x", "v", "C", "F"):
+        a, b = np.asarray(res[0][key]).ravel(), np.asarray(res[1][key]).ravel()
+        assert np.abs(a - b).max() <= (3 * N * 2.0 ** -23 + 1e-5) * np.abs(b).max(), key
+
+
 @pytest.mark.parametrize("N", [1, 31, 32, 33, 255, 257, 1000])
 @pytest.mark.parametrize("device", [False, True])
 def test_upload_download_round_trip(gpu, N, device):
