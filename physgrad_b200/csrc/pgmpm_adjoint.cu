@@ -21,6 +21,7 @@ namespace {
 __device__ __forceinline__ const SceneDev& scene_ref(const View& V, int s) { return V.scenes[s]; }
 
 __global__ void k_adj_grid(View V, AdjView A) {
+    step_wait();
     // the scatter has finished with the work cursor: leave it at zero, as the
     // forward's grid update does, so that a later replay of this step that
     // keeps its recorded sort (no counter reset) starts its P2G from zero
@@ -70,6 +71,7 @@ constexpr int MAX_SMEM_MATS = 64;
 
 template <bool MULTI, bool FLUID>
 __global__ void __launch_bounds__(GATHER_T, 4) k_adj_gather(View V, AdjView A) {
+    step_wait();
     __shared__ float sE[MAX_SMEM_MATS];
     const bool smem_e = V.M <= MAX_SMEM_MATS;
     for (int m = threadIdx.x; m < MAX_SMEM_MATS; m += blockDim.x) sE[m] = 0.f;
@@ -348,8 +350,7 @@ cudaError_t launch_adj_grid(const View& V, const AdjView& A, const Tuning& t, in
     int64_t nb = ((int64_t)V.total_nt + tiles_per_block - 1) / tiles_per_block;
     if (nb > num_sms * 8) nb = num_sms * 8;
     if (nb < 1) nb = 1;
-    k_adj_grid<<<(int)nb, t.grid_block, 0, st>>>(V, A);
-    return cudaGetLastError();
+    return launch_after(V.early, k_adj_grid, (int)nb, t.grid_block, st, V, A);
 }
 
 cudaError_t launch_adj_gather(const View& V, const AdjView& A, const PhysFlags& pf, const Tuning& t,
@@ -357,18 +358,9 @@ cudaError_t launch_adj_gather(const View& V, const AdjView& A, const PhysFlags& 
     (void)t;
     if (V.N == 0) return cudaSuccess;
     const int nb = blocks_for(V.N, GATHER_T);
-    if (pf.multi_mat) {
-        if (pf.has_fluid)
-            k_adj_gather<true, true><<<nb, GATHER_T, 0, st>>>(V, A);
-        else
-            k_adj_gather<true, false><<<nb, GATHER_T, 0, st>>>(V, A);
-    } else {
-        if (pf.has_fluid)
-            k_adj_gather<false, true><<<nb, GATHER_T, 0, st>>>(V, A);
-        else
-            k_adj_gather<false, false><<<nb, GATHER_T, 0, st>>>(V, A);
-    }
-    return cudaGetLastError();
+    auto kernel = pf.multi_mat ? (pf.has_fluid ? k_adj_gather<true, true> : k_adj_gather<true, false>)
+                               : (pf.has_fluid ? k_adj_gather<false, true> : k_adj_gather<false, false>);
+    return launch_after(V.early, kernel, nb, GATHER_T, st, V, A);
 }
 
 cudaError_t launch_state_to_planes(const float* x, const float* v, const float* C, const float* F,

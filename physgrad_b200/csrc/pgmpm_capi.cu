@@ -142,7 +142,9 @@ int conditional_sort(pgmpm_solver s, const View& V, const BinSortBufs& B, uint32
     CK(cudaStreamUpdateCaptureDependencies(st, &cn, 1, cudaStreamSetCaptureDependencies));
     cudaGraph_t body = np.conditional.phGraph_out[0];
     CK(cudaStreamBeginCaptureToGraph(s->body_stream, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-    const cudaError_t e = bin_sort_step(V, B, s->num_sms, false, s->body_stream);
+    View W = V;
+    W.early = false;
+    const cudaError_t e = bin_sort_step(W, B, s->num_sms, false, s->body_stream);
     cudaGraph_t out = nullptr;
     const cudaError_t e2 = cudaStreamEndCapture(s->body_stream, &out);
     CK(e);
@@ -165,6 +167,8 @@ int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, 
         return fail(PGMPM_ERR_STATE, "internal: keys counted ahead need the bin sort and the physical-order G2P");
     View V = s->view_for(b);
     if (count_next) V.cnt = s->sort_counts();
+    V.early = !timed;
+    V.early_first = counted && !timed;  // after the previous step's G2P
     // P2G variant 1 builds its payload from the state's v and C
     V.write_vc = write_vc || s->pf.physics != PHYS_MLS || s->tune.p2g_variant == 1 ? 1 : 0;
     // per-step resets: tile counts, active node count, work cursors, and the
@@ -191,10 +195,17 @@ int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, 
         CK(launch_mark(V, st));
     }
     if (timed) CK(cudaEventRecord(s->ev[1], st));
+    // P2G follows a copy, a memset or a conditional node where the step keeps
+    // its recorded order
+    const bool early = V.early;
+    V.early = early && s->tune.step_sort == 0 && b.sort_mode == 0;
     // a fused step's P2G was done by the previous step's G2P2G
     if (kind == STEP_SPLIT || kind == STEP_FUSED_FIRST) CK(launch_p2g(V, s->pf, s->tune, s->num_sms, st));
     if (timed) CK(cudaEventRecord(s->ev[2], st));
+    // (a fused step's grid update follows what its P2G would have)
+    if (kind == STEP_SPLIT || kind == STEP_FUSED_FIRST) V.early = early;
     CK(launch_grid(V, s->pf, s->tune, s->num_sms, st));
+    V.early = early;
     if (timed) CK(cudaEventRecord(s->ev[3], st));
     if (kind == STEP_FUSED_FIRST || kind == STEP_FUSED) {
         V.pay_out = nullptr;  // the payload stays in the SM; the buffer goes stale

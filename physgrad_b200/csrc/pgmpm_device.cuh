@@ -21,6 +21,14 @@
 
 namespace pgmpm {
 
+// First statement of the kernels that launch_after may launch early: waits until
+// the kernel before on the stream has completed and its writes are visible.
+// Nothing is read before it, and these kernels read what others of the step
+// write by plain loads, not through the read-only path.
+__device__ __forceinline__ void step_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 enum { PHYS_MLS = 0, PHYS_REF = 1 };
 enum { BC_NONE = 0, BC_STICKY = 1, BC_SLIP = 2, BC_SEPARATE = 3 };
 enum { MODEL_FCR = 0, MODEL_NH = 1, MODEL_EOS = 2, MODEL_VM = 3 };  // VM: neo-Hookean + von Mises

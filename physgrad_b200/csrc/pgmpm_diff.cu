@@ -223,6 +223,8 @@ int record_tape_reverse(pgmpm_solver s, const AdjView& A0, int len, cudaStream_t
         StepBufs b = tape_bufs(s, j, t, g0 < 0 ? -1 : g0 + j);
         View V = s->view_for(b);
         V.grid_mp = A.grid_gv;  // scatter target of the G2P reverse
+        V.early = true;
+        V.early_first = j < len - 1;  // after the previous slot's gather
         A.q_next = b.q_out;
         // the slot's P2G work cursor is zero: the grid update of the slot's
         // forward step cleared it after P2G (and a previous reverse's grid

@@ -973,6 +973,7 @@ constexpr int P2GS_BLOCKS = 4;  // resident blocks per SM
 
 template <bool SPARSE, bool ADJ>
 __global__ void __launch_bounds__(P2GS_T, P2GS_BLOCKS) k_p2g_slices(View V) {
+    step_wait();
     __shared__ float4 T4[3 * P2GS_PLANE];  // [z-offset][x-offset + 3 y-offset][cell]: (m, p) of the cell's node
     __shared__ uint4 s_item[2];            // this and the next item's tile (see View::ptile)
     __shared__ uint32_t s_slice[2];        // and its slice; ~0: no item
@@ -1130,6 +1131,7 @@ __global__ void __launch_bounds__(P2GS_T, P2GS_BLOCKS) k_p2g_slices(View V) {
 // it L2 hits).
 template <bool MULTI, bool FLUID>
 __global__ void __launch_bounds__(128) k_adj_payload(View V, AdjView AV) {
+    step_wait();
     const int64_t N = V.N;
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= N) return;
@@ -1147,6 +1149,7 @@ __global__ void __launch_bounds__(128) k_adj_payload(View V, AdjView AV) {
 // ------------------------------------------------------------ grid update
 template <int PHYS>
 __global__ void k_grid(View V) {
+    step_wait();
     // P2G has finished with its work cursor: leave it at zero for the reverse
     // of this step, whose scatter takes work from the same cursor
     if (blockIdx.x == 0 && threadIdx.x == 0) V.counters[CNT_P2G_CURSOR] = 0u;
@@ -2066,22 +2069,13 @@ cudaError_t launch_adj_scatter(const View& V, const AdjView& A, const PhysFlags&
     if (V.N == 0) return cudaSuccess;
     if (pf.physics != PHYS_MLS) return cudaErrorNotSupported;
     if (t.p2g_variant >= 4 && V.cell_range) {  // three threads per cell over the sort's cell table
-        const int nb = (int)((V.N + 127) / 128);
-        if (pf.multi_mat) {
-            if (pf.has_fluid)
-                k_adj_payload<true, true><<<nb, 128, 0, st>>>(V, A);
-            else
-                k_adj_payload<true, false><<<nb, 128, 0, st>>>(V, A);
-        } else {
-            if (pf.has_fluid)
-                k_adj_payload<false, true><<<nb, 128, 0, st>>>(V, A);
-            else
-                k_adj_payload<false, false><<<nb, 128, 0, st>>>(V, A);
-        }
+        auto payload = pf.multi_mat ? (pf.has_fluid ? k_adj_payload<true, true> : k_adj_payload<true, false>)
+                                    : (pf.has_fluid ? k_adj_payload<false, true> : k_adj_payload<false, false>);
+        const cudaError_t e = launch_after(V.early_first, payload, (int)((V.N + 127) / 128), 128, st, V, A);
+        if (e != cudaSuccess) return e;
         View S = V;
         S.pay = A.pay;
-        k_p2g_slices<false, true><<<num_sms * P2GS_BLOCKS, P2GS_T, 0, st>>>(S);
-        return cudaGetLastError();
+        return launch_after(V.early, k_p2g_slices<false, true>, num_sms * P2GS_BLOCKS, P2GS_T, st, S);
     }
     if (t.p2g_variant >= 2) {  // the adjoint scatter of variant 3 (and of 4 without a cell table) is variant 2's
         const int nb = num_sms * t.cell_blocks_per_sm;
@@ -2118,12 +2112,9 @@ cudaError_t launch_p2g(const View& V, const PhysFlags& pf, const Tuning& t, int 
     if (t.p2g_variant >= 3 && pf.physics == PHYS_MLS) {
         if (!V.pay) return cudaErrorInvalidValue;
         if (t.p2g_variant >= 4 && V.cell_range)  // without the sort's cell table: variant 3
-            if (V.sp.cap)
-                k_p2g_slices<true, false><<<num_sms * min(P2GS_BLOCKS, t.pair_blocks_per_sm), P2GS_T, 0, st>>>(V);
-            else
-                k_p2g_slices<false, false><<<num_sms * min(P2GS_BLOCKS, t.pair_blocks_per_sm), P2GS_T, 0, st>>>(V);
-        else
-            k_p2g_pairs<<<num_sms * t.pair_blocks_per_sm, P2GP_T, 0, st>>>(V);
+            return launch_after(V.early, V.sp.cap ? k_p2g_slices<true, false> : k_p2g_slices<false, false>,
+                                num_sms * min(P2GS_BLOCKS, t.pair_blocks_per_sm), P2GS_T, st, V);
+        k_p2g_pairs<<<num_sms * t.pair_blocks_per_sm, P2GP_T, 0, st>>>(V);
         return cudaGetLastError();
     }
     if (t.p2g_variant >= 2) {  // REF physics: variants 3 to 5 run variant 2
@@ -2172,11 +2163,8 @@ cudaError_t launch_grid(const View& V, const PhysFlags& pf, const Tuning& t, int
     const int cap = num_sms * 8;
     if (nb > cap) nb = cap;
     if (nb < 1) nb = 1;
-    if (pf.physics == PHYS_MLS)
-        k_grid<PHYS_MLS><<<(int)nb, t.grid_block, 0, st>>>(V);
-    else
-        k_grid<PHYS_REF><<<(int)nb, t.grid_block, 0, st>>>(V);
-    return cudaGetLastError();
+    return launch_after(V.early, pf.physics == PHYS_MLS ? k_grid<PHYS_MLS> : k_grid<PHYS_REF>, (int)nb, t.grid_block,
+                        st, V);
 }
 
 // ...: further template arguments of KERNEL

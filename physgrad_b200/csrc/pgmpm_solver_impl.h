@@ -243,6 +243,7 @@ struct pgmpm_solver_s {
         V.cell_range = tune.step_sort == 0 ? b.cell_range : nullptr;
         V.ptile = tune.step_sort == 0 ? b.ptile : nullptr;
         V.sort_work = bs_work.as<uint32_t>();
+        V.early = V.early_first = false;
         V.cnt = pgmpm::SortCounts{};
         V.counters = b.counters;
         V.total_ct = total_ct;

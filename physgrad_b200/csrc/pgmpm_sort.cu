@@ -261,8 +261,8 @@ __device__ __forceinline__ void bs_run(uint32_t bin, bool ok, int lane, int& sta
     end = after ? __ffs(after) - 1 : 32;
 }
 
-__global__ void __launch_bounds__(BS_T) bs_count(const uint32_t* __restrict__ keys, int64_t n, SortCounts c,
-                                                 uint32_t* __restrict__ counters) {
+__global__ void __launch_bounds__(BS_T) bs_count(const uint32_t* keys, int64_t n, SortCounts c, uint32_t* counters) {
+    step_wait();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // a new step stamp (sparse grids mark active node tiles with it)
     if (blockIdx.x == 0 && threadIdx.x == 0) counters[CNT_STAMP] += 1u;
@@ -322,8 +322,8 @@ __device__ __forceinline__ int bs_class(uint32_t count) {
 
 // tcount holds a multiple of 4 words past the tiles' and the overflow bin's
 // (zero), so a group of BS_GROUP or a run of 4 may be read whole
-__global__ void __launch_bounds__(BS_T) bs_groups(const uint32_t* __restrict__ tcount, int64_t n,
-                                                  uint32_t* __restrict__ gsum) {
+__global__ void __launch_bounds__(BS_T) bs_groups(const uint32_t* tcount, int64_t n, uint32_t* gsum) {
+    step_wait();
     static_assert(BS_GROUP == 4 * BS_T, "one 16-byte load per thread");
     __shared__ uint32_t s_sum[BS_T / 32];
     const int64_t i = (int64_t)blockIdx.x * BS_GROUP + 4 * threadIdx.x;
@@ -342,9 +342,9 @@ __global__ void __launch_bounds__(BS_T) bs_groups(const uint32_t* __restrict__ t
 // Blocks [0, cell_blocks): (a), the rest: (b).  See the overview above.
 // gsum: the groups' sums, or null where the tile counts are summed directly.
 template <int BT_PER_WARP>
-__global__ void __launch_bounds__(BS_T) bs_tiles(View V, SortCounts c, const uint32_t* __restrict__ gsum,
-                                                 uint2* __restrict__ cell_range, uint4* __restrict__ tile_info,
-                                                 int cell_blocks) {
+__global__ void __launch_bounds__(BS_T) bs_tiles(View V, SortCounts c, const uint32_t* gsum, uint2* cell_range,
+                                                 uint4* tile_info, int cell_blocks) {
+    step_wait();
     constexpr int BT_TILES = BT_PER_WARP * (BS_T / 32);
     static_assert(BT_TILES <= 64 && BT_TILES % 4 == 0, "two tiles per lane in the scan, 16-byte reads of the counts");
     __shared__ uint32_t s_cnt[BT_TILES], s_slot[BT_TILES], s_rank[BT_TILES], s_sum[BS_T / 32];
@@ -477,11 +477,10 @@ __global__ void __launch_bounds__(BS_T) bs_tiles(View V, SortCounts c, const uin
 // with u the grid coordinates and s the cell's lowest node, (v, index) and for
 // the reverse (gv + dt gx, 0).
 template <bool REC>
-__global__ void __launch_bounds__(BS_T) bs_scatter(View V, const uint32_t* __restrict__ keys, SortCounts c,
-                                                   const uint2* __restrict__ cell_range,
-                                                   const uint4* __restrict__ tile_info, uint4* __restrict__ ptile,
-                                                   uint32_t* __restrict__ ok_, uint32_t* __restrict__ ov,
-                                                   int tile_blocks, RefStep R) {
+__global__ void __launch_bounds__(BS_T) bs_scatter(View V, const uint32_t* keys, SortCounts c, const uint2* cell_range,
+                                                   const uint4* tile_info, uint4* ptile, uint32_t* ok_,
+                                                   uint32_t* ov, int tile_blocks, RefStep R) {
+    step_wait();
     const int64_t n = V.N;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if ((int)blockIdx.x < tile_blocks) {
@@ -559,27 +558,29 @@ cudaError_t bin_sort_step(const View& V, const BinSortBufs& B, int num_sms, bool
     if (!B.cell_range || !B.ptile || !V.sort_work) return cudaErrorInvalidValue;
     const int gk = (int)((n + BS_TILE - 1) / BS_TILE);
     const int64_t nct = V.total_ct;
-    if (!counted) bs_count<<<gk, BS_T, 0, st>>>(B.keys_in, n, B.cnt, V.counters);
+    cudaError_t e = cudaSuccess;
+    if (!counted) e = launch_after(V.early_first, bs_count, gk, BS_T, st, B.keys_in, n, B.cnt, V.counters);
+    bool early = counted ? V.early_first : V.early;
     const uint32_t* gsum = nct > BS_DIRECT_TILES ? B.gsum : nullptr;
-    if (gsum) bs_groups<<<(int)bin_sort_groups(nct), BS_T, 0, st>>>(B.cnt.tcount, nct + 1, B.gsum);
+    if (gsum && e == cudaSuccess) {
+        e = launch_after(early, bs_groups, (int)bin_sort_groups(nct), BS_T, st, B.cnt.tcount, nct + 1, B.gsum);
+        early = V.early;
+    }
+    if (e != cudaSuccess) return e;
     // sparse grids mark their node tiles from the occupied cell tiles
     const int node_blocks = V.sp.cap ? 0 : (V.total_nt + BS_T - 1) / BS_T;
     const int per_block = (nct <= BT_FEW_TILES ? BT_FEW : BT_MANY) * (BS_T / 32);
     const int cell_blocks = (int)((nct + per_block - 1) / per_block);
-    if (nct <= BT_FEW_TILES)
-        bs_tiles<BT_FEW><<<cell_blocks + node_blocks, BS_T, 0, st>>>(V, B.cnt, gsum, B.cell_range, B.tile_info,
-                                                                    cell_blocks);
-    else
-        bs_tiles<BT_MANY><<<cell_blocks + node_blocks, BS_T, 0, st>>>(V, B.cnt, gsum, B.cell_range, B.tile_info,
-                                                                     cell_blocks);
+    e = launch_after(early, nct <= BT_FEW_TILES ? bs_tiles<BT_FEW> : bs_tiles<BT_MANY>, cell_blocks + node_blocks, BS_T,
+                     st, V, B.cnt, gsum, B.cell_range, B.tile_info, cell_blocks);
+    if (e != cudaSuccess) return e;
     const int tile_blocks = (int)std::min<int64_t>(num_sms, (nct + BS_T - 1) / BS_T);
     if (rec)
-        bs_scatter<true><<<tile_blocks + (int)((n + BS_T * BS_REC_ITEMS - 1) / (BS_T * BS_REC_ITEMS)), BS_T, 0, st>>>(V, B.keys_in, B.cnt, B.cell_range, B.tile_info, B.ptile,
-                                                           nullptr, nullptr, tile_blocks, *rec);
-    else
-        bs_scatter<false><<<tile_blocks + gk, BS_T, 0, st>>>(V, B.keys_in, B.cnt, B.cell_range, B.tile_info, B.ptile,
-                                                            B.out_k, B.out_v, tile_blocks, RefStep{});
-    return cudaGetLastError();
+        return launch_after(V.early, bs_scatter<true>,
+                            tile_blocks + (int)((n + BS_T * BS_REC_ITEMS - 1) / (BS_T * BS_REC_ITEMS)), BS_T, st, V,
+                            B.keys_in, B.cnt, B.cell_range, B.tile_info, B.ptile, nullptr, nullptr, tile_blocks, *rec);
+    return launch_after(V.early, bs_scatter<false>, tile_blocks + gk, BS_T, st, V, B.keys_in, B.cnt, B.cell_range,
+                        B.tile_info, B.ptile, B.out_k, B.out_v, tile_blocks, RefStep{});
 }
 
 int64_t radix_sort_scratch_words(int64_t n) { return radix_scratch_words_for(n); }
