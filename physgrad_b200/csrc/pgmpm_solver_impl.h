@@ -147,6 +147,14 @@ struct pgmpm_solver_s {
     cudaStream_t cap_stream = nullptr;
     cudaGraphExec_t step_exec[pgmpm::STEP_KINDS][4] = {};
     cudaGraph_t step_graph[pgmpm::STEP_KINDS][4] = {};
+    int step_seen[pgmpm::STEP_KINDS][4] = {};  // such steps launched without a graph
+    static constexpr int kDirectSteps = 4;
+    // several split steps in one graph (run_steps): all steps of a call, and
+    // kMidSteps steps with others of their call before and after them
+    static constexpr int kCallSteps = 64, kCallRepeats = 3, kMidSteps = 16, kMidAtLeast = 128;
+    cudaGraphExec_t call_exec = nullptr, mid_exec = nullptr;
+    int call_steps = 0;               // steps of call_exec
+    int call_last = 0, call_seen = 0; // steps of the last call, and calls in a row that had as many
     cudaEvent_t ev[6] = {};
 
     // metrics
@@ -277,7 +285,12 @@ struct pgmpm_solver_s {
                 if (step_graph[k][m]) cudaGraphDestroy(step_graph[k][m]);
                 step_exec[k][m] = nullptr;
                 step_graph[k][m] = nullptr;
+                step_seen[k][m] = 0;
             }
+        if (call_exec) cudaGraphExecDestroy(call_exec);
+        if (mid_exec) cudaGraphExecDestroy(mid_exec);
+        call_exec = mid_exec = nullptr;
+        call_steps = call_last = call_seen = 0;
         drop_tape_graphs();
     }
 

@@ -83,6 +83,36 @@ def test_sorts_inside_a_call_equal_single_step_calls(gpu, N, n, boundary):
     _close(a.download(), b.download())
 
 
+@pytest.mark.parametrize("calls", [[1] * 7, [2] * 5, [5, 5, 3, 5, 5, 5, 3, 3, 3], [64, 64, 64, 64], [131, 146, 17, 200]])
+@pytest.mark.parametrize("sparse", [False, True])
+def test_steps_launched_one_by_one_and_in_graphs_agree(gpu, calls, sparse):
+    """Calls of equal and of changing lengths, which run step by step, as a
+    graph per step, per call or per 16 steps: against launches without graphs.
+    The particles are free (no stress, no gravity), so the difference of two
+    runs grows with the steps' rounding only: half an ulp of x (below 1.4) per
+    step on each side, 4 ulp of the largest v.  A step more or less moves the
+    fastest particles by dt |v| = 3e-4."""
+    rng = np.random.default_rng(11)
+    N, n = 700, (22, 21, 20)
+    dx = 1.0 / 16
+    scene = gpu.Scene(n, dx, 2e-4, (0.0, 0.0, 0.0), (0.0, 0.0, 0.0), 0, 0, 0)
+    st = _scene_state(rng, N, n, dx, margin=4.0)
+    mats = [gpu.createElasticMaterial(1000.0, 0.0, 0.3)]
+    outs = []
+    for graph in (1, 0):
+        sim = gpu.Simulator([scene], [N], mats, sparse_tiles=2048 if sparse else None)
+        sim.set_tuning(use_graph=graph)
+        sim.upload(st["x"], st["v"], st["C"], st["F"], st["m"], st["V0"])
+        for k in calls:
+            sim.step(k)
+        assert sim.status() == 0
+        assert sim.metrics()["total_steps"] == sum(calls)
+        outs.append(sim.download())
+    ulps = sum(calls) * 2.0 ** -23
+    assert np.abs(outs[0]["x"] - outs[1]["x"]).max() <= 1.4 * ulps + 1e-6
+    assert np.abs(outs[0]["v"] - outs[1]["v"]).max() <= (4 * ulps + 1e-6) * np.abs(outs[1]["v"]).max()
+
+
 @pytest.mark.parametrize("counts", [[1], [64], [1, 0, 3], [700], [5, 900, 2, 1, 40], [2000, 1]])
 @pytest.mark.parametrize("sparse", [False, True])
 def test_p2g_of_uneven_cells_equals_thread_per_cell(gpu, counts, sparse):
