@@ -43,7 +43,9 @@ struct pgmpm_hashgrid_s {
     bool built = false;
     DevBuf counts, starts;          // per cell
     DevBuf cell_ids;                // per particle: cell id (particle order)
-    DevBuf ka, va, kb, vb, scratch, pos_stage;  // sort buffers; va keeps the sorted particle indices
+    // sort buffers; between builds va keeps the sorted particle indices, ka and
+    // vb are the dense queries' (dense_index, the queries' cells)
+    DevBuf ka, va, kb, vb, scratch, pos_stage;
     DevBuf qcount, qstage, qout_stage, scan_tmp, stats;  // query scratch, kept between calls
     // dense queries (cells in grid order, x outer, z inner): z stretches and
     // block sums for the last half width and first[] of the cells' buckets (one
@@ -52,6 +54,7 @@ struct pgmpm_hashgrid_s {
     uint2* grid_rows() const { return grid_tables.as<uint2>(); }
     uint32_t* grid_sum() const { return reinterpret_cast<uint32_t*>(grid_rows() + total); }
     uint32_t* grid_first() const { return grid_sum() + total; }
+    uint32_t* dense_index() const { return mult_max > 1 ? grid_index.as<uint32_t>() : vb.as<uint32_t>(); }
     uint32_t mult_max = 0;    // most cells that hash to one bucket (0: not counted yet)
     bool grid_ready = false;  // grid_first and grid_index hold the last build's
     int64_t sum_src = -1;     // grid_rows and grid_sum hold the last build's for this half width
@@ -472,8 +475,10 @@ int dense_tables(pgmpm_hashgrid_s* g, const HGDev& G, uint32_t src, cudaStream_t
         CK(cudaMemcpyAsync(&g->mult_max, g->stats.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
     }
+    // with a cell per bucket the copy is as long as the particles, and takes a
+    // buffer of the build's sort (a new grid's first query 100 us less to allocate)
     if (g->mult_max > HG_DENSE_MULT || g->n * g->mult_max > 0xFFFFFFFFll ||
-        !have(g->grid_index.ensure(sizeof(uint32_t) * std::max<size_t>((size_t)g->n * g->mult_max, 1))))
+        (g->mult_max > 1 && !have(g->grid_index.ensure(sizeof(uint32_t) * std::max<size_t>((size_t)g->n * g->mult_max, 1)))))
         return 0;
     uint32_t* first = g->grid_first();
     if (!g->grid_ready) {
@@ -481,7 +486,7 @@ int dense_tables(pgmpm_hashgrid_s* g, const HGDev& G, uint32_t src, cudaStream_t
         int64_t* bsum = g->scan_tmp.as<int64_t>();
         k_hg_grid<<<nb, HG_T, 0, st>>>(G, g->counts.as<uint32_t>(), g->starts.as<uint32_t>(), sum, cstart);
         CK(exclusive_scan(sum, (int64_t)cells, bsum, first, st));
-        k_hg_expand<<<nb, HG_T, 0, st>>>(g->total, first, cstart, g->va.as<uint32_t>(), g->grid_index.as<uint32_t>());
+        k_hg_expand<<<nb, HG_T, 0, st>>>(g->total, first, cstart, g->va.as<uint32_t>(), g->dense_index());
     }
     if (!g->grid_ready || g->sum_src != (int64_t)src) {
         k_hg_rows<<<nb, HG_T, 0, st>>>(G, src, first, g->grid_rows());
@@ -637,10 +642,12 @@ int pgmpm_hashgrid_neighbors(pgmpm_hashgrid g, const float* queries, int64_t nq,
     const float* q = staged(g->qstage, queries, 3 * nq, ptr_kind, st, rc);
     if (rc) return rc;
     const HGDev G = dev_of(g);
-    CK(g->qcount.ensure(2 * sizeof(uint32_t) * std::max<int64_t>(nq, 1)));  // counts, then the queries' cells
+    // counts, then the queries' cells, unless those fit a buffer of the build's sort
+    const bool reuse = nq <= g->max_particles;
+    CK(g->qcount.ensure((reuse ? 1 : 2) * sizeof(uint32_t) * std::max<int64_t>(nq, 1)));
     const int64_t nb = std::max<int64_t>(1, (nq + SCAN_TILE - 1) / SCAN_TILE);
     const size_t off_bytes = sizeof(int64_t) * (size_t)(nq + 1);
-    uint32_t *qcount = g->qcount.as<uint32_t>(), *qcell = qcount + nq;
+    uint32_t *qcount = g->qcount.as<uint32_t>(), *qcell = reuse ? g->ka.as<uint32_t>() : qcount + nq;
     bool dense = false;
     if (nq > 0 && (int64_t)g->total <= HG_DENSE_CELLS * nq && g->total < 0x80000000u) {
         rc = dense_tables(g, G, src, st);
@@ -668,7 +675,7 @@ int pgmpm_hashgrid_neighbors(pgmpm_hashgrid g, const float* queries, int64_t nq,
     auto fill = [&](uint32_t* dout, int64_t cap) {
         auto dfill = [&](auto kernel, int qw) {
             kernel<<<(int)std::min<int64_t>(blocks_of(nq, qw * (HG_T / 32)), 148 * 64), HG_T, 0, st>>>(
-                G, q, nq, src, first, g->grid_rows(), g->grid_index.as<uint32_t>(), qcell,
+                G, q, nq, src, first, g->grid_rows(), g->dense_index(), qcell,
                 doff, cap, dout);
         };
         if (dense && src <= 1)  // 1 or 9 stretches per query
