@@ -295,9 +295,9 @@ int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
     // whole call of up to 64 steps the third time in a row a call has that many
     // (one such graph is kept), and 16 steps at a time inside calls of 128 and
     // more.  50 steps of 32,768 particles 1303 -> 1163 us, 5 of 4,096 150 -> 138,
-    // 20 of 2 M 4925 -> 4853.  Making a graph takes tens of us, so the first four
+    // 20 of 2 M 4925 -> 4853.  Making a graph takes tens of us, so the first eight
     // steps of each kind and place are launched kernel by kernel: the first call
-    // of 5 steps of a new 4,096-particle solver 407 -> 194 us, of 50 steps of
+    // of 5 steps of a new 4,096-particle solver 407 -> 182 us, of 50 steps of
     // 32,768 1455 -> 1354.
     const bool spans = s->use_graph && !s->profiling && !s->fused();
     if (spans && n_steps > 1 && n_steps <= s->kCallSteps) {

@@ -148,7 +148,7 @@ struct pgmpm_solver_s {
     cudaGraphExec_t step_exec[pgmpm::STEP_KINDS][4] = {};
     cudaGraph_t step_graph[pgmpm::STEP_KINDS][4] = {};
     int step_seen[pgmpm::STEP_KINDS][4] = {};  // such steps launched without a graph
-    static constexpr int kDirectSteps = 4;
+    static constexpr int kDirectSteps = 8;
     // several split steps in one graph (run_steps): all steps of a call, and
     // kMidSteps steps with others of their call before and after them
     static constexpr int kCallSteps = 64, kCallRepeats = 3, kMidSteps = 16, kMidAtLeast = 128;
