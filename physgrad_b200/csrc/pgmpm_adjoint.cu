@@ -65,7 +65,11 @@ __global__ void k_adj_grid(View V, AdjView A) {
 // z-slices of the stencil are a rolled loop, so that 18 loads instead of 54 are
 // in flight and four blocks of 128 registers fit an SM: 262,144 particles 44.0
 // -> 42.6 us, 8 scenes of 30,000: 38.8 -> 35.7 us (unrolled at 3 blocks: 168
-// registers; rolled at 3 and 5 blocks 44.9 / 38.6 and 47.6 / 36.5).
+// registers; rolled at 3 and 5 blocks 44.9 / 38.6 and 47.6 / 36.5).  The
+// adjoint it computes is the next scatter's input: forming that scatter's payload
+// here, from registers and three planes of the state before, adds 4.8 / 4.4 us and
+// saves a kernel of 9.5 / 6.3 us that read six more planes (forward + backward of
+// 48 steps of 262,144 particles 6604 -> 6432 us).
 constexpr int GATHER_T = 128;
 constexpr int MAX_SMEM_MATS = 64;
 
@@ -275,6 +279,13 @@ __global__ void __launch_bounds__(GATHER_T, 4) k_adj_gather(View V, AdjView A) {
         A.g[3 * N + p] = g3;
         A.g[4 * N + p] = g4;
         A.g[5 * N + p] = g5;
+        if (A.q_prev) {  // the payload of the step before this one, whose reverse is next
+            float xp[3], Fp[9], b[3], Ad[9];
+            Stencil sp;
+            unpack_xF(A.q_prev[p], A.q_prev[N + p], A.q_prev[2 * N + p], xp, Fp);
+            adj_payload_of<FLUID>(sc, xp, Fp, C, FLUID && mt.model == MODEL_EOS, ox, oF, ogv, oC, sp, flags, b, Ad);
+            store_adj_payload(A.pay, N, p, sp, b, Ad);
+        }
         if (smem_e) {
             // lanes of one material combine before one shared atomic
             const unsigned peers = __match_any_sync(__activemask(), mid);

@@ -707,4 +707,43 @@ __device__ __forceinline__ uint32_t apply_bc(const SceneDev& sc, int i, int j, i
     return zeroed;
 }
 
+// Reverse of G2P for one particle (MLS): the scatter payload of dL/dv_i
+// and dL/dm_i contributions, node o gets w_o (b + Ad o).  x, F: state before the
+// step; Cn: C after it (eos: the EOS reset follows the F update); gx, gF, gv, gC:
+// adjoint of the state after it.  Also fills the stencil (f, w) of x.
+template <bool FLUID>
+__device__ __forceinline__ void adj_payload_of(const SceneDev& sc, const float x[3], const float F[9],
+                                               const float Cn[9], bool eos, const float gx[3], float gF[9],
+                                               const float gv[3], const float gC[9], Stencil& st, uint32_t& flags,
+                                               float b[3], float Ad[9]) {
+    make_stencil<PHYS_MLS>(sc, x, st, flags);
+    if (FLUID && eos) {
+        float M[9], Fr[9], cof[9];
+#pragma unroll
+        for (int a = 0; a < 9; ++a) M[a] = sc.dt * Cn[a] + ((a % 4 == 0) ? 1.f : 0.f);
+        m3_mul(M, F, Fr);
+        m3_cof(Fr, cof);
+        const float J = Fr[0] * cof[0] + Fr[1] * cof[1] + Fr[2] * cof[2];
+        const float cc = cbrtf(J) / (3.f * J) * (gF[0] + gF[4] + gF[8]);
+#pragma unroll
+        for (int a = 0; a < 9; ++a) gF[a] = cc * cof[a];
+    }
+    float gFFt[9];
+    m3_mulT(gF, F, gFFt);
+    const float sD = sc.D * sc.dx;
+#pragma unroll
+    for (int a = 0; a < 9; ++a) Ad[a] = sD * (gC[a] + sc.dt * gFFt[a]);
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+        b[a] = (gv[a] + sc.dt * gx[a]) - (Ad[3 * a] * st.f[0] + Ad[3 * a + 1] * st.f[1] + Ad[3 * a + 2] * st.f[2]);
+}
+// in the layout of the P2G payload, without a mass
+__device__ __forceinline__ void store_adj_payload(float4* pay, int64_t N, int64_t p, const Stencil& st, const float b[3],
+                                                  const float Ad[9]) {
+    pay[p] = make_float4(b[0], b[1], b[2], 0.f);
+    pay[N + p] = make_float4(Ad[0], Ad[1], Ad[2], Ad[3]);
+    pay[2 * N + p] = make_float4(Ad[4], Ad[5], Ad[6], Ad[7]);
+    pay[3 * N + p] = make_float4(Ad[8], st.f[0], st.f[1], st.f[2]);
+}
+
 }  // namespace pgmpm

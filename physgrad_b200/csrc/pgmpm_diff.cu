@@ -219,6 +219,7 @@ int record_tape_forward(pgmpm_solver s, int len, cudaStream_t st, int t = 0, int
 // Reverse kernels of slots len-1 .. 0 of tape set t.
 int record_tape_reverse(pgmpm_solver s, const AdjView& A0, int len, cudaStream_t st, int t = 0, int g0 = -1) {
     AdjView A = A0;
+    A.q_prev = nullptr;
     for (int j = len - 1; j >= 0; --j) {
         StepBufs b = tape_bufs(s, j, t, g0 < 0 ? -1 : g0 + j);
         View V = s->view_for(b);
@@ -226,6 +227,9 @@ int record_tape_reverse(pgmpm_solver s, const AdjView& A0, int len, cudaStream_t
         V.early = true;
         V.early_first = j < len - 1;  // after the previous slot's gather
         A.q_next = b.q_out;
+        A.pay_ready = A.q_prev != nullptr;  // by the previous slot's gather
+        A.q_prev = j > 0 && adj_scatter_from_payload(V, s->tune) ? tape_bufs(s, j - 1, t, g0 < 0 ? -1 : g0 + j - 1).q
+                                                                 : nullptr;
         // the slot's P2G work cursor is zero: the grid update of the slot's
         // forward step cleared it after P2G (and a previous reverse's grid
         // adjoint after its scatter)

@@ -316,10 +316,14 @@ struct AdjView {
     float4* g;                 // 6 planes
     const float4* q_next;      // state after the step (C' for the F update and the fluid reset)
     float4* pay;               // the scatter's payload (4 planes of N float4)
+    bool pay_ready;            // pay holds this step's already
+    const float4* q_prev;      // state before the step before: the gather forms that step's payload (or null)
     float4* grid_gv;           // (0, dL/dv_i) scatter target, zeroed by the grid adjoint
     float4* grid_gpm;          // (dL/dp_i, dL/dm_i) per node
     float* gE;                 // [M] dL/dE accumulators
 };
+// launch_adj_scatter runs from A.pay (P2G variants 4 and 5 with the bin sort)
+inline bool adj_scatter_from_payload(const View& V, const Tuning& t) { return t.p2g_variant >= 4 && V.cell_range; }
 cudaError_t launch_adj_scatter(const View& V, const AdjView& A, const PhysFlags& pf, const Tuning& t, int num_sms,
                                cudaStream_t st);
 cudaError_t launch_adj_grid(const View& V, const AdjView& A, const Tuning& t, int num_sms, cudaStream_t st);

@@ -555,42 +555,18 @@ __global__ void __launch_bounds__(P2G_T, 3) k_p2g_tiles(View V, AdjView AV) {
     if (flags) atomicOr(&V.counters[CNT_FLAGS], flags);
 }
 
-// Reverse of G2P for one particle (MLS): the scatter payload of dL/dv_i
-// and dL/dm_i contributions, node o gets w_o (b + Ad o).  Also fills the
-// stencil (f, w) of the particle's position.
+// adj_payload_of for particle p of the step V, AV describe.
 template <bool MULTI, bool FLUID>
 __device__ __forceinline__ void adj_payload(const View& V, const AdjView& AV, const SceneDev& sc, int64_t p,
                                             Stencil& st, uint32_t& flags, float b[3], float Ad[9]) {
     const int64_t N = V.N;
-    const float4 q0 = V.q[p];
-    const float x[3] = {q0.x, q0.y, q0.z};
-    make_stencil<PHYS_MLS>(sc, x, st, flags);
-    const float4 q1 = V.q[N + p], q2 = V.q[2 * N + p];
-    float xx[3], F[9];
-    unpack_xF(q0, q1, q2, xx, F);
-    float gx[3], gF[9], gv[3], gC[9];
+    float x[3], F[9], gx[3], gF[9], gv[3], gC[9], Cn[9], vdum[3];
+    unpack_xF(V.q[p], V.q[N + p], V.q[2 * N + p], x, F);
     unpack_xF(AV.g[p], AV.g[N + p], AV.g[2 * N + p], gx, gF);
     unpack_vC(AV.g[3 * N + p], AV.g[4 * N + p], AV.g[5 * N + p], gv, gC);
-    if (FLUID && V.mats[MULTI ? V.mat[p] : 0].model == MODEL_EOS) {
-        float Cn[9], vdum[3], M[9], Fr[9], cof[9];
-        unpack_vC(AV.q_next[3 * N + p], AV.q_next[4 * N + p], AV.q_next[5 * N + p], vdum, Cn);
-#pragma unroll
-        for (int a = 0; a < 9; ++a) M[a] = sc.dt * Cn[a] + ((a % 4 == 0) ? 1.f : 0.f);
-        m3_mul(M, F, Fr);
-        m3_cof(Fr, cof);
-        const float J = Fr[0] * cof[0] + Fr[1] * cof[1] + Fr[2] * cof[2];
-        const float cc = cbrtf(J) / (3.f * J) * (gF[0] + gF[4] + gF[8]);
-#pragma unroll
-        for (int a = 0; a < 9; ++a) gF[a] = cc * cof[a];
-    }
-    float gFFt[9];
-    m3_mulT(gF, F, gFFt);
-    const float sD = sc.D * sc.dx;
-#pragma unroll
-    for (int a = 0; a < 9; ++a) Ad[a] = sD * (gC[a] + sc.dt * gFFt[a]);
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-        b[a] = (gv[a] + sc.dt * gx[a]) - (Ad[3 * a] * st.f[0] + Ad[3 * a + 1] * st.f[1] + Ad[3 * a + 2] * st.f[2]);
+    const bool eos = FLUID && V.mats[MULTI ? V.mat[p] : 0].model == MODEL_EOS;
+    if (eos) unpack_vC(AV.q_next[3 * N + p], AV.q_next[4 * N + p], AV.q_next[5 * N + p], vdum, Cn);
+    adj_payload_of<FLUID>(sc, x, F, Cn, eos, gx, gF, gv, gC, st, flags, b, Ad);
 }
 
 // Sum of the contributions to node (nx, ny, nz) of the 6^3 node block of a
@@ -1128,7 +1104,8 @@ __global__ void __launch_bounds__(P2GS_T, P2GS_BLOCKS) k_p2g_slices(View V) {
 // + scatter: 262,144 particles 39 -> 7.3 + 22.9 us, 8 scenes of 30,000: 46 ->
 // 6.5 + 21.4 us; the scatter at 3 and 5 blocks per SM 23.4 / 26.3 and 21.9 /
 // 23.3.  The payload is bound by memory (5.4 TB/s at 262,144 particles, much of
-// it L2 hits).
+// it L2 hits).  Launched for a segment's last step only: every other step's
+// payload comes from the reverse gather of the step after it.
 template <bool MULTI, bool FLUID>
 __global__ void __launch_bounds__(128) k_adj_payload(View V, AdjView AV) {
     step_wait();
@@ -1139,10 +1116,7 @@ __global__ void __launch_bounds__(128) k_adj_payload(View V, AdjView AV) {
     Stencil st;
     float b[3], Ad[9];
     adj_payload<MULTI, FLUID>(V, AV, scene_ref(V, scene_of_particle(V, p)), p, st, flags, b, Ad);
-    AV.pay[p] = make_float4(b[0], b[1], b[2], 0.f);
-    AV.pay[N + p] = make_float4(Ad[0], Ad[1], Ad[2], Ad[3]);
-    AV.pay[2 * N + p] = make_float4(Ad[4], Ad[5], Ad[6], Ad[7]);
-    AV.pay[3 * N + p] = make_float4(Ad[8], st.f[0], st.f[1], st.f[2]);
+    store_adj_payload(AV.pay, N, p, st, b, Ad);
     if (flags) atomicOr(&V.counters[CNT_FLAGS], flags);
 }
 
@@ -2068,14 +2042,18 @@ cudaError_t launch_adj_scatter(const View& V, const AdjView& A, const PhysFlags&
                                cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
     if (pf.physics != PHYS_MLS) return cudaErrorNotSupported;
-    if (t.p2g_variant >= 4 && V.cell_range) {  // three threads per cell over the sort's cell table
+    if (adj_scatter_from_payload(V, t)) {  // three threads per cell over the sort's cell table
         auto payload = pf.multi_mat ? (pf.has_fluid ? k_adj_payload<true, true> : k_adj_payload<true, false>)
                                     : (pf.has_fluid ? k_adj_payload<false, true> : k_adj_payload<false, false>);
-        const cudaError_t e = launch_after(V.early_first, payload, (int)((V.N + 127) / 128), 128, st, V, A);
-        if (e != cudaSuccess) return e;
+        bool early = V.early_first;
+        if (!A.pay_ready) {
+            const cudaError_t e = launch_after(early, payload, (int)((V.N + 127) / 128), 128, st, V, A);
+            if (e != cudaSuccess) return e;
+            early = V.early;
+        }
         View S = V;
         S.pay = A.pay;
-        return launch_after(V.early, k_p2g_slices<false, true>, num_sms * P2GS_BLOCKS, P2GS_T, st, S);
+        return launch_after(early, k_p2g_slices<false, true>, num_sms * P2GS_BLOCKS, P2GS_T, st, S);
     }
     if (t.p2g_variant >= 2) {  // the adjoint scatter of variant 3 (and of 4 without a cell table) is variant 2's
         const int nb = num_sms * t.cell_blocks_per_sm;
