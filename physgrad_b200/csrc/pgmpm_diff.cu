@@ -404,19 +404,27 @@ int pgmpm_forward_checkpointed(pgmpm_solver s, int32_t n_steps, int32_t checkpoi
     // (the tape starts from the state and its payload, with grid_mp clear).
     // g0 >= 0: the recorded forward's steps g0 .. (the record's keys g0 are
     // the state's already)
-    auto run_in_tape = [&](int len, int t, int g0) -> int {
+    // q_from, keys_from: the state to start from.  Only the last segment hands its
+    // state back to the live buffers; the one before it is followed by the last,
+    // which starts from its tape (7 copies of 5 us less).
+    auto run_in_tape = [&](int len, int t, int g0, const float4* q_from, const uint32_t* keys_from) -> int {
         int r = unprime(s, st);
         if (r) return r;
         const StepBufs first = tape_bufs(s, 0, t, g0);
-        CK(cudaMemcpyAsync(first.q, s->q.p, sizeof(float4) * 6 * N, cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(first.q, q_from, sizeof(float4) * 6 * N, cudaMemcpyDeviceToDevice, st));
         if (g0 < 0)
-            CK(cudaMemcpyAsync(first.keys_in, s->keys.p, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(s->tape_pay.p, s->pay.p, sizeof(float4) * 4 * N, cudaMemcpyDeviceToDevice, st));
+            CK(cudaMemcpyAsync(first.keys_in, keys_from, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, st));
+        if (q_from == s->q.as<float4>())  // the other set's last step left its payload there
+            CK(cudaMemcpyAsync(s->tape_pay.p, s->pay.p, sizeof(float4) * 4 * N, cudaMemcpyDeviceToDevice, st));
         const int kind = t == 0 ? 1 : 6;
         cudaGraphExec_t ex = nullptr;
         r = tape_graph(s, kind, len, g0, ex, [&](cudaStream_t cs) { return record_tape_forward(s, len, cs, t, g0); });
         if (r) return r;
         CK(cudaGraphLaunch(ex, st));
+        s->met.total_steps += len;
+        CK(launch_merge_flags(s->tape_counters.as<uint32_t>() + (size_t)CNT_WORDS * (g0 >= 0 ? g0 : s->tape_slots * t),
+                              len, s->counters.as<uint32_t>(), st));
+        if (t == 1) return PGMPM_OK;  // the last segment follows, and starts from this set's last state
         const StepBufs last = tape_bufs(s, len - 1, t, g0);
         CK(cudaMemcpyAsync(s->q.p, last.q_out, sizeof(float4) * 6 * N, cudaMemcpyDeviceToDevice, st));
         CK(cudaMemcpyAsync(s->keys.p, last.keys_out, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, st));
@@ -427,9 +435,6 @@ int pgmpm_forward_checkpointed(pgmpm_solver s, int32_t n_steps, int32_t checkpoi
                            cudaMemcpyDeviceToDevice, st));
         CK(cudaMemcpyAsync(s->counters.as<uint32_t>() + CNT_ACTIVE, last.counters + CNT_ACTIVE, 2 * sizeof(uint32_t),
                            cudaMemcpyDeviceToDevice, st));
-        CK(launch_merge_flags(s->tape_counters.as<uint32_t>() + (size_t)CNT_WORDS * (g0 >= 0 ? g0 : s->tape_slots * t),
-                              len, s->counters.as<uint32_t>(), st));
-        s->met.total_steps += len;
         return PGMPM_OK;
     };
     // with two tape sets (the overlapped backward) the second-to-last
@@ -439,10 +444,12 @@ int pgmpm_forward_checkpointed(pgmpm_solver s, int32_t n_steps, int32_t checkpoi
     // steps read and write the record's
     uint32_t* rk = rec ? s->rec_keys.as<uint32_t>() : nullptr;
     if (rec) CK(cudaMemcpyAsync(rk, s->keys.p, sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, st));
+    const float4* q_now = s->q.as<float4>();
+    const uint32_t* keys_now = s->keys.as<uint32_t>();
     for (int seg = 0; seg < nseg; ++seg) {
-        CK(cudaMemcpyAsync(s->ck_q.as<float4>() + 6 * N * seg, s->q.p, sizeof(float4) * 6 * N,
+        CK(cudaMemcpyAsync(s->ck_q.as<float4>() + 6 * N * seg, q_now, sizeof(float4) * 6 * N,
                            cudaMemcpyDeviceToDevice, st));
-        CK(cudaMemcpyAsync(s->ck_keys.as<uint32_t>() + N * seg, rec ? rk + N * (size_t)seg * k : s->keys.as<uint32_t>(),
+        CK(cudaMemcpyAsync(s->ck_keys.as<uint32_t>() + N * seg, rec ? rk + N * (size_t)seg * k : keys_now,
                            sizeof(uint32_t) * N, cudaMemcpyDeviceToDevice, st));
         const int len = std::min(k, n_steps - seg * k);
         if (s->N == 0 || seg + 2 < nseg || (seg + 2 == nseg && !prev_in_tape)) {
@@ -451,12 +458,16 @@ int pgmpm_forward_checkpointed(pgmpm_solver s, int32_t n_steps, int32_t checkpoi
             continue;
         }
         const int t = seg + 1 == nseg ? 0 : 1;
-        rc = run_in_tape(len, t, rec ? seg * k : -1);
+        rc = run_in_tape(len, t, rec ? seg * k : -1, q_now, keys_now);
         if (rc) return rc;
-        if (t == 0)
+        if (t == 0) {
             s->tape_has_last = true;
-        else
+        } else {
             s->tape_has_prev = true;
+            const StepBufs last = tape_bufs(s, len - 1, t, rec ? seg * k : -1);
+            q_now = last.q_out;
+            keys_now = last.keys_out;
+        }
     }
     s->ck_steps = n_steps;
     s->ck_every = k;
