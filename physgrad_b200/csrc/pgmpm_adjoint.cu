@@ -64,7 +64,7 @@ __global__ void k_adj_grid(View V, AdjView A) {
 // by the latency of the node loads at the occupancy its registers leave.  The
 // z-slices of the stencil are a rolled loop, so that 18 loads instead of 54 are
 // in flight and four blocks of 128 registers fit an SM: 262,144 particles 44.0
-// -> 42.6 us, 8 scenes of 30,000: 38.8 -> 35.7 us (unrolled at 3 blocks: 168
+// -> 42.6 us, 12 scenes of together 178 K: 38.8 -> 35.7 us (unrolled at 3 blocks: 168
 // registers; rolled at 3 and 5 blocks 44.9 / 38.6 and 47.6 / 36.5).  The
 // adjoint it computes is the next scatter's input: forming that scatter's payload
 // here, from registers and three planes of the state before, adds 4.8 / 4.4 us and

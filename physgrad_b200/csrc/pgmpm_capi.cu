@@ -301,7 +301,7 @@ int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
     // 32,768 1455 -> 1354.
     const bool spans = s->use_graph && !s->profiling && !s->fused();
     if (spans && n_steps > 1 && n_steps <= s->kCallSteps) {
-        s->call_seen = n_steps == s->call_last ? s->call_seen + 1 : 1;
+        s->call_seen = n_steps == s->call_last ? std::min(s->call_seen + 1, (int)s->kCallRepeats) : 1;
         s->call_last = n_steps;
         if (s->call_steps != n_steps && s->call_seen >= s->kCallRepeats) {
             s->call_steps = 0;
@@ -352,7 +352,7 @@ int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
             }
             CK(cudaGraphLaunch(s->step_exec[kind][place], st));
         } else {
-            s->step_seen[kind][place]++;
+            if (s->step_seen[kind][place] < s->kDirectSteps) s->step_seen[kind][place]++;
             const bool ahead = s->counts_ahead() && kind == STEP_SPLIT;
             int rc = record_step(s, s->live_bufs(), st, false, k + 1 == n_steps, kind, ahead && k > 0,
                                  ahead && k + 1 < n_steps);

@@ -1120,7 +1120,7 @@ __global__ void __launch_bounds__(P2GS_T, P2GS_BLOCKS) k_p2g_slices(View V) {
 // whole thread's registers and the state and adjoint planes, read once and in
 // order here.  Formed inside the scatter instead (a lane per balanced particle
 // run, the former kernel) it held the walk to 12 warps an SM.  Before -> payload
-// + scatter: 262,144 particles 39 -> 7.3 + 22.9 us, 8 scenes of 30,000: 46 ->
+// + scatter: 262,144 particles 39 -> 7.3 + 22.9 us, 12 scenes of together 178 K: 46 ->
 // 6.5 + 21.4 us; the scatter at 3 and 5 blocks per SM 23.4 / 26.3 and 21.9 /
 // 23.3.  The payload is bound by memory (5.4 TB/s at 262,144 particles, much of
 // it L2 hits).  Launched for a segment's last step only: every other step's
@@ -2072,7 +2072,8 @@ cudaError_t launch_adj_scatter(const View& V, const AdjView& A, const PhysFlags&
         }
         View S = V;
         S.pay = A.pay;
-        return launch_after(early, slices_ahead(V.N) ? k_p2g_slices<false, true, true> : k_p2g_slices<false, true, false>, num_sms * P2GS_BLOCKS, P2GS_T, st, S);
+        return launch_after(early, slices_ahead(V.N) ? k_p2g_slices<false, true, true> : k_p2g_slices<false, true, false>,
+                            num_sms * P2GS_BLOCKS, P2GS_T, st, S);
     }
     if (t.p2g_variant >= 2) {  // the adjoint scatter of variant 3 (and of 4 without a cell table) is variant 2's
         const int nb = num_sms * t.cell_blocks_per_sm;

@@ -28,8 +28,8 @@ constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
 constexpr int RS_MAXD = 256;
 static_assert(RS_TILE == RADIX_TILE && RS_MAXD == RADIX_MAX_DIGITS, "scratch sizing must match the kernels");
 
-__global__ void __launch_bounds__(RS_THREADS) rs_hist(const uint32_t* keys, int64_t n, int shift, int bits, uint32_t* hist,
-                                                      int nblocks) {
+__global__ void __launch_bounds__(RS_THREADS) rs_hist(const uint32_t* keys, int64_t n, int shift, int bits,
+                                                      uint32_t* hist, int nblocks) {
     step_wait();
     // warp-private histograms with native integer shared atomics, summed at the end
     __shared__ uint32_t cnt[RS_WARPS][RS_MAXD];
