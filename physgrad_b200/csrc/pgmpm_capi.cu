@@ -956,6 +956,12 @@ int pgmpm_set_step_sort(pgmpm_solver s, int32_t kind) {
         int rc = alloc_bin_sort(s);
         if (rc) return rc;
     }
+    if (kind != s->tune.step_sort) {
+        // each sort lists a step's tiles in buffers of its own: the segments a
+        // forward left on the tape (and a record of its sorts) hold the other
+        // sort's, so the backward replays every segment from its checkpoint
+        s->tape_has_last = s->tape_has_prev = s->ck_rec = false;
+    }
     s->tune.step_sort = kind;
     s->drop_graph();
     return PGMPM_OK;

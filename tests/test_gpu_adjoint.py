@@ -636,3 +636,39 @@ def test_backward_after_a_sort_or_kernel_change_replays_every_segment(gpu, chang
         print(f"{change} d/d{key}: {np.abs(a - b).max() / scale:.2e}, second backward {np.abs(a2 - b).max() / scale:.2e}")
         assert np.abs(a - b).max() <= 1e-4 * scale, key
         assert np.abs(a2 - b).max() <= 1e-4 * scale, key
+
+
+@pytest.mark.parametrize("record", [0, 1])
+@pytest.mark.parametrize("bins_first", [True, False])
+def test_backward_after_a_sort_change_in_either_direction(gpu, record, bins_first):
+    """The step sort switched between the forward and its backward, bins to
+    radix and radix to bins (which allocates nothing: the bin sort's buffers
+    are the default's), the forward recorded or not (a radix forward never
+    is).  The forward left its last segments on the tape with the first
+    sort's tile lists; the backward replays them, and the gradients equal
+    those of a run without the switch (the bound of the other sort changes)."""
+    from physgrad_b200 import _capi as C
+    from physgrad_b200 import workloads as W
+
+    scenes, counts, mats, st, _ = W.two_material_drop(n_particles=20000, n=32, seed=31)
+    N = counts[0]
+    kinds = (C.SORT_BINS, C.SORT_RADIX) if bins_first else (C.SORT_RADIX, C.SORT_BINS)
+    grads = []
+    for switch in (True, False):
+        sim = gpu.Simulator(scenes, counts, mats)
+        sim.set_sort_record(record)
+        sim.set_step_sort(kinds[0])
+        sim.upload(st["x"], st["v"], None, None, st["m"], st["V0"], st["mat"])
+        sim.forward_checkpointed(20, 8)
+        out = sim.download()
+        go = {"x": (out["x"] - 0.5).astype(np.float32) / N, "v": (out["v"] / N).astype(np.float32)}
+        if switch:
+            sim.set_step_sort(kinds[1])
+        grads.append([sim.backward(go), sim.backward(go)])
+        assert sim.status() == 0
+    for key in ("x", "v", "C", "F", "E"):
+        b = np.asarray(grads[1][0][key]).ravel()
+        scale = np.abs(b).max()
+        assert scale > 0.0, key
+        for g in grads[0]:
+            assert np.abs(np.asarray(g[key]).ravel() - b).max() <= 1e-4 * scale, key
