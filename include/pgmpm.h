@@ -216,6 +216,8 @@ PGMPM_API int pgmpm_download_grid(pgmpm_solver s, int32_t scene, float* mass, fl
                         void* stream);
 
 /* ---- simulation ------------------------------------------------------------ */
+/* After an error the particles are at some point of the call (upload them
+ * again); the solver stays usable. */
 PGMPM_API int pgmpm_step(pgmpm_solver s, int32_t n_steps, void* stream);
 
 /* One host-buffer call: upload state, advance n_steps, download state.

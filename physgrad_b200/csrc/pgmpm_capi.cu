@@ -231,6 +231,25 @@ int unprime(pgmpm_solver s, cudaStream_t st) {
     return refresh_payload(s, st);
 }
 
+int settle(pgmpm_solver s, cudaStream_t st) {
+    if (!s->unsettled) return PGMPM_OK;
+    int rc = unprime(s, st);
+    if (rc) return rc;
+    CK(cudaMemsetAsync(s->grid_mp.p, 0, s->grid_mp.bytes, st));
+    CK(cudaMemsetAsync(s->counters.p, 0, sizeof(uint32_t) * CNT_RESET, st));
+    if (s->bs_ccount.p) {
+        CK(cudaMemsetAsync(s->bs_ccount.p, 0, s->bs_ccount.bytes, st));
+        CK(cudaMemsetAsync(s->bs_tcount.p, 0, s->bs_tcount.bytes, st));
+        CK(cudaMemsetAsync(s->bs_work.p, 0, s->bs_work.bytes, st));
+    }
+    if (s->adj_grid_gv.p) CK(cudaMemsetAsync(s->adj_grid_gv.p, 0, s->adj_grid_gv.bytes, st));
+    // under a capture nothing has run yet
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    s->unsettled = cs != cudaStreamCaptureStatusNone;
+    return PGMPM_OK;
+}
+
 }  // namespace pgmpm
 
 namespace {
@@ -280,12 +299,11 @@ int build_span(pgmpm_solver s, int steps, bool whole, cudaGraphExec_t& exec) {
 
 }  // namespace
 
-namespace pgmpm {
+namespace {
 // Live steps.  With the fused kernel a call leaves the next step's P2G in
 // grid_mp (s->primed), so a following call continues without a P2G of its
 // own; anything that changes the state or its parameters unprimes first.
-int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
-    if (!s->uploaded) return fail(PGMPM_ERR_STATE, "no particles uploaded");
+int live_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
     if (!s->fused()) {
         int rc = unprime(s, st);
         if (rc) return rc;
@@ -363,7 +381,17 @@ int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
     }
     return PGMPM_OK;
 }
+}  // namespace
 
+namespace pgmpm {
+int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
+    if (!s->uploaded) return fail(PGMPM_ERR_STATE, "no particles uploaded");
+    int rc = settle(s, st);
+    if (rc) return rc;
+    rc = live_steps(s, n_steps, st);
+    if (rc) s->unsettled = true;
+    return rc;
+}
 }  // namespace pgmpm
 
 // ============================================================== C-ABI
@@ -577,6 +605,7 @@ int pgmpm_create_ex(const pgmpm_scene_desc* scenes, int32_t n_scenes, const int6
     for (int i = 0; i < 6 && e == cudaSuccess; ++i) e = cudaEventCreate(&s->ev[i]);
     if (e == cudaSuccess) e = cudaMallocHost(&s->h_counters, sizeof(uint32_t) * CNT_WORDS);
     if (e != cudaSuccess) {
+        cudaGetLastError();
         delete s;
         return fail(e == cudaErrorMemoryAllocation ? PGMPM_ERR_OOM : PGMPM_ERR_CUDA, "create: %s",
                     cudaGetErrorString(e));
@@ -998,7 +1027,9 @@ int pgmpm_autotune(pgmpm_solver s, int32_t reps, void* stream) {
     DeviceGuard dg(s->device);
     cudaStream_t st = ST(stream);
     if (reps < 1) reps = 3;
-    int rc0 = unprime(s, st);  // the trials run split steps from the payload
+    int rc0 = settle(s, st);
+    if (rc0) return rc0;
+    rc0 = unprime(s, st);  // the trials run split steps from the payload
     if (rc0) return rc0;
     // save state (planes + keys) and restore after the trials
     DevBuf save;
@@ -1033,6 +1064,7 @@ int pgmpm_autotune(pgmpm_solver s, int32_t reps, void* stream) {
         CK(cudaEventElapsedTime(&ms, s->ev[0], s->ev[1]));
         return PGMPM_OK;
     };
+    s->unsettled = true;  // until the trials' state is restored
     // one real step so the sorted order, tile lists and grid velocity exist
     int rc = record_step(s, s->live_bufs(), st, false);
     if (rc) return rc;
@@ -1089,6 +1121,7 @@ int pgmpm_autotune(pgmpm_solver s, int32_t reps, void* stream) {
     rc = refresh_payload(s, st);
     if (rc) return rc;
     CK(cudaStreamSynchronize(st));
+    s->unsettled = false;
     s->tune = best;
     s->use_graph = keep_graph;
     s->profiling = keep_prof;

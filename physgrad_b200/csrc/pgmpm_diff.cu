@@ -397,6 +397,8 @@ int pgmpm_forward_checkpointed(pgmpm_solver s, int32_t n_steps, int32_t checkpoi
     s->ck_rec = false;
     s->tape_has_last = false;
     s->tape_has_prev = false;
+    rc = settle(s, st);
+    if (rc) return rc;
     rc = unprime(s, st);  // checkpoints and replays start from the state alone
     if (rc) return rc;
     // Runs a segment in the slots of tape set t, so that the backward does
@@ -489,6 +491,8 @@ int pgmpm_backward(pgmpm_solver s, const float* gx_out, const float* gv_out, con
     const size_t Nz = (size_t)std::max<int64_t>(N, 1);
     const int M = s->M;
     int rc = ensure_tape(s, s->ck_every);
+    if (rc) return rc;
+    rc = settle(s, st);
     if (rc) return rc;
     // the replays accumulate their P2G in grid_mp: drop a pending fused P2G
     // of the live state (recomputed by its next step)
@@ -605,11 +609,16 @@ bool launch_adj_grids(pgmpm_solver s, cudaStream_t st) {
 
 // One step on the caller's arrays (launch_ref_step).
 void launch_ref(pgmpm_solver s, const RefStep& R, cudaStream_t st, const char* who) {
+    if (settle(s, st)) return;
     const StepBufs b = s->live_bufs();
-    if (launch_ref_step(s->view_for(b), s->bin_sort_bufs(b), R, s->pf, s->tune, s->num_sms, st) != cudaSuccess)
-        fail(PGMPM_ERR_CUDA, "%s: %s", who, cudaGetErrorString(cudaGetLastError()));
-    else if (!R.gx)
+    const cudaError_t e = launch_ref_step(s->view_for(b), s->bin_sort_bufs(b), R, s->pf, s->tune, s->num_sms, st);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        s->unsettled = true;
+        fail(PGMPM_ERR_CUDA, "%s: %s", who, cudaGetErrorString(e));
+    } else if (!R.gx) {
         s->met.total_steps++;
+    }
 }
 
 // per-call dt into the scene table (the dt word only: gravity arrives as a

@@ -552,6 +552,7 @@ int pgmpm_hashgrid_create(float cell_size, const float* domain_min, const float*
     if (e == cudaSuccess) e = g->scratch.alloc(sizeof(uint32_t) * radix_sort_scratch_words((int64_t)n));
     if (e == cudaSuccess) e = g->stats.alloc(sizeof(unsigned long long) * 3);
     if (e != cudaSuccess) {
+        cudaGetLastError();
         delete g;
         return fail(e == cudaErrorMemoryAllocation ? PGMPM_ERR_OOM : PGMPM_ERR_CUDA, "hashgrid: %s",
                     cudaGetErrorString(e));

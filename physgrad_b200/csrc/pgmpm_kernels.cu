@@ -2053,8 +2053,7 @@ cudaError_t launch_payload(const View& V, const PhysFlags& pf, cudaStream_t st) 
 
 cudaError_t launch_mark(const View& V, cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
-    k_mark<<<grid_for(V.N, 256), 256, 0, st>>>(V);
-    return cudaGetLastError();
+    return launch_after(false, k_mark, grid_for(V.N, 256), 256, st, V);
 }
 
 cudaError_t launch_adj_scatter(const View& V, const AdjView& A, const PhysFlags& pf, const Tuning& t, int num_sms,
@@ -2114,46 +2113,42 @@ cudaError_t launch_p2g(const View& V, const PhysFlags& pf, const Tuning& t, int 
                                          : slices_ahead(V.N) ? k_p2g_slices<false, false, true>
                                                              : k_p2g_slices<false, false, false>,
                                 num_sms * min(P2GS_BLOCKS, t.pair_blocks_per_sm), P2GS_T, st, V);
-        k_p2g_pairs<<<num_sms * t.pair_blocks_per_sm, P2GP_T, 0, st>>>(V);
-        return cudaGetLastError();
+        return launch_after(false, k_p2g_pairs, num_sms * t.pair_blocks_per_sm, P2GP_T, st, V);
     }
     if (t.p2g_variant >= 2) {  // REF physics: variants 3 to 5 run variant 2
         const int nb = num_sms * t.cell_blocks_per_sm;
         const AdjView none{};
         if (pf.physics == PHYS_MLS) {
             if (pf.multi_mat)
-                k_p2g_cells<MODE_MLS, true, false><<<nb, P2GC_T, 0, st>>>(V, none);
+                return launch_after(false, k_p2g_cells<MODE_MLS, true, false>, nb, P2GC_T, st, V, none);
             else
-                k_p2g_cells<MODE_MLS, false, false><<<nb, P2GC_T, 0, st>>>(V, none);
+                return launch_after(false, k_p2g_cells<MODE_MLS, false, false>, nb, P2GC_T, st, V, none);
         } else {
-            k_p2g_cells<MODE_REF, false, false><<<nb, P2GC_T, 0, st>>>(V, none);
+            return launch_after(false, k_p2g_cells<MODE_REF, false, false>, nb, P2GC_T, st, V, none);
         }
-        return cudaGetLastError();
     }
     if (t.p2g_variant == 0) {
         const int nb = num_sms * t.tile_blocks_per_sm;
         const AdjView none{};
         if (pf.physics == PHYS_MLS) {
             if (pf.multi_mat)
-                k_p2g_tiles<MODE_MLS, true, false><<<nb, P2G_T, 0, st>>>(V, none);
+                return launch_after(false, k_p2g_tiles<MODE_MLS, true, false>, nb, P2G_T, st, V, none);
             else
-                k_p2g_tiles<MODE_MLS, false, false><<<nb, P2G_T, 0, st>>>(V, none);
+                return launch_after(false, k_p2g_tiles<MODE_MLS, false, false>, nb, P2G_T, st, V, none);
         } else {
-            k_p2g_tiles<MODE_REF, false, false><<<nb, P2G_T, 0, st>>>(V, none);
+            return launch_after(false, k_p2g_tiles<MODE_REF, false, false>, nb, P2G_T, st, V, none);
         }
-        return cudaGetLastError();
     }
     const int64_t nb = (V.N + t.ppt - 1) / t.ppt;
     if (nb > 0x7FFFFFFF) return cudaErrorInvalidValue;
     if (pf.physics == PHYS_MLS) {
         if (pf.multi_mat)
-            k_p2g<PHYS_MLS, true><<<(int)nb, t.p2g_block, 0, st>>>(V, t.ppt);
+            return launch_after(false, k_p2g<PHYS_MLS, true>, (int)nb, t.p2g_block, st, V, t.ppt);
         else
-            k_p2g<PHYS_MLS, false><<<(int)nb, t.p2g_block, 0, st>>>(V, t.ppt);
+            return launch_after(false, k_p2g<PHYS_MLS, false>, (int)nb, t.p2g_block, st, V, t.ppt);
     } else {
-        k_p2g<PHYS_REF, false><<<(int)nb, t.p2g_block, 0, st>>>(V, t.ppt);
+        return launch_after(false, k_p2g<PHYS_REF, false>, (int)nb, t.p2g_block, st, V, t.ppt);
     }
-    return cudaGetLastError();
 }
 
 cudaError_t launch_grid(const View& V, const PhysFlags& pf, const Tuning& t, int num_sms, cudaStream_t st) {
@@ -2168,36 +2163,37 @@ cudaError_t launch_grid(const View& V, const PhysFlags& pf, const Tuning& t, int
 }
 
 // ...: further template arguments of KERNEL
-#define PGMPM_G2P_DISPATCH(KERNEL, GRID, BLOCK, ...)                                                  \
-    do {                                                                                              \
-        if (pf.physics == PHYS_MLS) {                                                                 \
-            if (pf.multi_mat) {                                                                       \
-                if (pf.has_fluid)                                                                     \
-                    KERNEL<PHYS_MLS, true, true __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);   \
-                else                                                                                  \
-                    KERNEL<PHYS_MLS, true, false __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);  \
-            } else {                                                                                  \
-                if (pf.has_fluid)                                                                     \
-                    KERNEL<PHYS_MLS, false, true __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);  \
-                else                                                                                  \
-                    KERNEL<PHYS_MLS, false, false __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V); \
-            }                                                                                         \
-        } else {                                                                                      \
-            KERNEL<PHYS_REF, false, false __VA_OPT__(, ) __VA_ARGS__><<<GRID, BLOCK, 0, st>>>(V);     \
-        }                                                                                             \
+#define PGMPM_G2P_DISPATCH(KERNEL, GRID, BLOCK, ...)                                                                        \
+    do {                                                                                                                    \
+        if (pf.physics == PHYS_MLS) {                                                                                       \
+            if (pf.multi_mat) {                                                                                             \
+                if (pf.has_fluid)                                                                                           \
+                    e = launch_after(false, KERNEL<PHYS_MLS, true, true __VA_OPT__(, ) __VA_ARGS__>, GRID, BLOCK, st, V);   \
+                else                                                                                                        \
+                    e = launch_after(false, KERNEL<PHYS_MLS, true, false __VA_OPT__(, ) __VA_ARGS__>, GRID, BLOCK, st, V);  \
+            } else {                                                                                                        \
+                if (pf.has_fluid)                                                                                           \
+                    e = launch_after(false, KERNEL<PHYS_MLS, false, true __VA_OPT__(, ) __VA_ARGS__>, GRID, BLOCK, st, V);  \
+                else                                                                                                        \
+                    e = launch_after(false, KERNEL<PHYS_MLS, false, false __VA_OPT__(, ) __VA_ARGS__>, GRID, BLOCK, st, V); \
+            }                                                                                                               \
+        } else {                                                                                                            \
+            e = launch_after(false, KERNEL<PHYS_REF, false, false __VA_OPT__(, ) __VA_ARGS__>, GRID, BLOCK, st, V);         \
+        }                                                                                                                   \
     } while (0)
 
 cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int num_sms, cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
     if (V.sp.cap) {  // sparse grids run the physical-order MLS G2P only
         if (pf.physics != PHYS_MLS) return cudaErrorNotSupported;
         const int nb = grid_for(V.N, t.g2p_block, 1 << 30);
-#define PGMPM_G2PS(M_, F_, P_)                                           \
-    do {                                                                 \
-        if (V.cnt.ccount)                                                \
-            k_g2p_sparse<M_, F_, P_, true><<<nb, t.g2p_block, 0, st>>>(V);  \
-        else                                                             \
-            k_g2p_sparse<M_, F_, P_, false><<<nb, t.g2p_block, 0, st>>>(V); \
+#define PGMPM_G2PS(M_, F_, P_)                                                                \
+    do {                                                                                      \
+        if (V.cnt.ccount)                                                                     \
+            e = launch_after(false, k_g2p_sparse<M_, F_, P_, true>, nb, t.g2p_block, st, V);  \
+        else                                                                                  \
+            e = launch_after(false, k_g2p_sparse<M_, F_, P_, false>, nb, t.g2p_block, st, V); \
     } while (0)
         if (pf.multi_mat) {
             if (pf.has_fluid) {
@@ -2213,12 +2209,12 @@ cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int 
             }
         }
 #undef PGMPM_G2PS
-        return cudaGetLastError();
+        return e;
     }
     if (V.resort) {  // a replay of recorded steps: physical order, keys checked
         if (pf.physics != PHYS_MLS) return cudaErrorNotSupported;
         const int nb = grid_for(V.N, t.g2p_block, 1 << 30);
-#define PGMPM_G2PC(M_, F_, P_) k_g2p_check<M_, F_, P_><<<nb, t.g2p_block, 0, st>>>(V)
+#define PGMPM_G2PC(M_, F_, P_) e = launch_after(false, k_g2p_check<M_, F_, P_>, nb, t.g2p_block, st, V)
         if (pf.multi_mat) {
             if (pf.has_fluid) {
                 if (pf.has_plastic) PGMPM_G2PC(true, true, true); else PGMPM_G2PC(true, true, false);
@@ -2233,7 +2229,7 @@ cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int 
             }
         }
 #undef PGMPM_G2PC
-        return cudaGetLastError();
+        return e;
     }
     if (t.g2p_variant == 0) {
         const int nb = num_sms * t.g2p_tiles_per_sm;
@@ -2253,20 +2249,21 @@ cudaError_t launch_g2p(const View& V, const PhysFlags& pf, const Tuning& t, int 
         else
             PGMPM_G2P_DISPATCH(k_g2p_phys, nb, t.g2p_block, false);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_g2p2g(const View& V, const PhysFlags& pf, const Tuning& t, int num_sms, cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
+    cudaError_t e = cudaSuccess;
     if (pf.physics != PHYS_MLS || !V.cell_range) return cudaErrorNotSupported;
     const int minb = t.g2p2g_blocks_per_sm == 6 ? 6 : 4;
     const int nb = num_sms * minb;
-#define PGMPM_G2P2G(M_, F_, P_)                                          \
-    do {                                                                 \
-        if (minb == 6)                                                   \
-            k_g2p2g<M_, F_, P_, 6><<<nb, G2_T, 0, st>>>(V);              \
-        else                                                             \
-            k_g2p2g<M_, F_, P_, 4><<<nb, G2_T, 0, st>>>(V);              \
+#define PGMPM_G2P2G(M_, F_, P_)                                               \
+    do {                                                                      \
+        if (minb == 6)                                                        \
+            e = launch_after(false, k_g2p2g<M_, F_, P_, 6>, nb, G2_T, st, V); \
+        else                                                                  \
+            e = launch_after(false, k_g2p2g<M_, F_, P_, 4>, nb, G2_T, st, V); \
     } while (0)
     if (pf.multi_mat) {
         if (pf.has_fluid) {
@@ -2282,7 +2279,7 @@ cudaError_t launch_g2p2g(const View& V, const PhysFlags& pf, const Tuning& t, in
         }
     }
 #undef PGMPM_G2P2G
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t launch_pack(const View& V, const float* x, const float* v, const float* C, const float* F,

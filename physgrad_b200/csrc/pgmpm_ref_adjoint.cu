@@ -506,22 +506,20 @@ cudaError_t launch_ref_step(const View& V, const BinSortBufs& B, const RefStep& 
     const bool adj = R.gx != nullptr;
     View K = V;
     K.cnt = B.cnt;
-    k_ref_keys<<<blocks_for(V.N, 256), 256, 0, st>>>(K, R);
-    cudaError_t e = bin_sort_step(V, B, num_sms, true, st, &R);
-    if (e != cudaSuccess) return e;
+    cudaError_t e = launch_after(false, k_ref_keys, blocks_for(V.N, 256), 256, st, K, R);
+    if (e == cudaSuccess) e = bin_sort_step(V, B, num_sms, true, st, &R);
     const int nb = (int)((V.N + 127) / 128);
     if (!adj) {
-        k_ref_p2g<false><<<num_sms * 4, P2GS_T, 0, st>>>(V, R);
-        e = launch_grid(V, pf, t, num_sms, st);
-        if (e != cudaSuccess) return e;
-        k_ref_g2p<<<nb, 128, 0, st>>>(V, R);
+        if (e == cudaSuccess) e = launch_after(false, k_ref_p2g<false>, num_sms * 4, P2GS_T, st, V, R);
+        if (e == cudaSuccess) e = launch_grid(V, pf, t, num_sms, st);
+        if (e == cudaSuccess) e = launch_after(false, k_ref_g2p, nb, 128, st, V, R);
     } else {
-        k_ref_p2g<true><<<num_sms * 3, P2GS_T, 0, st>>>(V, R);
         const int gb = (int)std::min<int64_t>(((int64_t)V.total_nt + 3) / 4, (int64_t)num_sms * 4);
-        k_ref_grid_adj<<<gb < 1 ? 1 : gb, 256, 0, st>>>(V, R);
-        k_ref_gather_sorted<<<nb, 128, 0, st>>>(V, R);
+        if (e == cudaSuccess) e = launch_after(false, k_ref_p2g<true>, num_sms * 3, P2GS_T, st, V, R);
+        if (e == cudaSuccess) e = launch_after(false, k_ref_grid_adj, gb < 1 ? 1 : gb, 256, st, V, R);
+        if (e == cudaSuccess) e = launch_after(false, k_ref_gather_sorted, nb, 128, st, V, R);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace pgmpm

@@ -21,9 +21,11 @@ int fail(int code, const char* fmt, ...);
 #define CK(expr)                                                                                             \
     do {                                                                                                     \
         cudaError_t e_ = (expr);                                                                             \
-        if (e_ != cudaSuccess)                                                                               \
+        if (e_ != cudaSuccess) {                                                                             \
+            cudaGetLastError(); /* reported here: not left for a later call to find */                       \
             return ::pgmpm::fail(e_ == cudaErrorMemoryAllocation ? PGMPM_ERR_OOM : PGMPM_ERR_CUDA,           \
                                  "%s: %s (%s:%d)", #expr, cudaGetErrorString(e_), __FILE__, __LINE__);       \
+        }                                                                                                    \
     } while (0)
 
 struct DevBuf {
@@ -140,6 +142,10 @@ struct pgmpm_solver_s {
     // the live state, done by the last step's G2P2G (the payload buffer is
     // then stale).  Cleared by pgmpm::unprime.
     bool primed = false;
+
+    // a call returned an error among a step's launches: what every step finds
+    // and leaves zero may not be (pgmpm::settle)
+    bool unsettled = false;
 
     // graphs, one per step kind and place in its call: bit 0, a step of the
     // same call follows (v, C not stored, the next keys counted); bit 1, a
@@ -373,6 +379,11 @@ StepKind step_kind(pgmpm_solver s, int k, int n, bool primed, bool drain);
 // Drops the pending P2G of the fused path (grid_mp cleared, payload
 // recomputed from the state), so that the next step starts with its own P2G.
 int unprime(pgmpm_solver s, cudaStream_t st);
+// Clears what a call that failed among a step's launches may have left in the
+// counters of the bin sort, the work cursors and the P2G accumulator, which
+// every step needs to find zero (s->unsettled); a sort on top of old counts
+// would read past the order array.  First in every call that runs steps.
+int settle(pgmpm_solver s, cudaStream_t st);
 // Run n steps of the live state (graph, eager or profiled).
 int run_steps(pgmpm_solver s, int n_steps, cudaStream_t st);
 }  // namespace pgmpm

@@ -1,0 +1,187 @@
+"""Calls that fail among a step's launches, and what the next call finds.
+
+The failures are made on the host: a preloaded stand-in for the launch entry
+of the CUDA runtime returns an error for the k-th launch without launching
+(child processes), or an error is left pending in the thread.  Two runs of
+one state differ by FP32 summation order: x <= 1e-6 absolute, v <= 1e-4 of
+the largest, F <= 1e-5, as in test_gpu_step_kernels.py.
+"""
+import ctypes
+import os
+import subprocess
+import sys
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SHIM = r"""
+#define _GNU_SOURCE
+#include <dlfcn.h>
+#include <stddef.h>
+static int launch_left = 0, build_left = 0;
+void fail_launch(int k) { launch_left = k; }   /* the k-th launch from now fails; 0: none */
+void fail_builds(int k) { build_left = k; }    /* the next k graph instantiations fail */
+static void* real(const char* name) {
+    return dlsym(dlopen("libcudart.so.12", RTLD_NOLOAD | RTLD_LAZY), name);
+}
+int cudaLaunchKernelExC(const void* cfg, const void* f, void** args) {
+    static int (*next)(const void*, const void*, void**) = NULL;
+    if (!next) next = (int (*)(const void*, const void*, void**))real("cudaLaunchKernelExC");
+    if (launch_left > 0 && --launch_left == 0) return 701; /* cudaErrorLaunchOutOfResources */
+    return next(cfg, f, args);
+}
+int cudaGraphInstantiate(void** exec, void* graph, unsigned long long flags) {
+    static int (*next)(void**, void*, unsigned long long) = NULL;
+    if (!next) next = (int (*)(void**, void*, unsigned long long))real("cudaGraphInstantiate");
+    if (build_left > 0) {
+        --build_left;
+        return 2; /* cudaErrorMemoryAllocation */
+    }
+    return next(exec, graph, flags);
+}
+"""
+
+COMMON = r"""
+import ctypes, sys
+import numpy as np
+import physgrad_b200 as pg
+from physgrad_b200 import _capi as C, workloads as W
+shim = ctypes.CDLL(None)
+
+def close(a, b):
+    assert np.abs(a["x"] - b["x"]).max() <= 1e-6
+    assert np.abs(a["v"] - b["v"]).max() <= 1e-4 * np.abs(b["v"]).max() + 1e-7
+    assert np.abs(a["F"] - b["F"]).max() <= 1e-5
+
+def raises(fn):
+    try:
+        fn()
+    except Exception as e:
+        return True
+    return False
+
+scenes, counts, mats, st, _ = W.elastic_cube(n_particles=3000, n=24, v_sigma=0.5, seed=5)
+N = counts[0]
+def solver():
+    return pg.Simulator(scenes, counts, mats, sparse_tiles=512 if SPARSE else None)
+def upload(s):
+    s.upload(st["x"], st["v"], None, None, st["m"], st["V0"])
+fresh = solver()
+upload(fresh)
+fresh.step(5)
+want = fresh.download()
+"""
+
+STEPS = COMMON + r"""
+sim = solver()
+sim.set_tuning(use_graph=0)
+failed = 0
+for k in range(1, 17):  # 6 + 5 + 5 launches
+    upload(sim)
+    shim.fail_launch(k)
+    failed += raises(lambda: sim.step(3))
+    shim.fail_launch(0)
+    before = sim.get_array(C.ARRAY_KEYS)
+    sim.step(1)
+    order = sim.get_array(C.ARRAY_SORTED_ORDER)
+    assert np.array_equal(np.sort(order), np.arange(N)), k
+    assert np.array_equal(before[order], np.sort(before)), k
+    upload(sim)
+    sim.step(5)
+    assert sim.status() == 0
+    close(sim.download(), want)
+assert failed == 16, failed
+print("CHILD OK")
+"""
+
+PIC = r"""
+import ctypes
+import numpy as np, torch
+from physgrad_b200.autograd import MPMTimestep
+shim = ctypes.CDLL(None)
+rng = np.random.default_rng(3)
+N, res = 3000, 32
+t = lambda a: torch.tensor(a.astype(np.float32), device="cuda")
+x, v, m, g = t(rng.uniform(0.2, 0.8, (N, 3))), t(rng.normal(0, 1, (N, 3))), t(rng.uniform(0.5, 1.5, N)), t(np.array([0, -9.8, 1]))
+gx, gv = t(rng.normal(0, 1, (N, 3))), t(rng.normal(0, 1, (N, 3)))
+for a in (x, v, m, g):
+    a.requires_grad_(True)
+def step(fwd=0, bwd=0):
+    torch.cuda.synchronize()
+    shim.fail_launch(fwd)
+    xo, vo = MPMTimestep.apply(x, v, m, g, res, 1e-3)
+    shim.fail_launch(bwd)
+    gr = torch.autograd.grad([xo, vo], [x, v, m, g], [gx, gv])
+    shim.fail_launch(0)
+    return [a.detach().cpu().numpy() for a in (xo, vo, *gr)]
+want = step()
+failed = 0
+for k in range(1, 7):  # 6 launches each way
+    for way in ({"fwd": k}, {"bwd": k}):
+        try:
+            step(**way)
+        except Exception:
+            failed += 1
+        shim.fail_launch(0)
+        for a, b in zip(step(), want):
+            assert np.abs(a - b).max() <= 1e-5 * np.abs(b).max(), (k, way)
+assert failed == 12, failed
+print("CHILD OK")
+"""
+
+
+@pytest.fixture(scope="module")
+def shim(tmp_path_factory):
+    d = tmp_path_factory.mktemp("shim")
+    (d / "shim.c").write_text(SHIM)
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-o", str(d / "shim.so"), str(d / "shim.c"), "-ldl"], check=True)
+    return str(d / "shim.so")
+
+
+def _child(shim, code):
+    env = dict(os.environ, LD_PRELOAD=shim, PYTHONPATH=ROOT)
+    r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and "CHILD OK" in r.stdout, r.stdout[-2000:] + r.stderr[-4000:]
+
+
+@pytest.mark.parametrize("sparse", [False, True])
+def test_steps_after_a_call_that_failed_between_launches(gpu, shim, sparse):
+    """A three-step call whose k-th launch fails, for every k: the next step
+    sorts each particle once (a step's G2P counts the next step's keys, which a
+    failed call leaves counted), and after an upload five steps are those of a
+    fresh solver."""
+    _child(shim, f"SPARSE = {sparse}\n" + STEPS)
+
+
+def test_pic_steps_after_a_call_that_failed_between_launches(gpu, shim):
+    """The same for each launch of the PIC step's forward and backward."""
+    _child(shim, PIC)
+
+
+def test_steps_with_an_error_pending_in_the_thread(gpu):
+    """An error that an earlier CUDA call of the thread left pending is not
+    taken for a step's own, and a create that runs out of memory leaves none."""
+    from physgrad_b200 import PGMPMError
+    from physgrad_b200 import workloads as W
+
+    rt = ctypes.CDLL("libcudart.so.12")
+    scenes, counts, mats, st, _ = W.elastic_cube(n_particles=3000, n=24, v_sigma=0.5, seed=5)
+    outs = []
+    for pending in (False, True):
+        sim = gpu.Simulator(scenes, counts, mats)
+        sim.upload(st["x"], st["v"], None, None, st["m"], st["V0"])
+        if pending:
+            with pytest.raises(PGMPMError):  # 206 GB of state planes
+                gpu.Simulator(scenes, [2 ** 31 - 16], mats)
+            assert rt.cudaPeekAtLastError() == 0
+            assert rt.cudaSetDevice(4096) != 0 and rt.cudaPeekAtLastError() != 0
+        sim.step(5)
+        rt.cudaGetLastError()
+        assert sim.status() == 0
+        outs.append(sim.download())
+    assert np.abs(outs[0]["x"] - outs[1]["x"]).max() <= 1e-6
+    assert np.abs(outs[0]["v"] - outs[1]["v"]).max() <= 1e-4 * np.abs(outs[0]["v"]).max()
