@@ -66,16 +66,24 @@ __global__ void k_mforce_out(const float4* __restrict__ mf, const float4* __rest
     }
 }
 
+// Margin, in cells, of the cut at cell coordinate g.  A coordinate is the
+// rounded quotient of a rounded difference (2^-23 of it off), and a cell's face
+// is formed with as much error again: 2^-22 g, the same for a bound of the z
+// window.  1e-3 alone dropped one pair in a few thousand at the edge of the
+// sphere from 60,000 cells an axis on.  The last sum and difference need none:
+// rounding keeps the order of what the pair test rounds too.
+__device__ __forceinline__ float cpl_margin(float g) { return 1e-3f + 0x1p-21f * g; }
 // Distance from y to cell g along axis a, a lower bound for any particle stored
 // there (the last cell also holds clamped particles: 0).
 __device__ __forceinline__ float cpl_gap(const HGDev& G, int a, float y, uint32_t g) {
-    const float lo = G.dmin[a] + ((float)g - 1e-3f) * G.cell, hi = G.dmin[a] + ((float)g + 1.001f) * G.cell;
+    const float m = cpl_margin((float)g);
+    const float lo = G.dmin[a] + ((float)g - m) * G.cell, hi = G.dmin[a] + ((float)g + (1.f + m)) * G.cell;
     return g + 1u == G.res[a] ? 0.f : fmaxf(fmaxf(g == 0u ? 0.f : lo - y, y - hi), 0.f);
 }
 // hg_row cut to the cells that the sphere of radius r around y (cell c) can
 // reach: of the 125 cells of half a radius each around a particle the sphere
-// meets about 60%.  The margins (1e-3 of a cell, 1e-5 of r^2) are far above the
-// rounding of the cell coordinates, so that the cut drops no pair.
+// meets about 60%.  The margins (cpl_margin, and 1e-5 of r^2 for the rounding
+// of the squared distances) are above the rounding, so that the cut drops no pair.
 __device__ __forceinline__ uint2 cpl_row(const HGDev& G, const uint32_t c[3], uint32_t src, uint32_t dx, uint32_t dy,
                                          const float y[3], float r, const uint32_t* __restrict__ first) {
     const uint32_t gx = c[0] + dx - src, gy = c[1] + dy - src;
@@ -84,7 +92,8 @@ __device__ __forceinline__ uint2 cpl_row(const HGDev& G, const uint32_t c[3], ui
     const float z2 = r * r * 1.00001f - a * a - b * b;
     if (z2 < 0.f) return make_uint2(0u, 0u);
     const float zr = sqrtf(z2), inv = 1.f / G.cell;
-    const float f0 = floorf((y[2] - zr - G.dmin[2]) * inv - 1e-3f), f1 = floorf((y[2] + zr - G.dmin[2]) * inv + 1e-3f);
+    const float t0 = (y[2] - zr - G.dmin[2]) * inv, t1 = (y[2] + zr - G.dmin[2]) * inv;
+    const float f0 = floorf(t0 - cpl_margin(fabsf(t0))), f1 = floorf(t1 + cpl_margin(fabsf(t1)));
     // the window [c2 - src, c2 + src] as signed 64-bit, cut at the sphere and the grid
     const long long z = (long long)(int)c[2], last = (long long)G.res[2] - 1;
     long long z0 = max(z - (long long)src, 0ll), z1 = min(z + (long long)src, last);

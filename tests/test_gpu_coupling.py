@@ -131,3 +131,36 @@ def test_kinetic_energy_per_material_counts(gpu, oracle, n_mats):
     if n_mats > 1:
         assert per[-1] == 0.0
     assert abs(tot - ref.sum()) <= 1e-9 * ref.sum()
+
+
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("origin", [0.0, -100.0])
+def test_pairs_at_the_edge_of_the_radius_on_a_long_axis(gpu, axis, origin):
+    """200,000 cells along one axis, pairs a rounding inside the radius along
+    it: the walk's cut to the sphere keeps every pair that the cells of one
+    radius around the SPH particle hold (counted here in the reference's
+    float operations)."""
+    rng = np.random.default_rng(17 + axis)
+    dx = np.float32(0.026)
+    dims = [8, 8, 8]
+    dims[axis] = 100000
+    r = np.float32(0.5) * dx  # the cell: half of it would make too many cells
+    n = 20000
+    f = np.float32
+    at = (np.arange(n) + 0.5) * ((dims[axis] - 5) * float(dx) / n) + 2 * float(dx)  # 10 cells apart
+    y = (f(origin) + (at + rng.uniform(-0.5, 0.5, n) * float(dx)).astype(f)).astype(f)
+    side = np.where(rng.random(n) < 0.5, f(-1), f(1))
+    x = (y + side * r).astype(f)
+    for _ in range(4):
+        x = np.where(np.abs(x - y) < r, x, np.nextafter(x, y)).astype(f)
+    d = np.sqrt(((x - y) * (x - y)).astype(f))
+    cell = lambda a: np.trunc(((a - f(origin)).astype(f) / r).astype(f))
+    want = int(np.sum((d < r) & (np.abs(cell(x) - cell(y)) <= 1)))
+    assert want > 0.9 * n
+    px = np.full((n, 3), origin + 3.3 * float(dx), f)
+    py = px.copy()
+    px[:, axis], py[:, axis] = x, y
+    scene = gpu.Scene(tuple(dims), float(dx), 1e-4, (0.0, 0.0, 0.0), (origin,) * 3)
+    sim = gpu.Simulator([scene], [n], [gpu.createElasticMaterial(1000.0, 1e4, 0.3)])
+    sim.upload(px, None, None, None, np.ones(n, f), np.full(n, 1e-6, f))
+    assert sim.sph_coupling(py, np.zeros_like(py), radius=float(r))[2] == want
