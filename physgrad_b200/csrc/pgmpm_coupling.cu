@@ -385,8 +385,8 @@ int pgmpm_sph_coupling(pgmpm_solver s, const pgmpm_sph_coupling_config* cfg, con
                 return fail(PGMPM_ERR_ARG, "hashgrid: each axis needs 1 .. 2^32-1 cells");
             G.res[a] = (uint32_t)n;
             total *= G.res[a];
+            if (total > 0xFFFFFFFFull) return fail(PGMPM_ERR_ARG, "hashgrid: more than 2^32 - 1 cells");
         }
-        if (total > 0xFFFFFFFFull) return fail(PGMPM_ERR_ARG, "hashgrid: more than 2^32 - 1 cells");
         const float sr = std::ceil(cfg->coupling_radius / cell);  // cells a radius spans
         float d2_max = cfg->coupling_radius * cfg->coupling_radius;
         while (d2_max > 0.f && std::sqrt(d2_max) >= cfg->coupling_radius) d2_max = std::nextafter(d2_max, 0.f);

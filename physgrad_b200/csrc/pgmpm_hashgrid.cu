@@ -532,10 +532,10 @@ int pgmpm_hashgrid_create(float cell_size, const float* domain_min, const float*
         }
         g->res[a] = (uint32_t)r;
         total *= g->res[a];
-    }
-    if (total > 0xFFFFFFFFull) {
-        delete g;
-        return fail(PGMPM_ERR_ARG, "hashgrid: more than 2^32 - 1 cells");
+        if (total > 0xFFFFFFFFull) {  // per factor: three of them overflow 64 bits
+            delete g;
+            return fail(PGMPM_ERR_ARG, "hashgrid: more than 2^32 - 1 cells");
+        }
     }
     g->total = (uint32_t)total;
     g->key_bits = std::max(1, bits_for(total));

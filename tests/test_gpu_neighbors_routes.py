@@ -95,3 +95,15 @@ def test_contact_pairs_equal_brute_force(gpu, nodes, radius, N, Q):
     assert abs(energy - want_e) <= 1e-5 * want_e + 1e-12
     assert np.abs(f - want_f).max() <= 1e-5 * np.abs(want_f).max() + 1e-6
     assert np.abs(mf - want_m).max() <= 1e-5 * np.abs(want_m).max() + 1e-6
+
+
+def test_more_cells_than_32_bits_are_refused(gpu):
+    """2^22 cells an axis: their number is a multiple of 2^64, which the check
+    of the whole product took for none."""
+    with pytest.raises(gpu.PGMPMError, match="more than"):
+        gpu.SpatialHashGrid(2.0 ** -22, (0.0, 0.0, 0.0), (1.0, 1.0, 1.0), max_particles=100)
+    one = np.ones(1, np.float32)
+    sim = gpu.Simulator([gpu.Scene((65,) * 3, 1.0 / 64, 1e-4)], [1], [gpu.createElasticMaterial(1000.0, 1e4, 0.3)])
+    sim.upload(np.full((1, 3), 0.5, np.float32), None, None, None, one, one)
+    with pytest.raises(gpu.PGMPMError, match="more than"):
+        sim.sph_coupling(np.full((1, 3), 0.5, np.float32), np.zeros((1, 3), np.float32), radius=2.0 ** -22)
