@@ -452,7 +452,14 @@ PGMPM_API void launch_mpm_timestep_backward(const float* grad_positions, const f
  * that step's masses and gravity (may be NULL: the last forward's) instead of
  * relying on the last forward call, and leaves them as the last call's.  A
  * first forward call with the device, particle count and resolution must have
- * been made. */
+ * been made.
+ *
+ * Calls of all four with one device, particle count and resolution share a
+ * solver.  They may come from several threads and streams: each waits, on the
+ * device, for the one before.  (What a call relies on from the last forward
+ * is the last one of any thread.)  Under a stream capture a call does not wait
+ * and is not waited for: order the graph's launches after other calls of the
+ * size. */
 PGMPM_API void pgmpm_mpm_timestep_forward(const float* positions, const float* velocities, const float* masses,
                                 float* positions_out, float* velocities_out, int num_particles, int grid_resolution,
                                 float dt, const float* gravity, void* stream);

@@ -592,6 +592,40 @@ namespace {
 struct LaunchEntry {
     pgmpm_solver s = nullptr;
     pgmpm::DevBuf masses;  // the last forward's masses: the backward's signature carries none
+    std::mutex mu;              // held while a call enqueues its work
+    cudaEvent_t done = nullptr; // the end of the last call's work,
+    unsigned long long stream = 0;  // which went to the stream of this id
+};
+
+// One call's use of an entry: its solver's counters, state and accumulators
+// are shared by all calls of one size, so calls enqueue one after another and
+// a call on another stream than the last one's waits for that one's work
+// (an event per call, 1 us of host time).  A call under a capture neither
+// waits nor is waited for: its graph's launches are for the caller to order.
+class LaunchUse {
+  public:
+    LaunchUse(LaunchEntry& e, cudaStream_t st) : e_(e), st_(st), lock_(e.mu) {
+        cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+        ok_ = cudaStreamIsCapturing(st, &cs) == cudaSuccess;
+        capturing_ = cs != cudaStreamCaptureStatusNone;
+        if (!ok_ || capturing_) return;
+        ok_ = cudaStreamGetId(st, &id_) == cudaSuccess &&
+              (e.done ? id_ == e.stream || cudaStreamWaitEvent(st, e.done, 0) == cudaSuccess
+                      : cudaEventCreateWithFlags(&e.done, cudaEventDisableTiming) == cudaSuccess);
+    }
+    ~LaunchUse() {
+        if (!ok_ || capturing_) return;
+        cudaEventRecord(e_.done, st_);
+        e_.stream = id_;
+    }
+    bool ok() const { return ok_; }
+
+  private:
+    LaunchEntry& e_;
+    cudaStream_t st_;
+    std::lock_guard<std::mutex> lock_;
+    bool ok_ = false, capturing_ = false;
+    unsigned long long id_ = 0;
 };
 std::mutex g_launch_mu;
 std::map<std::tuple<int, int, int>, LaunchEntry> g_launch_solvers;
@@ -672,6 +706,11 @@ void timestep_forward(const char* who, const float* positions, const float* velo
             s = entry->s;
         }
     }
+    LaunchUse use(*entry, st);
+    if (!use.ok()) {
+        fail(PGMPM_ERR_CUDA, "%s: %s", who, cudaGetErrorString(cudaGetLastError()));
+        return;
+    }
     if (!launch_set_dt(s, dt, st, who)) return;
     // the masses (and the gravity, in the scene table) are kept for
     // launch_mpm_timestep_backward
@@ -748,18 +787,28 @@ void timestep_backward(const char* who, const float* grad_positions, const float
     int dev = 0;
     cudaGetDevice(&dev);
     cudaStream_t st = ST(stream);
-    pgmpm_solver s = nullptr;
-    float* kept = nullptr;
+    LaunchEntry* entry = nullptr;
     {
         std::lock_guard<std::mutex> lk(g_launch_mu);
         auto it = g_launch_solvers.find(std::make_tuple(dev, num_particles, grid_resolution));
-        if (it == g_launch_solvers.end() || !it->second.masses.p) {
-            fail(PGMPM_ERR_STATE,
-                 "%s: no launch_mpm_timestep_forward call with this device, particle count and resolution", who);
-            return;
-        }
-        s = it->second.s;
-        kept = it->second.masses.as<float>();
+        if (it != g_launch_solvers.end()) entry = &it->second;
+    }
+    const char* no_forward =
+        "%s: no launch_mpm_timestep_forward call with this device, particle count and resolution";
+    if (!entry) {
+        fail(PGMPM_ERR_STATE, no_forward, who);
+        return;
+    }
+    LaunchUse use(*entry, st);
+    if (!use.ok()) {
+        fail(PGMPM_ERR_CUDA, "%s: %s", who, cudaGetErrorString(cudaGetLastError()));
+        return;
+    }
+    pgmpm_solver s = entry->s;
+    float* kept = entry->masses.as<float>();
+    if (!kept) {
+        fail(PGMPM_ERR_STATE, no_forward, who);
+        return;
     }
     if (!launch_set_dt(s, dt, st, who)) return;
     if (s->tune.step_sort == 0) {  // on the caller's arrays
