@@ -281,7 +281,7 @@ def run_ours(args, rank, world, device):
         sim.autotune(reps=3)
         sim.upload(st["x"], st["v"], Cm, Fm, st["m"], st["V0"], st["mat"])
     stream = torch.cuda.current_stream()
-    # warm-up (also builds the CUDA graph)
+    # warm-up
     sim.step(args.warmup, stream=stream)
     torch.cuda.synchronize()
     if world > 1:

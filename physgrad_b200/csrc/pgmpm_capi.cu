@@ -153,7 +153,7 @@ int conditional_sort(pgmpm_solver s, const View& V, const BinSortBufs& B, uint32
 }
 
 int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, bool write_vc, StepKind kind,
-                bool counted, bool count_next) {
+                bool counted, bool count_next, bool after_graph) {
     if (s->N == 0) {  // nothing to move; keep the timing events consistent
         if (timed)
             for (int i = 0; i < 5; ++i) CK(cudaEventRecord(s->ev[i], st));
@@ -168,7 +168,7 @@ int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, 
     View V = s->view_for(b);
     if (count_next) V.cnt = s->sort_counts();
     V.early = !timed;
-    V.early_first = counted && !timed;  // after the previous step's G2P
+    V.early_first = counted && !timed && !after_graph;  // after the previous step's G2P
     // P2G variant 1 builds its payload from the state's v and C
     V.write_vc = write_vc || s->pf.physics != PHYS_MLS || s->tune.p2g_variant == 1 ? 1 : 0;
     // per-step resets: tile counts, active node count, work cursors, and the
@@ -273,7 +273,9 @@ int build_graph(pgmpm_solver s, StepKind kind, int place) {
     }
     CK(e);
     graph = g;
-    CK(cudaGraphInstantiate(&exec, g, 0));
+    e = cudaGraphInstantiate(&exec, g, 0);
+    if (e != cudaSuccess) exec = nullptr;
+    CK(e);
     return PGMPM_OK;
 }
 
@@ -290,7 +292,10 @@ int build_span(pgmpm_solver s, int steps, bool whole, cudaGraphExec_t& exec) {
     }
     cudaGraph_t g = nullptr;
     cudaError_t e = cudaStreamEndCapture(s->cap_stream, &g);
-    if (rc == PGMPM_OK && e == cudaSuccess) e = cudaGraphInstantiate(&exec, g, 0);
+    if (rc == PGMPM_OK && e == cudaSuccess) {
+        e = cudaGraphInstantiate(&exec, g, 0);
+        if (e != cudaSuccess) exec = nullptr;
+    }
     if (g) cudaGraphDestroy(g);
     if (rc) return rc;
     CK(e);
@@ -300,6 +305,42 @@ int build_span(pgmpm_solver s, int steps, bool whole, cudaGraphExec_t& exec) {
 }  // namespace
 
 namespace {
+// Makes the graphs that calls like this one will use, after its launches,
+// while the GPU works on them: a step's graph takes 100 us of host time, a
+// call's of 50 steps 900, the first one of a process ms on some hosts, where a
+// call that stopped in its middle to make one let the GPU run dry (20 steps of
+// 2 M particles 4.4 -> 13.7 ms once).  It pays for itself over some ten calls,
+// so it waits for kSeenStep calls that launched such a step kernel by kernel,
+// or kSeenCall calls (in a row, for a call's graph) of one length.  A graph
+// that cannot be made leaves the steps to their kernels.
+void make_graphs(pgmpm_solver s, int n_steps, bool spans, const bool direct[STEP_KINDS][4]) {
+    int rc = PGMPM_OK;
+    const std::string message = g_err;
+    auto now = [&](int& seen, int at_least) {  // seen calls, this one included
+        if (seen < at_least) ++seen;
+        return seen >= at_least && !s->graphs_failed && !rc;
+    };
+    if (spans && n_steps > 1 && n_steps <= s->kCallSteps) {
+        if (n_steps != s->call_last) s->call_seen = 0;
+        s->call_last = n_steps;
+        if (now(s->call_seen, s->kSeenCall)) {
+            s->call_steps = 0;
+            rc = build_span(s, n_steps, true, s->call_exec);
+            if (!rc) s->call_steps = n_steps;
+        }
+    }
+    if (spans && n_steps >= s->kMidAtLeast && !s->mid_exec && now(s->mid_seen, s->kSeenCall))
+        rc = build_span(s, s->kMidSteps, false, s->mid_exec);
+    for (int kind = 0; kind < STEP_KINDS; ++kind)
+        for (int place = 0; place < 4; ++place)
+            if (direct[kind][place] && s->call_steps != n_steps && now(s->step_seen[kind][place], s->kSeenStep))
+                rc = build_graph(s, (StepKind)kind, place);
+    if (rc) {
+        s->graphs_failed = true;
+        g_err = message;  // the steps are enqueued: not this call's error
+    }
+}
+
 // Live steps.  With the fused kernel a call leaves the next step's P2G in
 // grid_mp (s->primed), so a following call continues without a P2G of its
 // own; anything that changes the state or its parameters unprimes first.
@@ -310,38 +351,31 @@ int live_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
     }
     // How steps are launched.  The GPU is idle for 2 us between two graphs, 8%
     // of a step of a small scene, so steps that recur are captured together: a
-    // whole call of up to 64 steps the third time in a row a call has that many
-    // (one such graph is kept), and 16 steps at a time inside calls of 128 and
-    // more.  50 steps of 32,768 particles 1303 -> 1163 us, 5 of 4,096 150 -> 138,
-    // 20 of 2 M 4925 -> 4853.  Making a graph takes tens of us, so the first eight
-    // steps of each kind and place are launched kernel by kernel: the first call
-    // of 5 steps of a new 4,096-particle solver 407 -> 182 us, of 50 steps of
-    // 32,768 1455 -> 1354.
-    const bool spans = s->use_graph && !s->profiling && !s->fused();
-    if (spans && n_steps > 1 && n_steps <= s->kCallSteps) {
-        s->call_seen = n_steps == s->call_last ? std::min(s->call_seen + 1, (int)s->kCallRepeats) : 1;
+    // whole call of up to 64 steps (one such graph is kept), and 16 steps at a
+    // time inside calls of 130 and more.  50 steps of 32,768 particles 1303 ->
+    // 1163 us, 5 of 4,096 150 -> 138, 20 of 2 M 4925 -> 4853.  Steps without a
+    // graph are launched kernel by kernel, all of them under the caller's
+    // capture (a graph cannot be launched into one).
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    CK(cudaStreamIsCapturing(st, &cs));
+    const bool graphs = s->use_graph && cs == cudaStreamCaptureStatusNone;
+    if (s->use_graph && !graphs && s->fused())  // a replay would not know whether the next P2G is done
+        return fail(PGMPM_ERR_UNSUPPORTED, "fused steps cannot be captured");
+    const bool spans = graphs && !s->profiling && !s->fused();
+    if (spans && n_steps > 1 && n_steps <= s->kCallSteps && s->call_steps == n_steps) {
+        CK(cudaGraphLaunch(s->call_exec, st));
         s->call_last = n_steps;
-        if (s->call_steps != n_steps && s->call_seen >= s->kCallRepeats) {
-            s->call_steps = 0;
-            int rc = build_span(s, n_steps, true, s->call_exec);
-            if (rc) return rc;
-            s->call_steps = n_steps;
-        }
-        if (s->call_steps == n_steps) {
-            CK(cudaGraphLaunch(s->call_exec, st));
-            s->met.total_steps += n_steps;
-            return PGMPM_OK;
-        }
+        s->met.total_steps += n_steps;
+        return PGMPM_OK;
     }
+    bool direct[STEP_KINDS][4] = {};
+    bool after_graph = false;
     for (int k = 0; k < n_steps; ++k) {
-        if (spans && k > 0 && k + s->kMidSteps < n_steps && (s->mid_exec || n_steps - 1 - k >= s->kMidAtLeast)) {
-            if (!s->mid_exec) {
-                int rc = build_span(s, s->kMidSteps, false, s->mid_exec);
-                if (rc) return rc;
-            }
+        if (spans && s->mid_exec && k > 0 && k + s->kMidSteps < n_steps) {
             CK(cudaGraphLaunch(s->mid_exec, st));
             s->met.total_steps += s->kMidSteps;
             k += s->kMidSteps - 1;
+            after_graph = true;
             continue;
         }
         const StepKind kind = step_kind(s, k, n_steps, s->primed, false);
@@ -363,22 +397,21 @@ int live_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
             s->met.average_step_ms =
                 (s->met.average_step_ms * s->met.total_steps + s->met.last_step_ms) / (s->met.total_steps + 1);
             s->met.particle_steps_per_s = s->met.average_step_ms > 0 ? s->N / (s->met.average_step_ms * 1e-3) : 0;
-        } else if (s->use_graph && s->step_seen[kind][place] >= s->kDirectSteps) {
-            if (!s->step_exec[kind][place]) {
-                int rc = build_graph(s, kind, place);
-                if (rc) return rc;
-            }
+        } else if (graphs && s->step_exec[kind][place]) {
             CK(cudaGraphLaunch(s->step_exec[kind][place], st));
+            after_graph = true;
         } else {
-            if (s->step_seen[kind][place] < s->kDirectSteps) s->step_seen[kind][place]++;
             const bool ahead = s->counts_ahead() && kind == STEP_SPLIT;
             int rc = record_step(s, s->live_bufs(), st, false, k + 1 == n_steps, kind, ahead && k > 0,
-                                 ahead && k + 1 < n_steps);
+                                 ahead && k + 1 < n_steps, after_graph);
             if (rc) return rc;
+            direct[kind][place] = true;
+            after_graph = false;
         }
         if (kind == STEP_FUSED_FIRST || kind == STEP_FUSED) s->primed = true;
         s->met.total_steps++;
     }
+    if (graphs && !s->profiling) make_graphs(s, n_steps, spans, direct);
     return PGMPM_OK;
 }
 }  // namespace

@@ -153,14 +153,16 @@ struct pgmpm_solver_s {
     cudaStream_t cap_stream = nullptr;
     cudaGraphExec_t step_exec[pgmpm::STEP_KINDS][4] = {};
     cudaGraph_t step_graph[pgmpm::STEP_KINDS][4] = {};
-    int step_seen[pgmpm::STEP_KINDS][4] = {};  // such steps launched without a graph
-    static constexpr int kDirectSteps = 8;
+    int step_seen[pgmpm::STEP_KINDS][4] = {};  // calls that launched such steps without a graph
     // several split steps in one graph (run_steps): all steps of a call, and
     // kMidSteps steps with others of their call before and after them
-    static constexpr int kCallSteps = 64, kCallRepeats = 3, kMidSteps = 16, kMidAtLeast = 128;
+    static constexpr int kCallSteps = 64, kMidSteps = 16, kMidAtLeast = 130;
     cudaGraphExec_t call_exec = nullptr, mid_exec = nullptr;
     int call_steps = 0;               // steps of call_exec
     int call_last = 0, call_seen = 0; // steps of the last call, and calls in a row that had as many
+    int mid_seen = 0;                 // calls that could have used mid_exec
+    static constexpr int kSeenCall = 5, kSeenStep = 8;  // calls after which a graph is made
+    bool graphs_failed = false;       // one could not be made: no further attempts until drop_graph
     cudaEvent_t ev[6] = {};
 
     // metrics
@@ -296,7 +298,8 @@ struct pgmpm_solver_s {
         if (call_exec) cudaGraphExecDestroy(call_exec);
         if (mid_exec) cudaGraphExecDestroy(mid_exec);
         call_exec = mid_exec = nullptr;
-        call_steps = call_last = call_seen = 0;
+        call_steps = call_last = call_seen = mid_seen = 0;
+        graphs_failed = false;
         drop_tape_graphs();
     }
 
@@ -370,8 +373,10 @@ int alloc_bin_sort(pgmpm_solver s);
 // counted: the bin sort's counters hold the counts of b.keys_in already;
 // count_next: this step's G2P counts the keys it writes (counts_ahead(); the
 // step that sorts b.keys_out must be recorded next, counted).
+// after_graph: a graph, not a kernel, is before this step on the stream (a
+// counted step's first kernel is then not launched early).
 int record_step(pgmpm_solver s, const StepBufs& b, cudaStream_t st, bool timed, bool write_vc = true,
-                StepKind kind = STEP_SPLIT, bool counted = false, bool count_next = false);
+                StepKind kind = STEP_SPLIT, bool counted = false, bool count_next = false, bool after_graph = false);
 // The kind of step k of n consecutive steps that start from a state whose
 // P2G is (primed) or is not already in grid_mp; drain: the last step leaves
 // nothing pending (G2P instead of G2P2G).

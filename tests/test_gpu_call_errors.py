@@ -134,6 +134,32 @@ print("CHILD OK")
 """
 
 
+BUILDS = COMMON + r"""
+direct = solver()
+direct.set_tuning(use_graph=0)
+sim = solver()
+shim.fail_builds(1000)
+for calls in ([5] * 7, [1] * 10, [140] * 6):
+    for s in (sim, direct):
+        upload(s)
+        for k in calls:
+            s.step(k)
+    assert sim.status() == direct.status() == 0
+    assert pg.lib().pgmpm_last_error() == b""
+    if calls[0] < 100:  # (longer runs drift apart by rounding)
+        close(sim.download(), direct.download())
+shim.fail_builds(0)
+sim.set_tuning(use_graph=1)
+upload(sim)
+for _ in range(7):
+    sim.step(5)
+upload(sim)
+sim.step(5)
+close(sim.download(), want)
+print("CHILD OK")
+"""
+
+
 @pytest.fixture(scope="module")
 def shim(tmp_path_factory):
     d = tmp_path_factory.mktemp("shim")
@@ -160,6 +186,12 @@ def test_steps_after_a_call_that_failed_between_launches(gpu, shim, sparse):
 def test_pic_steps_after_a_call_that_failed_between_launches(gpu, shim):
     """The same for each launch of the PIC step's forward and backward."""
     _child(shim, PIC)
+
+
+def test_steps_whose_graphs_cannot_be_made(gpu, shim):
+    """Every graph instantiation fails for want of memory: the steps run
+    kernel by kernel, no call fails, and graphs are made again afterwards."""
+    _child(shim, "SPARSE = False\n" + BUILDS)
 
 
 def test_steps_with_an_error_pending_in_the_thread(gpu):

@@ -255,3 +255,44 @@ def test_pic_step_routes_agree(gpu, n_near):
     for a, b in zip(*outs):
         assert np.isfinite(b).all()
         assert np.abs(a - b).max() <= 8e-6 * np.abs(b).max() + 1e-9
+
+
+@pytest.mark.parametrize("calls", [[1] * 11, [2] * 11, [5, 5, 3] + [5] * 8 + [3] * 7 + [5, 7] * 9, [64] * 7,
+                                   [131, 146, 17, 140, 130, 17, 135, 40, 17, 133]])
+@pytest.mark.parametrize("sparse", [False, True])
+@pytest.mark.parametrize("outer", [False, True])
+def test_steps_before_and_after_their_graphs_are_made(gpu, calls, sparse, outer):
+    """Call lengths repeated until a step's, a call's and the 16-step graph are
+    made and used, also inside the caller's own capture (outer: every third
+    call is captured and its graph launched): against launches without graphs.
+    Free particles and the bounds of
+    test_steps_launched_one_by_one_and_in_graphs_agree."""
+    import torch
+
+    rng = np.random.default_rng(12)
+    N, n = 700, (32, 31, 30)
+    dx = 1.0 / 16
+    scene = gpu.Scene(n, dx, 2e-4, (0.0, 0.0, 0.0), (0.0, 0.0, 0.0), 0, 0, 0)
+    st = _scene_state(rng, N, n, dx, margin=8.0)
+    mats = [gpu.createElasticMaterial(1000.0, 0.0, 0.3)]
+    outs = []
+    for graph in (1, 0):
+        sim = gpu.Simulator([scene], [N], mats, sparse_tiles=2048 if sparse else None)
+        sim.set_tuning(use_graph=graph)
+        sim.upload(st["x"], st["v"], st["C"], st["F"], st["m"], st["V0"])
+        graphs, s = [], torch.cuda.Stream()
+        for i, k in enumerate(calls):
+            if outer and graph and i % 3 == 2:
+                torch.cuda.synchronize()
+                graphs.append(torch.cuda.CUDAGraph())
+                with torch.cuda.graph(graphs[-1], stream=s):
+                    sim.step(k, stream=torch.cuda.current_stream())
+                graphs[-1].replay()
+                torch.cuda.synchronize()
+            else:
+                sim.step(k)
+        assert sim.status() == 0
+        outs.append(sim.download())
+    ulps = sum(calls) * 2.0 ** -23
+    assert np.abs(outs[0]["x"] - outs[1]["x"]).max() <= 1.4 * ulps + 1e-6
+    assert np.abs(outs[0]["v"] - outs[1]["v"]).max() <= (4 * ulps + 1e-6) * np.abs(outs[1]["v"]).max()
