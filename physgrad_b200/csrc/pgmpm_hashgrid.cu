@@ -25,6 +25,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "pgmpm_hashgrid.cuh"
 #include "pgmpm_solver_impl.h"
@@ -41,23 +42,34 @@ struct pgmpm_hashgrid_s {
     int64_t max_particles = 0;
     int64_t n = 0;  // particles of the last build
     bool built = false;
-    DevBuf counts, starts;          // per cell
-    DevBuf cell_ids;                // per particle: cell id (particle order)
-    // sort buffers; between builds va keeps the sorted particle indices, ka and
-    // vb are the dense queries' (dense_index, the queries' cells)
-    DevBuf ka, va, kb, vb, scratch, pos_stage;
-    DevBuf qcount, qstage, qout_stage, scan_tmp, stats;  // query scratch, kept between calls
-    // dense queries (cells in grid order, x outer, z inner): z stretches and
-    // block sums for the last half width and first[] of the cells' buckets (one
-    // allocation), and the buckets themselves
-    DevBuf grid_tables, grid_index;
-    uint2* grid_rows() const { return grid_tables.as<uint2>(); }
-    uint32_t* grid_sum() const { return reinterpret_cast<uint32_t*>(grid_rows() + total); }
-    uint32_t* grid_first() const { return grid_sum() + total; }
-    uint32_t* dense_index() const { return mult_max > 1 ? grid_index.as<uint32_t>() : vb.as<uint32_t>(); }
-    uint32_t mult_max = 0;    // most cells that hash to one bucket (0: not counted yet)
-    bool grid_ready = false;  // grid_first and grid_index hold the last build's
+    // Buffers of a size known at creation, in one allocation (every one of a
+    // megabyte and more takes 0.34 ms; see layout())
+    DevBuf mem;
+    uint32_t *counts = nullptr, *starts = nullptr;  // per cell
+    uint32_t* cell_ids = nullptr;                   // per particle: cell id (particle order)
+    // sort buffers; between builds va keeps the sorted particle indices, ka
+    // holds the queries' cells, and kb and vb, one stretch, the index in grid order
+    uint32_t *ka = nullptr, *va = nullptr, *kb = nullptr, *vb = nullptr, *scratch = nullptr;
+    unsigned long long* stats = nullptr;
+    int64_t* scan = nullptr;    // block sums of a scan over cells or up to max_particles queries
+    int64_t* result = nullptr;  // [0] length of a query set's lists, [1] entries of the index in grid order
+    uint32_t* qcount = nullptr; // counts of up to max_particles queries (null: qlarge)
+    // dense queries (cells in grid order, x outer, z inner; null: hashed queries
+    // only): z stretches and block sums for the last half width, and first[] of
+    // the cells' buckets
+    uint2* grid_rows = nullptr;
+    uint32_t *grid_sum = nullptr, *grid_first = nullptr;
+    DevBuf pos_stage, qstage, qout_stage, off_stage;  // host arrays on the device
+    DevBuf qlarge;      // counts, cells and block sums of more than max_particles queries
+    DevBuf grid_index;  // the index in grid order where kb and vb are too short for it
+    int64_t index_need = 0;   // entries that did not fit
+    bool grid_ready = false;  // grid_first and the index hold the last build's
     int64_t sum_src = -1;     // grid_rows and grid_sum hold the last build's for this half width
+
+    int64_t stride() const { return (std::max<int64_t>(max_particles, 1) + 63) & ~63ll; }
+    uint32_t* index() const { return grid_index.p ? grid_index.as<uint32_t>() : kb; }
+    int64_t index_capacity() const { return grid_index.p ? (int64_t)(grid_index.bytes / sizeof(uint32_t)) : 2 * stride(); }
+    size_t layout(bool dense);  // places the buffers in mem (if it is allocated); their bytes together
 };
 
 namespace {
@@ -223,9 +235,11 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_carry(int64_t* __restrict__ bsu
     }
 }
 // OutT: int64 query offsets or uint32 cell starts
+// (TOTAL: out[n] too, and the total in 64 bits where asked for)
 template <class OutT, bool TOTAL>
 __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const uint32_t* __restrict__ in, int64_t n,
-                                                       const int64_t* __restrict__ bsum, OutT* __restrict__ out) {
+                                                       const int64_t* __restrict__ bsum, OutT* __restrict__ out,
+                                                       int64_t* __restrict__ total) {
     __shared__ int64_t sh[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + warp * (32 * SCAN_ROWS) + lane;
@@ -246,18 +260,22 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const uint32_t* __restric
     for (int k = 0; k < SCAN_ROWS; ++k) {
         const int64_t i = base + 32 * k;
         if (i < n) out[i] = (OutT)(before + x[k] - v[k]);
-        if (TOTAL && i == n - 1) out[n] = (OutT)(before + x[k]);
+        if (TOTAL && i == n - 1) {
+            out[n] = (OutT)(before + x[k]);
+            if (total) *total = before + x[k];
+        }
     }
 }
 
 // ------------------------------------------------------ dense query sets
-// When the queries are at least 1/4 of the cells (HG_DENSE_CELLS), the index is first laid out
-// again in grid order (x outer, z inner): every cell's bucket, one after the
+// When the queries are at least 1/4 of the cells and have 2^19 cells to look up
+// (HG_DENSE_CELLS, HG_DENSE_WORK), the index is first laid out again in grid order (x outer, z inner): every cell's bucket, one after the
 // other, so that the 2s+1 cells of a query's block along z are one stretch of
 // it and no query hashes anything:
 //   k_hg_grid    (start, count) of every cell, scanned into the stretches
-//   k_hg_expand  the buckets in grid order (buckets that several cells hash to
-//                are repeated: at most mult_max times the particles)
+//   k_hg_expand  the buckets in grid order (those that several cells hash to are
+//                repeated: up to 1.8 times the particles for uniform clouds in a
+//                cube of cells, none where its edge is a power of two)
 //   k_hg_rows    each cell's stretch of 2s+1 cells along z
 //   k_hg_blocks  and the particles of its whole block, once per cell instead of
 //                once per query
@@ -272,18 +290,6 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const uint32_t* __restric
 // with one query per warp and a lane per cell).
 constexpr uint32_t HG_OUTSIDE = 0xFFFFFFFFu;  // qcell: the query is outside the grid
 
-__global__ void k_hg_mult(HGDev G, uint32_t* __restrict__ mult) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= G.total) return;
-    const uint32_t z = c % G.res[2], xy = c / G.res[2], y = xy % G.res[1], x = xy / G.res[1];
-    atomicAdd(&mult[hg_mod(hg_morton(x, y, z), G)], 1u);
-}
-__global__ void k_hg_max(const uint32_t* __restrict__ v, uint32_t n, uint32_t* __restrict__ out) {
-    uint32_t m = 0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) m = max(m, v[i]);
-    m = __reduce_max_sync(0xFFFFFFFFu, m);
-    if ((threadIdx.x & 31) == 0) atomicMax(out, m);
-}
 __global__ void k_hg_grid(HGDev G, const uint32_t* __restrict__ counts, const uint32_t* __restrict__ starts,
                           uint32_t* __restrict__ ccount, uint32_t* __restrict__ cstart) {
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -293,9 +299,12 @@ __global__ void k_hg_grid(HGDev G, const uint32_t* __restrict__ counts, const ui
     ccount[c] = counts[id];
     cstart[c] = starts[id];
 }
-// first[c] .. first[c + 1]: cell c's bucket in grid order
+// first[c] .. first[c + 1]: cell c's bucket in grid order.  Nothing is written
+// when the entries exceed capacity (first may then have wrapped, too).
 __global__ void k_hg_expand(uint32_t total, const uint32_t* __restrict__ first, const uint32_t* __restrict__ cstart,
-                            const uint32_t* __restrict__ sorted_index, uint32_t* __restrict__ out) {
+                            const uint32_t* __restrict__ sorted_index, const int64_t* __restrict__ entries,
+                            int64_t capacity, uint32_t* __restrict__ out) {
+    if (*entries > capacity) return;
     // warps copy their 32 cells' buckets together: one stretch of out
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t f = c < total ? first[c] : 0u, k = c < total ? first[c + 1] - f : 0u;
@@ -345,7 +354,8 @@ __global__ void k_hg_dcount(HGDev G, const float* __restrict__ q, int64_t nq, ui
     qcount[i] = k;
     qcell[i] = in ? lin : HG_OUTSIDE;
 }
-// Nothing is written when the lists (offsets[nq] entries) exceed capacity.
+// Nothing is written when the lists (offsets[nq] entries) exceed capacity, or
+// the index in grid order was not written.
 // QW: queries a warp takes together; their lists are one stretch of out, and
 // (2 src + 1)^2 QW <= 32 stretches come from one read per lane.  QW = 1 also
 // takes wider blocks, 32 stretches at a time.
@@ -354,9 +364,10 @@ __global__ void __launch_bounds__(HG_T) k_hg_dfill(HGDev G, const float* __restr
                                                    const uint32_t* __restrict__ first, const uint2* __restrict__ rows,
                                                    const uint32_t* __restrict__ index,
                                                    const uint32_t* __restrict__ qcell,
+                                                   const int64_t* __restrict__ entries, int64_t index_capacity,
                                                    const int64_t* __restrict__ offsets, int64_t capacity,
                                                    uint32_t* __restrict__ out) {
-    if (offsets[nq] > capacity) return;
+    if (offsets[nq] > capacity || *entries > index_capacity) return;
     const uint32_t w = 2 * src + 1, nrow = w * w;
     const int lane = threadIdx.x & 31;
     const uint32_t mine = QW > 1 ? lane / nrow : 0u;  // this lane's query of the warp's, and its row of it
@@ -442,55 +453,38 @@ const float* staged(DevBuf& stage, const float* p, int64_t nfloat, int32_t kind,
     return stage.as<float>();
 }
 
-// Cells per query up to which the dense tables pay: laying them out costs 30 ps
-// per cell (2 M cells), and a hashed query of 27 cells 0.2 ns more than a dense
-// one.
-constexpr int64_t HG_DENSE_CELLS = 4;
-constexpr uint32_t HG_DENSE_MULT = 8;  // most cells per bucket (grid_index is that many times the particles)
+// Where the grid-order tables pay: laying them out costs 30 ps per cell (2 M
+// cells), and a hashed query of 27 cells 0.2 ns more than a dense one; and their
+// seven launches cost about as much as 2^19 cell lookups of the queries.  First
+// query of a build, hashed and dense: 500 queries of 27 cells 61 and 80 us, 8,000
+// 68 and 78, 20,000 76 and 76, 5,000 of 125 cells 115 and 81, 60,000 of 27 88 and
+// 82, 200,000 119 and 103, 2 M 1075 and 368 us.
+constexpr int64_t HG_DENSE_CELLS = 4;         // most cells per query
+constexpr int64_t HG_DENSE_WORK = 1ll << 19;  // least cells of all queries' blocks together
 
 // The grid-order tables of the last build for blocks of half width src (kept
-// until the next build).  1: ready; 0: too many cells share a bucket, or their
-// memory is not to be had (the hashed queries need none); < 0: an error.
+// until the next build).  1: ready, unless result[1] shows more entries than
+// the index holds; 0: the memory for it is not to be had; < 0: an error.
 int dense_tables(pgmpm_hashgrid_s* g, const HGDev& G, uint32_t src, cudaStream_t st) {
-    const size_t cells = g->total;
-    const int nb = blocks_of((int64_t)cells, HG_T);
-    const int64_t sb = ((int64_t)cells + SCAN_TILE - 1) / SCAN_TILE;
-    auto have = [](cudaError_t e) {
-        if (e != cudaSuccess) cudaGetLastError();  // clear the failed allocation
-        return e == cudaSuccess;
-    };
-    if (!have(g->grid_tables.ensure((sizeof(uint2) + 2 * sizeof(uint32_t)) * cells + sizeof(uint32_t))) ||
-        !have(g->scan_tmp.ensure(sizeof(int64_t) * sb)))
-        return 0;
-    uint32_t* sum = g->grid_sum();
-    // a cube of 2^k cells an axis has no two cells in a bucket; otherwise count
-    // once per grid, since it is a property of the resolution
-    if (g->res[0] == g->res[1] && g->res[1] == g->res[2] && (g->res[0] & (g->res[0] - 1u)) == 0u) g->mult_max = 1;
-    if (g->mult_max == 0) {
-        CK(cudaMemsetAsync(sum, 0, sizeof(uint32_t) * cells, st));
-        CK(cudaMemsetAsync(g->stats.p, 0, sizeof(uint32_t), st));
-        k_hg_mult<<<nb, HG_T, 0, st>>>(G, sum);
-        k_hg_max<<<std::min(nb, 148 * 8), HG_T, 0, st>>>(sum, g->total, g->stats.as<uint32_t>());
-        CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(&g->mult_max, g->stats.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-        CK(cudaStreamSynchronize(st));
+    if (g->index_need > g->index_capacity()) {
+        const size_t words = (size_t)g->index_need + (size_t)g->index_need / 4;
+        if (g->grid_index.alloc(sizeof(uint32_t) * words) != cudaSuccess) {
+            cudaGetLastError();  // clear the failed allocation
+            return 0;
+        }
+        g->grid_ready = false;
     }
-    // with a cell per bucket the copy is as long as the particles, and takes a
-    // buffer of the build's sort (the first query of 2 M on a new grid 1771 -> 1250 us)
-    if (g->mult_max > HG_DENSE_MULT || g->n * g->mult_max > 0xFFFFFFFFll ||
-        (g->mult_max > 1 && !have(g->grid_index.ensure(sizeof(uint32_t) * std::max<size_t>((size_t)g->n * g->mult_max, 1)))))
-        return 0;
-    uint32_t* first = g->grid_first();
+    const int nb = blocks_of((int64_t)g->total, HG_T);
     if (!g->grid_ready) {
-        uint32_t* cstart = reinterpret_cast<uint32_t*>(g->grid_rows());  // until k_hg_rows writes it
-        int64_t* bsum = g->scan_tmp.as<int64_t>();
-        k_hg_grid<<<nb, HG_T, 0, st>>>(G, g->counts.as<uint32_t>(), g->starts.as<uint32_t>(), sum, cstart);
-        CK(exclusive_scan(sum, (int64_t)cells, bsum, first, st));
-        k_hg_expand<<<nb, HG_T, 0, st>>>(g->total, first, cstart, g->va.as<uint32_t>(), g->dense_index());
+        uint32_t* cstart = reinterpret_cast<uint32_t*>(g->grid_rows);  // until k_hg_rows writes it
+        k_hg_grid<<<nb, HG_T, 0, st>>>(G, g->counts, g->starts, g->grid_sum, cstart);
+        CK(exclusive_scan(g->grid_sum, (int64_t)g->total, g->scan, g->grid_first, st, g->result + 1));
+        k_hg_expand<<<nb, HG_T, 0, st>>>(g->total, g->grid_first, cstart, g->va, g->result + 1, g->index_capacity(),
+                                         g->index());
     }
     if (!g->grid_ready || g->sum_src != (int64_t)src) {
-        k_hg_rows<<<nb, HG_T, 0, st>>>(G, src, first, g->grid_rows());
-        k_hg_blocks<<<nb, HG_T, 0, st>>>(G, src, g->grid_rows(), sum);
+        k_hg_rows<<<nb, HG_T, 0, st>>>(G, src, g->grid_first, g->grid_rows);
+        k_hg_blocks<<<nb, HG_T, 0, st>>>(G, src, g->grid_rows, g->grid_sum);
     }
     CK(cudaGetLastError());
     g->grid_ready = true;
@@ -502,14 +496,43 @@ int dense_tables(pgmpm_hashgrid_s* g, const HGDev& G, uint32_t src, cudaStream_t
 
 namespace pgmpm {
 size_t exclusive_scan_bytes(int64_t n) { return sizeof(int64_t) * (size_t)((n + SCAN_TILE - 1) / SCAN_TILE); }
-cudaError_t exclusive_scan(const uint32_t* in, int64_t n, int64_t* scratch, uint32_t* out, cudaStream_t st) {
+cudaError_t exclusive_scan(const uint32_t* in, int64_t n, int64_t* scratch, uint32_t* out, cudaStream_t st,
+                           int64_t* total) {
     const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
     k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(in, n, scratch);
     k_scan_carry<<<1, SCAN_T, 0, st>>>(scratch, nb);
-    k_scan_apply<uint32_t, true><<<(int)nb, SCAN_T, 0, st>>>(in, n, scratch, out);
+    k_scan_apply<uint32_t, true><<<(int)nb, SCAN_T, 0, st>>>(in, n, scratch, out, total);
     return cudaGetLastError();
 }
 }  // namespace pgmpm
+
+size_t pgmpm_hashgrid_s::layout(bool dense) {
+    char* base = mem.as<char>();
+    size_t at = 0;
+    auto place = [&](auto*& p, size_t count) {
+        p = base ? reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at) : nullptr;
+        at += (sizeof(*p) * count + 255) & ~(size_t)255;
+    };
+    const size_t n = (size_t)stride(), cells = total;
+    place(counts, cells);
+    place(starts, cells);
+    place(cell_ids, n);
+    place(ka, n);
+    place(va, n);
+    place(kb, 2 * n);
+    vb = kb ? kb + n : nullptr;
+    place(scratch, (size_t)radix_sort_scratch_words((int64_t)n));
+    place(stats, 3);
+    place(scan, (std::max(n, cells) + SCAN_TILE - 1) / SCAN_TILE);
+    place(result, 2);
+    if (dense) {
+        place(qcount, n);
+        place(grid_rows, cells);
+        place(grid_sum, cells);
+        place(grid_first, cells + 1);
+    }
+    return at;
+}
 
 extern "C" {
 
@@ -541,16 +564,17 @@ int pgmpm_hashgrid_create(float cell_size, const float* domain_min, const float*
     g->key_bits = std::max(1, bits_for(total));
     g->max_particles = max_particles;
     DeviceGuard dg(device);
-    const size_t n = (size_t)std::max<int64_t>(max_particles, 1);
-    cudaError_t e = g->counts.alloc(sizeof(uint32_t) * total);
-    if (e == cudaSuccess) e = g->starts.alloc(sizeof(uint32_t) * total);
-    if (e == cudaSuccess) e = g->cell_ids.alloc(sizeof(uint32_t) * n);
-    if (e == cudaSuccess) e = g->ka.alloc(sizeof(uint32_t) * n);
-    if (e == cudaSuccess) e = g->va.alloc(sizeof(uint32_t) * n);
-    if (e == cudaSuccess) e = g->kb.alloc(sizeof(uint32_t) * n);
-    if (e == cudaSuccess) e = g->vb.alloc(sizeof(uint32_t) * n);
-    if (e == cudaSuccess) e = g->scratch.alloc(sizeof(uint32_t) * radix_sort_scratch_words((int64_t)n));
-    if (e == cudaSuccess) e = g->stats.alloc(sizeof(unsigned long long) * 3);
+    // with the dense queries' tables (16 bytes per cell) where as many queries as
+    // particles would use them
+    const bool dense = (int64_t)total <= HG_DENSE_CELLS * max_particles && total < 0x80000000ull;
+    cudaError_t e = g->mem.alloc(g->layout(dense));
+    if (e == cudaSuccess) {
+        g->layout(dense);
+    } else if (dense) {
+        cudaGetLastError();
+        e = g->mem.alloc(g->layout(false));
+        if (e == cudaSuccess) g->layout(false);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         delete g;
@@ -578,8 +602,7 @@ int pgmpm_hashgrid_build(pgmpm_hashgrid g, const float* positions, int64_t n, in
     const float* pos = staged(g->pos_stage, positions, 3 * n, ptr_kind, st, rc);
     if (rc) return rc;
     const HGDev G = dev_of(g);
-    uint32_t* ids = g->cell_ids.as<uint32_t>();
-    uint32_t* counts = g->counts.as<uint32_t>();
+    uint32_t *ids = g->cell_ids, *counts = g->counts;
     const uint32_t* sorted_index = nullptr;
     // per-cell counts (histogram of the cell ids), starts = their exclusive scan
     CK(cudaMemsetAsync(counts, 0, sizeof(uint32_t) * g->total, st));
@@ -588,22 +611,20 @@ int pgmpm_hashgrid_build(pgmpm_hashgrid g, const float* positions, int64_t n, in
         CK(cudaGetLastError());
     }
     const int64_t nb = ((int64_t)g->total + SCAN_TILE - 1) / SCAN_TILE;
-    CK(g->scan_tmp.ensure(sizeof(int64_t) * nb));
-    int64_t* bsum = g->scan_tmp.as<int64_t>();
+    int64_t* bsum = g->scan;
     k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(counts, g->total, bsum);
     k_scan_carry<<<1, SCAN_T, 0, st>>>(bsum, nb);
-    k_scan_apply<uint32_t, false><<<(int)nb, SCAN_T, 0, st>>>(counts, g->total, bsum, g->starts.as<uint32_t>());
+    k_scan_apply<uint32_t, false><<<(int)nb, SCAN_T, 0, st>>>(counts, g->total, bsum, g->starts, nullptr);
     CK(cudaGetLastError());
     // particles ordered by cell, by index within a cell (stable sort)
     if (n > 0) {
         int which = 0;
-        CK(radix_sort_pairs(ids, nullptr, g->ka.as<uint32_t>(), g->va.as<uint32_t>(), g->kb.as<uint32_t>(),
-                            g->vb.as<uint32_t>(), g->scratch.as<uint32_t>(), n, g->key_bits, &which, st));
-        sorted_index = which ? g->vb.as<uint32_t>() : g->va.as<uint32_t>();
+        CK(radix_sort_pairs(ids, nullptr, g->ka, g->va, g->kb, g->vb, g->scratch, n, g->key_bits, &which, st));
+        sorted_index = which ? g->vb : g->va;
     }
     // keep the sorted indices where queries read them
-    if (n > 0 && sorted_index != g->va.as<uint32_t>())
-        CK(cudaMemcpyAsync(g->va.p, sorted_index, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
+    if (n > 0 && sorted_index != g->va)
+        CK(cudaMemcpyAsync(g->va, sorted_index, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, st));
     g->n = n;
     g->built = true;
     g->grid_ready = false;
@@ -618,10 +639,10 @@ int pgmpm_hashgrid_get_table(pgmpm_hashgrid g, uint32_t* counts, uint32_t* start
     DeviceGuard dg(g->device);
     cudaStream_t st = ST(stream);
     const cudaMemcpyKind k = ptr_kind == PGMPM_PTR_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    if (counts) CK(cudaMemcpyAsync(counts, g->counts.p, sizeof(uint32_t) * g->total, k, st));
-    if (starts) CK(cudaMemcpyAsync(starts, g->starts.p, sizeof(uint32_t) * g->total, k, st));
-    if (particle_indices && g->n) CK(cudaMemcpyAsync(particle_indices, g->va.p, sizeof(uint32_t) * g->n, k, st));
-    if (cell_ids && g->n) CK(cudaMemcpyAsync(cell_ids, g->cell_ids.p, sizeof(uint32_t) * g->n, k, st));
+    if (counts) CK(cudaMemcpyAsync(counts, g->counts, sizeof(uint32_t) * g->total, k, st));
+    if (starts) CK(cudaMemcpyAsync(starts, g->starts, sizeof(uint32_t) * g->total, k, st));
+    if (particle_indices && g->n) CK(cudaMemcpyAsync(particle_indices, g->va, sizeof(uint32_t) * g->n, k, st));
+    if (cell_ids && g->n) CK(cudaMemcpyAsync(cell_ids, g->cell_ids, sizeof(uint32_t) * g->n, k, st));
     if (ptr_kind == PGMPM_PTR_HOST) CK(cudaStreamSynchronize(st));
     return PGMPM_OK;
 }
@@ -643,64 +664,76 @@ int pgmpm_hashgrid_neighbors(pgmpm_hashgrid g, const float* queries, int64_t nq,
     const float* q = staged(g->qstage, queries, 3 * nq, ptr_kind, st, rc);
     if (rc) return rc;
     const HGDev G = dev_of(g);
-    // counts, then the queries' cells, unless those fit a buffer of the build's sort
-    const bool reuse = nq <= g->max_particles;
-    CK(g->qcount.ensure((reuse ? 1 : 2) * sizeof(uint32_t) * std::max<int64_t>(nq, 1)));
     const int64_t nb = std::max<int64_t>(1, (nq + SCAN_TILE - 1) / SCAN_TILE);
     const size_t off_bytes = sizeof(int64_t) * (size_t)(nq + 1);
-    uint32_t *qcount = g->qcount.as<uint32_t>(), *qcell = reuse ? g->ka.as<uint32_t>() : qcount + nq;
+    int64_t* bsum = g->scan;
+    uint32_t *qcount = g->qcount, *qcell = g->ka;
+    if (nq > g->max_particles || !qcount) {
+        CK(g->qlarge.ensure(sizeof(int64_t) * nb + 2 * sizeof(uint32_t) * std::max<int64_t>(nq, 1)));
+        bsum = g->qlarge.as<int64_t>();
+        qcount = reinterpret_cast<uint32_t*>(bsum + nb);
+        qcell = qcount + nq;
+    }
+    if (ptr_kind == PGMPM_PTR_HOST) CK(g->off_stage.ensure(off_bytes));
+    int64_t* doff = ptr_kind == PGMPM_PTR_HOST ? g->off_stage.as<int64_t>() : offsets;
     bool dense = false;
-    if (nq > 0 && (int64_t)g->total <= HG_DENSE_CELLS * nq && g->total < 0x80000000u) {
+    const int64_t block = (int64_t)(2 * src + 1) * (2 * src + 1) * (2 * src + 1);
+    if (g->grid_rows && (int64_t)g->total <= HG_DENSE_CELLS * nq && nq >= (HG_DENSE_WORK + block - 1) / block) {
         rc = dense_tables(g, G, src, st);
         if (rc < 0) return rc;
         dense = rc == 1;
     }
-    // scan_tmp: block sums, then the offsets when the caller's are on the host
-    CK(g->scan_tmp.ensure(sizeof(int64_t) * nb + (ptr_kind == PGMPM_PTR_HOST ? off_bytes : 0)));
-    int64_t* bsum = g->scan_tmp.as<int64_t>();
-    int64_t* doff = ptr_kind == PGMPM_PTR_HOST ? bsum + nb : offsets;
-    const uint32_t* first = dense ? g->grid_first() : nullptr;
-    if (nq > 0) {
-        if (dense)
-            k_hg_dcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, first, g->grid_sum(), qcount,
-                                                              qcell);
-        else
-            k_hg_qcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts.as<uint32_t>(), qcount);
-        k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum);
-        k_scan_carry<<<1, SCAN_T, 0, st>>>(bsum, nb);
-        k_scan_apply<int64_t, true><<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum, doff);
-        CK(cudaGetLastError());
-    } else {
-        CK(cudaMemsetAsync(doff, 0, sizeof(int64_t), st));
-    }
     auto fill = [&](uint32_t* dout, int64_t cap) {
         auto dfill = [&](auto kernel, int qw) {
             kernel<<<(int)std::min<int64_t>(blocks_of(nq, qw * (HG_T / 32)), 148 * 64), HG_T, 0, st>>>(
-                G, q, nq, src, first, g->grid_rows(), g->dense_index(), qcell,
-                doff, cap, dout);
+                G, q, nq, src, g->grid_first, g->grid_rows, g->index(), qcell, g->result + 1, g->index_capacity(), doff,
+                cap, dout);
         };
         if (dense && src <= 1)  // 1 or 9 stretches per query
             src == 0 ? dfill(k_hg_dfill<32>, 32) : dfill(k_hg_dfill<3>, 3);
         else if (dense)
             dfill(k_hg_dfill<1>, 1);
         else
-            k_hg_qfill<<<blocks_of(nq * HG_FG, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts.as<uint32_t>(),
-                                                                     g->starts.as<uint32_t>(), g->va.as<uint32_t>(),
-                                                                     doff, dout);
+            k_hg_qfill<<<blocks_of(nq * HG_FG, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts, g->starts, g->va, doff,
+                                                                     dout);
     };
-    // into a device buffer the dense fill follows at once (it checks the
-    // capacity itself); otherwise the host learns the total first
-    const bool early = dense && indices && capacity > 0 && ptr_kind == PGMPM_PTR_DEVICE;
-    if (early) {
-        fill(indices, capacity);
-        CK(cudaGetLastError());
-    }
     int64_t tot = 0;
-    CK(cudaMemcpyAsync(&tot, doff + nq, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
+    bool filled = false;
+    for (;; dense = false) {
+        if (nq > 0) {
+            if (dense)
+                k_hg_dcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->grid_first, g->grid_sum, qcount,
+                                                                  qcell);
+            else
+                k_hg_qcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts, qcount);
+            k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum);
+            k_scan_carry<<<1, SCAN_T, 0, st>>>(bsum, nb);
+            k_scan_apply<int64_t, true><<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum, doff, g->result);
+            CK(cudaGetLastError());
+        } else {
+            CK(cudaMemsetAsync(doff, 0, sizeof(int64_t), st));
+            CK(cudaMemsetAsync(g->result, 0, sizeof(int64_t), st));
+        }
+        // into a device buffer the dense fill follows at once (it checks the
+        // capacities itself); otherwise the host learns the total first
+        filled = dense && indices && capacity > 0 && ptr_kind == PGMPM_PTR_DEVICE;
+        if (filled) {
+            fill(indices, capacity);
+            CK(cudaGetLastError());
+        }
+        int64_t r[2] = {0, 0};
+        CK(cudaMemcpyAsync(r, g->result, sizeof(int64_t) * (dense ? 2 : 1), cudaMemcpyDeviceToHost, st));
+        CK(cudaStreamSynchronize(st));
+        tot = r[0];
+        if (!dense || r[1] <= g->index_capacity()) break;
+        // particles crowd in buckets that several cells share: hashed queries
+        // now, a longer index for the next ones
+        g->index_need = r[1];
+        g->grid_ready = false;
+    }
     *total = tot;
     if (ptr_kind == PGMPM_PTR_HOST) CK(cudaMemcpyAsync(offsets, doff, off_bytes, cudaMemcpyDeviceToHost, st));
-    if (!early && indices && tot <= capacity && tot > 0) {
+    if (!filled && indices && tot <= capacity && tot > 0) {
         uint32_t* dout = indices;
         if (ptr_kind == PGMPM_PTR_HOST) {
             CK(g->qout_stage.ensure(sizeof(uint32_t) * tot));
@@ -722,11 +755,10 @@ int pgmpm_hashgrid_stats(pgmpm_hashgrid g, pgmpm_hashgrid_info* out) {
     DeviceGuard dg(g->device);
     unsigned long long h[3] = {0, 0, 0};  // before a build: no particles
     if (g->built) {
-        CK(cudaMemset(g->stats.p, 0, sizeof(h)));
-        k_hg_stats<<<std::min(blocks_of(g->total, HG_T), 148 * 8), HG_T>>>(g->counts.as<uint32_t>(), g->total,
-                                                                          g->stats.as<unsigned long long>());
+        CK(cudaMemset(g->stats, 0, sizeof(h)));
+        k_hg_stats<<<std::min(blocks_of(g->total, HG_T), 148 * 8), HG_T>>>(g->counts, g->total, g->stats);
         CK(cudaGetLastError());
-        CK(cudaMemcpy(h, g->stats.p, sizeof(h), cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(h, g->stats, sizeof(h), cudaMemcpyDeviceToHost));
     }
     std::memset(out, 0, sizeof(*out));
     out->occupied_cells = (uint32_t)h[0];

@@ -77,10 +77,11 @@ __device__ __forceinline__ uint2 hg_row(const HGDev& G, const uint32_t c[3], uin
     return make_uint2(f, __ldg(&first[row + (uint32_t)z1 + 1u]) - f);
 }
 
-// Exclusive scan of n counts into out[0..n] (out[n] = total); scratch of
-// exclusive_scan_bytes(n).
+// Exclusive scan of n counts into out[0..n] (out[n] = total, which may wrap;
+// *total in 64 bits where asked for); scratch of exclusive_scan_bytes(n).
 size_t exclusive_scan_bytes(int64_t n);
-cudaError_t exclusive_scan(const uint32_t* in, int64_t n, int64_t* scratch, uint32_t* out, cudaStream_t st);
+cudaError_t exclusive_scan(const uint32_t* in, int64_t n, int64_t* scratch, uint32_t* out, cudaStream_t st,
+                           int64_t* total = nullptr);
 
 // Walks the entries of up to 32 segments (start s0 and length k of this lane's
 // segment, k = 0 for none) as one list, the warp's lanes taking consecutive

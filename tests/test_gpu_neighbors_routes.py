@@ -107,3 +107,77 @@ def test_more_cells_than_32_bits_are_refused(gpu):
     sim.upload(np.full((1, 3), 0.5, np.float32), None, None, None, one, one)
     with pytest.raises(gpu.PGMPMError, match="more than"):
         sim.sph_coupling(np.full((1, 3), 0.5, np.float32), np.zeros((1, 3), np.float32), radius=2.0 ** -22)
+
+
+@pytest.mark.parametrize("res", [(16, 16, 1), (32, 32, 2), (64, 8, 8), (20, 20, 20)])
+@pytest.mark.parametrize("device", [False, True])
+def test_grid_order_index_longer_than_the_sort_buffers(gpu, res, device):
+    """Buckets that several cells share are repeated in the grid-order index;
+    with more than two entries a particle (or all particles in such a bucket)
+    the first query set finds the buffers too short and takes the hashed route,
+    the next ones a longer index, also after other builds.  Lists against small
+    query sets, which are hashed."""
+    import torch
+    from physgrad_b200 import _capi as C
+    rng = np.random.default_rng(sum(res))
+    cell = 0.125
+    ext = np.array(res) * cell
+    n = max(6 * int(np.prod(res)) + 5, 20011)  # 2^19 cells to look up: not hashed for want of work
+    clouds = [rng.uniform(0, ext, (n, 3)), rng.uniform(0, ext, (n, 3))]
+    clouds[1][:] = clouds[1][0]  # one cell
+    clouds[1][: n // 3] = rng.uniform(0, ext, (n // 3, 3))
+    L, st, tot = gpu.lib(), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream), ctypes.c_int64()
+    g = gpu.SpatialHashGrid(cell, (0.0, 0.0, 0.0), tuple(float(e) for e in ext), max_particles=n)
+    for build in (0, 1, 0):
+        pts = clouds[build].astype(np.float32)
+        # (the crowded cell's lists are long: fewer queries ask for it)
+        qs = np.concatenate([pts[: n // 3], rng.uniform(0, ext, (n - n // 3, 3)).astype(np.float32)])
+        g.buildHashTable(pts)
+        want = [g.neighbors(qs[k:k + 20], 0.1) for k in range(0, n, n // 9)]
+        for _ in range(3):
+            if device:
+                q = torch.tensor(qs, device="cuda")
+                off = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+                for cap in (0, None):  # the length, then the lists
+                    idx = torch.full((tot.value if cap is None else 1,), -7, dtype=torch.int32, device="cuda")
+                    C.check(L.pgmpm_hashgrid_neighbors(g._h, q.data_ptr(), n, 0.1, off.data_ptr(), idx.data_ptr(),
+                                                       idx.numel() if cap is None else 0, ctypes.byref(tot),
+                                                       C.PTR_DEVICE, st))
+                off, idx = off.cpu().numpy(), idx.cpu().numpy().view(np.uint32)
+            else:
+                off, idx = g.neighbors(qs, 0.1)
+            assert off[-1] == len(idx)
+            for (o, i), k in zip(want, range(0, n, n // 9)):
+                assert np.array_equal(o, off[k:k + len(o)] - off[k])
+                assert np.array_equal(i, idx[off[k]:off[k] + len(i)])
+
+
+@pytest.mark.parametrize("res,src,clustered", [((16, 16, 16), 1, False), ((13, 9, 21), 1, True), ((13, 9, 21), 2, True),
+                                               ((7, 30, 5), 0, False), ((3, 2, 1), 3, False), ((1, 1, 1), 1, False),
+                                               ((61, 2, 2), 1, False), ((700, 1, 2), 1, False), ((9, 9, 9), 5, False)])
+@pytest.mark.parametrize("more_queries_than_particles", [False, True])
+def test_many_queries_on_small_grids_equal_hashed_queries(gpu, res, src, clustered, more_queries_than_particles):
+    """Enough queries for the grid-order tables on grids of few cells and odd
+    shapes, inside the grid and outside, in the sort's buffers and in their
+    own: offsets and lists against small query sets, which are hashed."""
+    rng = np.random.default_rng(sum(res) + 7 * src)
+    cell = 0.125
+    ext = np.array(res) * cell
+    nq = -(-(1 << 19) // (2 * src + 1) ** 3) + 3
+    n = min(nq, 2 * int(np.prod(res)) + 9)
+    cap = n if more_queries_than_particles else nq
+    pts = rng.uniform(-0.3, ext + 0.3, (n, 3))
+    if clustered:
+        pts[: n // 2] = ext * 0.4 + rng.normal(0, cell, (n // 2, 3))
+    qs = rng.uniform(-0.3, ext + 0.3, (nq, 3)).astype(np.float32)
+    g = gpu.SpatialHashGrid(cell, (0.0, 0.0, 0.0), tuple(float(e) for e in ext), max_particles=cap)
+    assert g.resolution == tuple(res)
+    g.buildHashTable(pts.astype(np.float32))
+    radius = (src - 0.5) * cell if src else 0.0
+    off, idx = g.neighbors(qs, radius)
+    assert off[0] == 0 and np.all(np.diff(off) >= 0) and off[-1] == len(idx)
+    part = min(nq // 8, 300)
+    for k in (0, nq // 3, nq - part):
+        o, i = g.neighbors(qs[k:k + part], radius)
+        assert np.array_equal(o, off[k:k + part + 1] - off[k])
+        assert np.array_equal(i, idx[off[k]:off[k + part]])
