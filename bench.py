@@ -60,6 +60,22 @@ def make_workload(name):
     return W.config2()
 
 
+# kernel of each variant (MLS, bin sort), as the captures name it
+P2G_KERNELS = {0: "k_p2g_tiles", 1: "k_p2g", 2: "k_p2g_cells", 3: "k_p2g_pairs", 4: "k_p2g_slices"}
+G2P_KERNELS = {0: "k_g2p_tiles", 1: "k_g2p", 2: "k_g2p_phys"}
+
+
+def captured_counters(workload, running):
+    """The DRAM bytes and FLOPs per launch that profiles/traffic.json holds for
+    a workload: those of the kernels that run (running: stage -> kernel)."""
+    path = os.path.join(ROOT, "profiles", "traffic.json")
+    if not os.path.exists(path):
+        return {}
+    with open(path) as f:
+        prof = json.load(f).get(workload, {})
+    return {k: v for k, v in prof.items() if v.get("kernel") and v["kernel"] == running.get(k)}
+
+
 def algorithmic_bytes(N, A, multi_mat):
     """Algorithmic HBM bytes per launch (FP32), in the unfused accounting the
     measurement contract states: P2G reads x, m, v, C, F (100 B per particle,
@@ -328,11 +344,9 @@ def run_ours(args, rank, world, device):
     comp = compulsory_bytes(N, A, multi)
     fb = fused_bytes(N, A, multi)
     hbm, peak_kind = peaks()
-    prof = {}
-    tpath = os.path.join(ROOT, "profiles", "traffic.json")
-    if os.path.exists(tpath):
-        with open(tpath) as f:
-            prof = json.load(f).get(args.workload, {})
+    met = sim.metrics()
+    prof = captured_counters(args.workload, {"p2g": P2G_KERNELS.get(met["p2g_variant"]),
+                                             "g2p": G2P_KERNELS.get(met["g2p_variant"])})
     kernels = {}
     for k in (("g2p2g", "grid") if fused else ("p2g", "g2p", "grid")):
         ms_k = kern_ms["g2p"] if k == "g2p2g" else kern_ms[k]

@@ -37,3 +37,28 @@ def test_targets_keys_of_the_bench_line(monkeypatch):
     assert cube["replays"] == {"sort_record": True, "replayed_steps_sorted_again": 0}
     assert set(line["targets"]) >= {"sparse_grid_two_material_drop", "differentiable_elastic_cube",
                                     "batched_forward_64_scenes", "batched_forward_adjoint_32_scenes"}
+
+
+def test_captured_counters_are_those_of_the_kernels_that_run():
+    """Every entry of profiles/traffic.json names a kernel of the sources, and
+    the bench takes only entries of the kernels it runs."""
+    import json
+    import re
+
+    sys.path.insert(0, ROOT)
+    import bench
+
+    csrc = os.path.join(ROOT, "physgrad_b200", "csrc")
+    text = "".join(open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc)) if f.endswith(".cu"))
+    kernels = set(re.findall(r"__global__\s+void\s+(?:__launch_bounds__\([^)]*\)\s*)?(\w+)\(", text))
+    with open(os.path.join(ROOT, "profiles", "traffic.json")) as f:
+        prof = json.load(f)
+    entries = [(w, k, e) for w, d in prof.items() if not w.startswith("_") for k, e in d.items()]
+    assert entries
+    for w, k, e in entries:
+        assert e["kernel"] in kernels, (w, k)
+        assert bench.captured_counters(w, {k: e["kernel"]}) == {k: e}
+        assert bench.captured_counters(w, {k: "another kernel"}) == {}
+    assert set(bench.P2G_KERNELS.values()) | set(bench.G2P_KERNELS.values()) <= kernels
+    assert prof["cfg2"]["p2g"]["kernel"] == bench.P2G_KERNELS[4]  # the defaults
+    assert prof["cfg2"]["g2p"]["kernel"] == bench.G2P_KERNELS[2]
