@@ -228,8 +228,9 @@ int record_tape_reverse(pgmpm_solver s, const AdjView& A0, int len, cudaStream_t
         V.early_first = j < len - 1;  // after the previous slot's gather
         A.q_next = b.q_out;
         A.pay_ready = A.q_prev != nullptr;  // by the previous slot's gather
-        A.q_prev = j > 0 && adj_scatter_from_payload(V, s->tune) ? tape_bufs(s, j - 1, t, g0 < 0 ? -1 : g0 + j - 1).q
-                                                                 : nullptr;
+        A.q_prev = j > 0 && adj_scatter_from_payload(V, A, s->tune)
+                       ? tape_bufs(s, j - 1, t, g0 < 0 ? -1 : g0 + j - 1).q
+                       : nullptr;
         // the slot's P2G work cursor is zero: the grid update of the slot's
         // forward step cleared it after P2G (and a previous reverse's grid
         // adjoint after its scatter)
@@ -499,7 +500,11 @@ int pgmpm_backward(pgmpm_solver s, const float* gx_out, const float* gv_out, con
     rc = unprime(s, st);
     if (rc) return rc;
     CK(s->adj_g.ensure(sizeof(float4) * 6 * Nz));
-    CK(s->adj_pay.ensure(sizeof(float4) * 4 * Nz));
+    // the scatter's payload; without memory for it each scatter reads the state
+    // and the adjoint itself
+    if (s->tune.p2g_variant >= 4 && s->tune.step_sort == 0 &&
+        s->adj_pay.ensure(sizeof(float4) * 4 * Nz) != cudaSuccess)
+        cudaGetLastError();
     CK(s->adj_grid_gv.ensure(sizeof(float4) * nodes_of(s)));
     CK(s->adj_grid_gpm.ensure(sizeof(float4) * nodes_of(s)));
     CK(s->adj_gE.ensure(sizeof(float) * M));

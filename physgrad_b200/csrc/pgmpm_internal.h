@@ -322,8 +322,11 @@ struct AdjView {
     float4* grid_gpm;          // (dL/dp_i, dL/dm_i) per node
     float* gE;                 // [M] dL/dE accumulators
 };
-// launch_adj_scatter runs from A.pay (P2G variants 4 and 5 with the bin sort)
-inline bool adj_scatter_from_payload(const View& V, const Tuning& t) { return t.p2g_variant >= 4 && V.cell_range; }
+// launch_adj_scatter runs from A.pay (P2G variants 4 and 5 with the bin sort,
+// where there was memory for it)
+inline bool adj_scatter_from_payload(const View& V, const AdjView& A, const Tuning& t) {
+    return t.p2g_variant >= 4 && V.cell_range && A.pay;
+}
 cudaError_t launch_adj_scatter(const View& V, const AdjView& A, const PhysFlags& pf, const Tuning& t, int num_sms,
                                cudaStream_t st);
 cudaError_t launch_adj_grid(const View& V, const AdjView& A, const Tuning& t, int num_sms, cudaStream_t st);

@@ -2060,7 +2060,7 @@ cudaError_t launch_adj_scatter(const View& V, const AdjView& A, const PhysFlags&
                                cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
     if (pf.physics != PHYS_MLS) return cudaErrorNotSupported;
-    if (adj_scatter_from_payload(V, t)) {  // three threads per cell over the sort's cell table
+    if (adj_scatter_from_payload(V, A, t)) {  // three threads per cell over the sort's cell table
         auto payload = pf.multi_mat ? (pf.has_fluid ? k_adj_payload<true, true> : k_adj_payload<true, false>)
                                     : (pf.has_fluid ? k_adj_payload<false, true> : k_adj_payload<false, false>);
         bool early = V.early_first;
