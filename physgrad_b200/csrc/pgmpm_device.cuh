@@ -23,8 +23,9 @@ namespace pgmpm {
 
 // First statement of the kernels that launch_after may launch early: waits until
 // the kernel before on the stream has completed and its writes are visible.
-// Nothing is read before it, and these kernels read what others of the step
-// write by plain loads, not through the read-only path.
+// Nothing is read before it.  What that kernel wrote is read by plain loads;
+// older data, complete when an early kernel starts, may come through the
+// read-only path (k_adj_gather's node velocities).
 __device__ __forceinline__ void step_wait() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }

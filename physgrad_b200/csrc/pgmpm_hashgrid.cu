@@ -91,11 +91,6 @@ __global__ void k_hg_cells(HGDev G, const float* __restrict__ pos, int64_t n, ui
     atomicAdd(&counts[id], 1u);
 }
 
-// Fill pass, HG_FG lanes per query: they take the block's cells in the
-// reference's order (linear index t = (dx (2s+1) + dy) (2s+1) + dz), HG_FG at
-// a time, give each cell its place by a scan over the lanes and copy the
-// cell's particles, so a query's list is written into one contiguous stretch
-// by its lanes together.
 // Count pass, one thread per query: the block's cells in nested loops (the
 // reference's order does not matter for a sum)
 __global__ void k_hg_qcount(HGDev G, const float* __restrict__ q, int64_t nq, uint32_t src,
@@ -122,6 +117,11 @@ __global__ void k_hg_qcount(HGDev G, const float* __restrict__ q, int64_t nq, ui
     qcount[i] = k;
 }
 
+// Fill pass, HG_FG lanes per query: they take the block's cells in the
+// reference's order (linear index t = (dx (2s+1) + dy) (2s+1) + dz), HG_FG at
+// a time, give each cell its place by a scan over the lanes and copy the
+// cell's particles, so a query's list is written into one contiguous stretch
+// by its lanes together.
 constexpr int HG_FG = 8;  // lanes per query in the fill (4 queries per warp; 4 lanes and 32 were slower)
 __global__ void k_hg_qfill(HGDev G, const float* __restrict__ q, int64_t nq, uint32_t src,
                            const uint32_t* __restrict__ counts, const uint32_t* __restrict__ starts,

@@ -171,14 +171,15 @@ __device__ __forceinline__ uint32_t run_slot(const KeyRun& r) {
 // another; an early launch (programmatic stream serialization) sets the grid
 // up while the kernel before it on the stream drains, and its threads wait in
 // step_wait() for that kernel's end.  Early only right after a kernel (not
-// after a copy, a memset, an event or a conditional node), and only kernels that
-// begin with step_wait(): since each waits for the one before (or is launched the
-// plain way), order holds along the whole chain.  32,768 particles 1374 -> 1306 us for 50 steps; at 2 M the
-// same time.  The kernels do not signal their successors before their end:
-// blocks that wait on the SM keep the running kernel's out (262,144 particles
-// with gradients 6733 -> 7024 us).  G2P is launched the plain way: its node
-// reads want the read-only path (plain loads: 96 -> 108 us at 2 M), and the early
-// launch gave it nothing on top.
+// after a copy, a memset, an event, a graph or a conditional node), and only
+// kernels that begin with step_wait(): since each waits for the one before (or is
+// launched the plain way), order holds along the whole chain.  32,768 particles
+// 1374 -> 1306 us for 50 steps; at 2 M the same time.  The kernels do not signal
+// their successors before their end: blocks that wait on the SM keep the running
+// kernel's out (262,144 particles with gradients 6733 -> 7024 us).  G2P is
+// launched the plain way: its node reads want the read-only path (plain loads:
+// 96 -> 108 us at 2 M), and the early launch gave it nothing on top.  The status
+// is the launch's own, not an error that something else left in the thread.
 template <class... P, class... A>
 inline cudaError_t launch_after(bool early, void (*kernel)(P...), int grid, int block, cudaStream_t st, A... a) {
     cudaLaunchConfig_t c = {};

@@ -233,7 +233,11 @@ __global__ void __launch_bounds__(P2GS_T, ADJ ? 3 : 4) k_ref_p2g(View V, RefStep
     const int q = t / 3, k = t - 3 * (t / 3);
     const SceneDev& sc = V.scenes[0];
     const uint32_t ntiles = V.counters[CNT_CTILES];
-    // slices of a cell's particles when tiles are few (as k_p2g_slices)
+    // slices of a cell's particles when tiles are few.  Rounded up, at most 4,
+    // where k_p2g_slices rounds down, to 8: items go to the blocks in turn here,
+    // without claims (median of forward and reverse, that rule after this one:
+    // 200,000 particles on 40^3 nodes 29.1 and 30.1 us, 10,000 on 32^3 11.0 and
+    // 8.3, 2,000 to 400,000 on 24^3 to 96^3 otherwise the same)
     const uint32_t S = ntiles ? min(4u, max(1u, (gridDim.x + ntiles - 1) / ntiles)) : 1u;
     // this thread's cell of a work item: particles b, b + S, .. < e; the next
     // item's are loaded while this one is summed

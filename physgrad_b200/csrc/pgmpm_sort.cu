@@ -228,8 +228,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs_scatter(const uint32_t* kin, co
 //   bs_scatter   particle -> cell begin + slot; the occupied tiles' places in
 //                the largest-first list P2G takes work from (the last tiles a
 //                persistent P2G block picks up are then small ones, which
-//                shortens the kernel's tail); clears the tile and group
-//                counters and publishes the step's counter words.
+//                shortens the kernel's tail); clears the tile counters and
+//                publishes the step's counter words.
 // The counters are left zero for the next step by their readers, so a step
 // costs O(N + occupied cells + tiles) with no clearing pass.  Keys come out
 // sorted; particles that share a cell in atomic-arrival order, which the
