@@ -296,3 +296,27 @@ def test_steps_before_and_after_their_graphs_are_made(gpu, calls, sparse, outer)
     ulps = sum(calls) * 2.0 ** -23
     assert np.abs(outs[0]["x"] - outs[1]["x"]).max() <= 1.4 * ulps + 1e-6
     assert np.abs(outs[0]["v"] - outs[1]["v"]).max() <= (4 * ulps + 1e-6) * np.abs(outs[1]["v"]).max()
+
+
+@pytest.mark.parametrize("N", [1, 31, 33, 257, 1000])
+def test_downloads_of_every_subset(gpu, N):
+    """Each choice of x, v, C and F comes back bit for bit, and the words around
+    the arrays stay: x and v alone are stored from their planes, records with C
+    or F through shared memory."""
+    import itertools
+
+    import torch
+    rng = np.random.default_rng(N)
+    dx = 1.0 / 32
+    st = _scene_state(rng, N, (20, 24, 28), dx)
+    sim = gpu.Simulator([gpu.Scene((20, 24, 28), dx, 1e-4)], [N], [gpu.createElasticMaterial(1000.0, 1e4, 0.3)])
+    sim.upload(st["x"], st["v"], st["C"], st["F"], st["m"], st["V0"])
+    widths = {"x": 3, "v": 3, "C": 9, "F": 9}
+    for r in range(1, 5):
+        for names in itertools.combinations(widths, r):
+            bufs = {k: torch.full((N * widths[k] + 3,), 7.0, device="cuda") for k in names}
+            sim.download({k: b[1:1 + N * widths[k]] for k, b in bufs.items()})
+            torch.cuda.synchronize()
+            for k, b in bufs.items():
+                assert b[0] == 7.0 and torch.all(b[-2:] == 7.0)
+                assert np.array_equal(b[1:1 + N * widths[k]].cpu().numpy().reshape(N, -1), st[k].reshape(N, -1)), (names, k)
