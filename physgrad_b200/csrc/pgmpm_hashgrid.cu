@@ -173,12 +173,20 @@ __global__ void k_hg_qfill(HGDev G, const float* __restrict__ q, int64_t nq, uin
 
 // Exclusive scan of n uint32 counts into out[0..n] (out[n] = total, where
 // asked for): per-block sums, one block scanning the sums, then each block's
-// scan plus its carry.  A warp takes SCAN_ROWS rows of 32 counts, so that every
-// access is a full line (2 M counts: sums 10 -> 3.9 us, apply 11.4 -> 7.7 us
-// against one count per thread).
+// scan plus its carry.  A warp takes ROWS rows of 32 counts, every access a full
+// line: 4 rows for many counts (2 M: sums 10 -> 3.9 us, apply 11.4 -> 7.7 us
+// against one count per thread), one where latency counts (apply of 1 to 20,000
+// counts 2.0-2.2 us, 2.9-3.2 with four).
 constexpr int SCAN_T = 1024;
-constexpr int SCAN_ROWS = 4;
-constexpr int SCAN_TILE = SCAN_T * SCAN_ROWS;  // counts per block
+constexpr int64_t SCAN_FEW = (int64_t)1 << 18;  // most counts for one row
+constexpr int scan_rows(int64_t n) { return n <= SCAN_FEW ? 1 : 4; }
+constexpr int64_t scan_blocks(int64_t n) {
+    return (n + SCAN_T * scan_rows(n) - 1) / (SCAN_T * scan_rows(n));
+}
+// block sums of any scan of up to n counts
+constexpr int64_t scan_words(int64_t n) {
+    return n <= SCAN_FEW ? scan_blocks(n) : scan_blocks(n) > scan_blocks(SCAN_FEW) ? scan_blocks(n) : scan_blocks(SCAN_FEW);
+}
 __device__ __forceinline__ int64_t warp_incl_scan(int64_t x, int lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -198,14 +206,15 @@ __device__ __forceinline__ int64_t block_incl_scan(int64_t x, int64_t* sh) {
     __syncthreads();
     return r;
 }
+template <int ROWS>
 __global__ void __launch_bounds__(SCAN_T) k_scan_sums(const uint32_t* __restrict__ in, int64_t n,
                                                       int64_t* __restrict__ bsum) {
     __shared__ int64_t sh[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int64_t s = 0;
 #pragma unroll
-    for (int k = 0; k < SCAN_ROWS; ++k) {
-        const int64_t i = (int64_t)blockIdx.x * SCAN_TILE + k * SCAN_T + threadIdx.x;
+    for (int k = 0; k < ROWS; ++k) {
+        const int64_t i = (int64_t)blockIdx.x * (SCAN_T * ROWS) + k * SCAN_T + threadIdx.x;
         s += i < n ? in[i] : 0u;
     }
 #pragma unroll
@@ -236,18 +245,18 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_carry(int64_t* __restrict__ bsu
 }
 // OutT: int64 query offsets or uint32 cell starts
 // (TOTAL: out[n] too, and the total in 64 bits where asked for)
-template <class OutT, bool TOTAL>
+template <int ROWS, class OutT, bool TOTAL>
 __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const uint32_t* __restrict__ in, int64_t n,
                                                        const int64_t* __restrict__ bsum, OutT* __restrict__ out,
                                                        int64_t* __restrict__ total) {
     __shared__ int64_t sh[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + warp * (32 * SCAN_ROWS) + lane;
-    int64_t v[SCAN_ROWS], x[SCAN_ROWS], run = 0;
+    const int64_t base = (int64_t)blockIdx.x * (SCAN_T * ROWS) + warp * (32 * ROWS) + lane;
+    int64_t v[ROWS], x[ROWS], run = 0;
 #pragma unroll
-    for (int k = 0; k < SCAN_ROWS; ++k) v[k] = base + 32 * k < n ? in[base + 32 * k] : 0u;
+    for (int k = 0; k < ROWS; ++k) v[k] = base + 32 * k < n ? in[base + 32 * k] : 0u;
 #pragma unroll
-    for (int k = 0; k < SCAN_ROWS; ++k) {  // inclusive over the warp's rows so far
+    for (int k = 0; k < ROWS; ++k) {  // inclusive over the warp's rows so far
         x[k] = run + warp_incl_scan(v[k], lane);
         run = __shfl_sync(0xFFFFFFFFu, x[k], 31);
     }
@@ -257,7 +266,7 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const uint32_t* __restric
     __syncthreads();
     const int64_t before = bsum[blockIdx.x] + (warp ? sh[warp - 1] : 0);
 #pragma unroll
-    for (int k = 0; k < SCAN_ROWS; ++k) {
+    for (int k = 0; k < ROWS; ++k) {
         const int64_t i = base + 32 * k;
         if (i < n) out[i] = (OutT)(before + x[k] - v[k]);
         if (TOTAL && i == n - 1) {
@@ -265,6 +274,23 @@ __global__ void __launch_bounds__(SCAN_T) k_scan_apply(const uint32_t* __restric
             if (total) *total = before + x[k];
         }
     }
+}
+
+// (out[n] and *total where TOTAL; n > 0, bsum of scan_words(n))
+template <class OutT, bool TOTAL>
+cudaError_t scan_counts(const uint32_t* in, int64_t n, int64_t* bsum, OutT* out, int64_t* total, cudaStream_t st) {
+    const int nb = (int)scan_blocks(n);
+    const bool few = scan_rows(n) == 1;
+    if (few)
+        k_scan_sums<1><<<nb, SCAN_T, 0, st>>>(in, n, bsum);
+    else
+        k_scan_sums<4><<<nb, SCAN_T, 0, st>>>(in, n, bsum);
+    k_scan_carry<<<1, SCAN_T, 0, st>>>(bsum, nb);
+    if (few)
+        k_scan_apply<1, OutT, TOTAL><<<nb, SCAN_T, 0, st>>>(in, n, bsum, out, total);
+    else
+        k_scan_apply<4, OutT, TOTAL><<<nb, SCAN_T, 0, st>>>(in, n, bsum, out, total);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------ dense query sets
@@ -495,14 +521,10 @@ int dense_tables(pgmpm_hashgrid_s* g, const HGDev& G, uint32_t src, cudaStream_t
 }  // namespace
 
 namespace pgmpm {
-size_t exclusive_scan_bytes(int64_t n) { return sizeof(int64_t) * (size_t)((n + SCAN_TILE - 1) / SCAN_TILE); }
+size_t exclusive_scan_bytes(int64_t n) { return sizeof(int64_t) * (size_t)scan_words(n); }
 cudaError_t exclusive_scan(const uint32_t* in, int64_t n, int64_t* scratch, uint32_t* out, cudaStream_t st,
                            int64_t* total) {
-    const int64_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-    k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(in, n, scratch);
-    k_scan_carry<<<1, SCAN_T, 0, st>>>(scratch, nb);
-    k_scan_apply<uint32_t, true><<<(int)nb, SCAN_T, 0, st>>>(in, n, scratch, out, total);
-    return cudaGetLastError();
+    return scan_counts<uint32_t, true>(in, n, scratch, out, total, st);
 }
 }  // namespace pgmpm
 
@@ -523,7 +545,7 @@ size_t pgmpm_hashgrid_s::layout(bool dense) {
     vb = kb ? kb + n : nullptr;
     place(scratch, (size_t)radix_sort_scratch_words((int64_t)n));
     place(stats, 3);
-    place(scan, (std::max(n, cells) + SCAN_TILE - 1) / SCAN_TILE);
+    place(scan, (size_t)scan_words((int64_t)std::max(n, cells)));
     place(result, 2);
     if (dense) {
         place(qcount, n);
@@ -610,12 +632,7 @@ int pgmpm_hashgrid_build(pgmpm_hashgrid g, const float* positions, int64_t n, in
         k_hg_cells<<<blocks_of(n, HG_T), HG_T, 0, st>>>(G, pos, n, ids, counts);
         CK(cudaGetLastError());
     }
-    const int64_t nb = ((int64_t)g->total + SCAN_TILE - 1) / SCAN_TILE;
-    int64_t* bsum = g->scan;
-    k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(counts, g->total, bsum);
-    k_scan_carry<<<1, SCAN_T, 0, st>>>(bsum, nb);
-    k_scan_apply<uint32_t, false><<<(int)nb, SCAN_T, 0, st>>>(counts, g->total, bsum, g->starts, nullptr);
-    CK(cudaGetLastError());
+    CK((scan_counts<uint32_t, false>(counts, g->total, g->scan, g->starts, nullptr, st)));
     // particles ordered by cell, by index within a cell (stable sort)
     if (n > 0) {
         int which = 0;
@@ -664,7 +681,7 @@ int pgmpm_hashgrid_neighbors(pgmpm_hashgrid g, const float* queries, int64_t nq,
     const float* q = staged(g->qstage, queries, 3 * nq, ptr_kind, st, rc);
     if (rc) return rc;
     const HGDev G = dev_of(g);
-    const int64_t nb = std::max<int64_t>(1, (nq + SCAN_TILE - 1) / SCAN_TILE);
+    const int64_t nb = scan_words(std::max<int64_t>(nq, 1));
     const size_t off_bytes = sizeof(int64_t) * (size_t)(nq + 1);
     int64_t* bsum = g->scan;
     uint32_t *qcount = g->qcount, *qcell = g->ka;
@@ -706,10 +723,7 @@ int pgmpm_hashgrid_neighbors(pgmpm_hashgrid g, const float* queries, int64_t nq,
                                                                   qcell);
             else
                 k_hg_qcount<<<blocks_of(nq, HG_T), HG_T, 0, st>>>(G, q, nq, src, g->counts, qcount);
-            k_scan_sums<<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum);
-            k_scan_carry<<<1, SCAN_T, 0, st>>>(bsum, nb);
-            k_scan_apply<int64_t, true><<<(int)nb, SCAN_T, 0, st>>>(qcount, nq, bsum, doff, g->result);
-            CK(cudaGetLastError());
+            CK((scan_counts<int64_t, true>(qcount, nq, bsum, doff, g->result, st)));
         } else {
             CK(cudaMemsetAsync(doff, 0, sizeof(int64_t), st));
             CK(cudaMemsetAsync(g->result, 0, sizeof(int64_t), st));

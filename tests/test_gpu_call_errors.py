@@ -34,11 +34,17 @@ int cudaLaunchKernelExC(const void* cfg, const void* f, void** args) {
     if (launch_left > 0 && --launch_left == 0) return 701; /* cudaErrorLaunchOutOfResources */
     return next(cfg, f, args);
 }
+static int alloc_left = 0;
+void fail_allocs(int k) { alloc_left = k; }      /* the next k allocations fail */
 static size_t no_alloc = 0;
 void fail_alloc(size_t bytes) { no_alloc = bytes; }  /* allocations of this size fail; 0: none */
 int cudaMalloc(void** p, size_t bytes) {
     static int (*next)(void**, size_t) = NULL;
     if (!next) next = (int (*)(void**, size_t))real("cudaMalloc");
+    if (alloc_left > 0) {
+        --alloc_left;
+        return 2; /* cudaErrorMemoryAllocation */
+    }
     return no_alloc && bytes == no_alloc ? 2 : next(p, bytes);
 }
 int cudaGraphInstantiate(void** exec, void* graph, unsigned long long flags) {
@@ -189,6 +195,43 @@ for size in (64 * N, 0):  # without memory for the scatter's payload, then with 
 print("CHILD OK")
 """
 
+HASH = COMMON + r"""
+rng = np.random.default_rng(4)
+pts = rng.uniform(0, 1, (20011, 3)).astype(np.float32)
+grid = lambda: pg.SpatialHashGrid(0.07, (0.0, 0.0, 0.0), (1.0, 1.0, 1.0), max_particles=len(pts))
+a = grid()
+shim.fail_allocs(1)
+b = grid()  # without the tables of the dense queries
+shim.fail_allocs(2)
+assert raises(grid)
+shim.fail_allocs(0)
+a.buildHashTable(pts)
+b.buildHashTable(pts)
+for _ in range(2):
+    (oa, ia), (ob, ib) = a.neighbors(pts, 0.07), b.neighbors(pts, 0.07)
+    assert np.array_equal(oa, ob) and np.array_equal(ia, ib)
+# a bucket of its own for nearly all particles: more entries than the sort's
+# buffers hold, and no memory for a longer index
+c = grid()
+pts[: len(pts) - 100] = pts[0]
+c.buildHashTable(pts)
+b.buildHashTable(pts)
+qs = rng.uniform(0, 1, (20011, 3)).astype(np.float32)
+want = b.neighbors(qs, 0.07)
+for k in (0, 1, 0):
+    shim.fail_allocs(k)
+    L, tot = pg.lib(), ctypes.c_int64()
+    got = c.neighbors(qs, 0.07) if not k else None
+    if k:  # into arrays that are there (host staging is)
+        off, idx = np.zeros(len(qs) + 1, np.int64), np.zeros(len(want[1]), np.uint32)
+        assert L.pgmpm_hashgrid_neighbors(c._h, qs.ctypes.data, len(qs), 0.07, off.ctypes.data, idx.ctypes.data, len(idx),
+                                          ctypes.byref(tot), C.PTR_HOST, None) == 0
+        got = off, idx
+    shim.fail_allocs(0)
+    assert np.array_equal(want[0], got[0]) and np.array_equal(want[1], got[1])
+print("CHILD OK")
+"""
+
 
 @pytest.fixture(scope="module")
 def shim(tmp_path_factory):
@@ -230,6 +273,13 @@ def test_backward_without_memory_for_the_scatter_payload(gpu, shim):
     (sums of FP32 terms in another order, the bound of the other reverse
     scatters' comparison on a whole rollout)."""
     _child(shim, "SPARSE = False\n" + BACKWARD)
+
+
+def test_hash_grid_without_memory_for_the_dense_queries(gpu, shim):
+    """A grid whose tables cannot be had answers by the hashed queries, as one
+    whose index in grid order cannot grow; without memory for the rest its
+    creation fails.  Lists are whole numbers and equal."""
+    _child(shim, "SPARSE = False\n" + HASH)
 
 
 def test_steps_with_an_error_pending_in_the_thread(gpu):

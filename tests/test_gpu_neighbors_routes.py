@@ -181,3 +181,23 @@ def test_many_queries_on_small_grids_equal_hashed_queries(gpu, res, src, cluster
         o, i = g.neighbors(qs[k:k + part], radius)
         assert np.array_equal(o, off[k:k + part + 1] - off[k])
         assert np.array_equal(i, idx[off[k]:off[k + part]])
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 4097, (1 << 18) - 1, 1 << 18, (1 << 18) + 1, (1 << 18) + 4097])
+def test_counts_scanned_at_the_edges_of_blocks_and_rows(gpu, n):
+    """The exclusive scan takes one or four rows a warp by the number of counts:
+    offsets of n queries and the starts of n cells against numpy's sums."""
+    rng = np.random.default_rng(n)
+    pts = rng.uniform(0, 1, (500, 3))
+    pts[:, 0] *= n  # n cells in a row
+    g = gpu.SpatialHashGrid(1.0, (0.0, 0.0, 0.0), (float(n), 1.0, 1.0), max_particles=700)
+    assert g.total_cells == n
+    g.buildHashTable(pts.astype(np.float32))
+    counts, starts = g.getCellParticleCounts().astype(np.int64), g.getCellStartIndices()
+    assert counts.sum() == 500 and np.array_equal(starts, np.concatenate([[0], np.cumsum(counts)[:-1]]))
+    qs = rng.uniform(0, 1, (n, 3)) * [n, 1, 1]
+    off, idx = g.neighbors(qs.astype(np.float32), 0.0)
+    assert off[0] == 0 and off[-1] == len(idx) and np.all(np.diff(off) >= 0)
+    for k in np.unique(np.concatenate([[0, n - 1], rng.integers(0, n, 40)])):
+        o, i = g.neighbors(qs[k:k + 1].astype(np.float32), 0.0)
+        assert o[1] == off[k + 1] - off[k] and np.array_equal(i, idx[off[k]:off[k + 1]])
