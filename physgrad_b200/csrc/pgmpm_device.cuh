@@ -186,25 +186,28 @@ __device__ __forceinline__ void planes_to_records(const float4* __restrict__ q, 
         const uint32_t ok = __ballot_sync(0xFFFFFFFFu, i < N);  // records with a particle
         __syncwarp();
         if (i < N) {
-            const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+            // all loads first: between them, the stores below would wait
+            float4 p0, p1, p2, p3, p4, p5;
+            p0 = p1 = p2 = p3 = p4 = p5 = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (x || F) p0 = q[i];
+            if (F) p1 = q[N + i], p2 = q[2 * N + i];
+            if (v || C) p3 = q[3 * N + i];
+            if (C) p4 = q[4 * N + i], p5 = q[5 * N + i];
             float xx[3], FF[9], vv[3], CC[9];
-            if (x || F) {
-                unpack_xF(q[i], F ? q[N + i] : none, F ? q[2 * N + i] : none, xx, FF);
+            unpack_xF(p0, p1, p2, xx, FF);
+            unpack_vC(p3, p4, p5, vv, CC);
 #pragma unroll
-                for (int a = 0; a < 3; ++a) sx[3 * lane + a] = xx[a];
-                if (F) {
-#pragma unroll
-                    for (int a = 0; a < 9; ++a) sF[9 * lane + a] = FF[a];
-                }
+            for (int a = 0; a < 3; ++a) {
+                sx[3 * lane + a] = xx[a];
+                sv[3 * lane + a] = vv[a];
             }
-            if (v || C) {
-                unpack_vC(q[3 * N + i], C ? q[4 * N + i] : none, C ? q[5 * N + i] : none, vv, CC);
+            if (F) {
 #pragma unroll
-                for (int a = 0; a < 3; ++a) sv[3 * lane + a] = vv[a];
-                if (C) {
+                for (int a = 0; a < 9; ++a) sF[9 * lane + a] = FF[a];
+            }
+            if (C) {
 #pragma unroll
-                    for (int a = 0; a < 9; ++a) sC[9 * lane + a] = CC[a];
-                }
+                for (int a = 0; a < 9; ++a) sC[9 * lane + a] = CC[a];
             }
         }
         __syncwarp();

@@ -330,11 +330,12 @@ __global__ void k_hg_grid(HGDev G, const uint32_t* __restrict__ counts, const ui
 __global__ void k_hg_expand(uint32_t total, const uint32_t* __restrict__ first, const uint32_t* __restrict__ cstart,
                             const uint32_t* __restrict__ sorted_index, const int64_t* __restrict__ entries,
                             int64_t capacity, uint32_t* __restrict__ out) {
-    if (*entries > capacity) return;
+    const int64_t have = *entries;  // (read along with first)
     // warps copy their 32 cells' buckets together: one stretch of out
     const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t f = c < total ? first[c] : 0u, k = c < total ? first[c + 1] - f : 0u;
     const int lane = threadIdx.x & 31;
+    if (have > capacity) return;
     uint32_t* dst = out + __shfl_sync(0xFFFFFFFFu, f, 0);
     hg_walk(c < total ? cstart[c] : 0u, k, lane, [&](bool valid, uint32_t e, uint32_t pos) {
         if (valid) dst[e] = __ldg(&sorted_index[pos]);
@@ -393,7 +394,8 @@ __global__ void __launch_bounds__(HG_T) k_hg_dfill(HGDev G, const float* __restr
                                                    const int64_t* __restrict__ entries, int64_t index_capacity,
                                                    const int64_t* __restrict__ offsets, int64_t capacity,
                                                    uint32_t* __restrict__ out) {
-    if (offsets[nq] > capacity || *entries > index_capacity) return;
+    const int64_t length = offsets[nq], have = *entries;
+    if (length > capacity || have > index_capacity) return;
     const uint32_t w = 2 * src + 1, nrow = w * w;
     const int lane = threadIdx.x & 31;
     const uint32_t mine = QW > 1 ? lane / nrow : 0u;  // this lane's query of the warp's, and its row of it
