@@ -323,7 +323,11 @@ void make_graphs(pgmpm_solver s, int n_steps, bool spans, const bool direct[STEP
     if (spans && n_steps > 1 && n_steps <= s->kCallSteps) {
         if (n_steps != s->call_last) s->call_seen = 0;
         s->call_last = n_steps;
-        if (now(s->call_seen, s->kSeenCall)) {
+        if (now(s->call_seen, s->call_need)) {
+            // one that replaces another which was hardly used: lengths change too
+            // often, the next one waits for twice as many calls
+            if (s->call_steps && s->call_used < 2 * s->call_need) s->call_need = std::min(2 * s->call_need, 1 << 20);
+            s->call_used = 0;
             s->call_steps = 0;
             rc = build_span(s, n_steps, true, s->call_exec);
             if (!rc) s->call_steps = n_steps;
@@ -365,6 +369,7 @@ int live_steps(pgmpm_solver s, int n_steps, cudaStream_t st) {
     if (spans && n_steps > 1 && n_steps <= s->kCallSteps && s->call_steps == n_steps) {
         CK(cudaGraphLaunch(s->call_exec, st));
         s->call_last = n_steps;
+        if (s->call_used < 1 << 30) ++s->call_used;
         s->met.total_steps += n_steps;
         return PGMPM_OK;
     }

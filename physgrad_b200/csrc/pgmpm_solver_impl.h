@@ -157,11 +157,13 @@ struct pgmpm_solver_s {
     // several split steps in one graph (run_steps): all steps of a call, and
     // kMidSteps steps with others of their call before and after them
     static constexpr int kCallSteps = 64, kMidSteps = 16, kMidAtLeast = 130;
+    static constexpr int kSeenCall = 5, kSeenStep = 8;  // calls after which a graph is made
     cudaGraphExec_t call_exec = nullptr, mid_exec = nullptr;
     int call_steps = 0;               // steps of call_exec
     int call_last = 0, call_seen = 0; // steps of the last call, and calls in a row that had as many
+    int call_used = 0;                // launches of call_exec
+    int call_need = kSeenCall;        // calls in a row before a call's graph is made
     int mid_seen = 0;                 // calls that could have used mid_exec
-    static constexpr int kSeenCall = 5, kSeenStep = 8;  // calls after which a graph is made
     bool graphs_failed = false;       // one could not be made: no further attempts until drop_graph
     cudaEvent_t ev[6] = {};
 
@@ -298,7 +300,8 @@ struct pgmpm_solver_s {
         if (call_exec) cudaGraphExecDestroy(call_exec);
         if (mid_exec) cudaGraphExecDestroy(mid_exec);
         call_exec = mid_exec = nullptr;
-        call_steps = call_last = call_seen = mid_seen = 0;
+        call_steps = call_last = call_seen = call_used = mid_seen = 0;
+        call_need = kSeenCall;
         graphs_failed = false;
         drop_tape_graphs();
     }

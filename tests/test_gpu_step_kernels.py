@@ -258,6 +258,7 @@ def test_pic_step_routes_agree(gpu, n_near):
 
 
 @pytest.mark.parametrize("calls", [[1] * 11, [2] * 11, [5, 5, 3] + [5] * 8 + [3] * 7 + [5, 7] * 9, [64] * 7,
+                                   ([4] * 6 + [3] * 6) * 3 + [4] * 25,
                                    [131, 146, 17, 140, 130, 17, 135, 40, 17, 133]])
 @pytest.mark.parametrize("sparse", [False, True])
 @pytest.mark.parametrize("outer", [False, True])
