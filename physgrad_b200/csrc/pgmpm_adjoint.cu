@@ -341,11 +341,12 @@ __global__ void k_state_to_planes(const float* __restrict__ x, const float* __re
     }
 }
 
+template <bool ALL>
 __global__ void __launch_bounds__(PACK_T) k_planes_to_state(const float4* __restrict__ g,
                                                             const uint32_t* __restrict__ phys_of_user,
                                                             float* __restrict__ x, float* __restrict__ v,
                                                             float* __restrict__ C, float* __restrict__ F, int64_t N) {
-    planes_to_records(g, N, phys_of_user, x, v, C, F);
+    planes_to_records<ALL>(g, N, phys_of_user, x, v, C, F);
 }
 
 inline int blocks_for(int64_t n, int block) {
@@ -384,7 +385,8 @@ cudaError_t launch_state_to_planes(const float* x, const float* v, const float* 
 cudaError_t launch_planes_to_state(const float4* g, const uint32_t* phys_of_user, float* x, float* v, float* C,
                                    float* F, int64_t N, cudaStream_t st) {
     if (N == 0) return cudaSuccess;
-    k_planes_to_state<<<blocks_for(N, PACK_T), PACK_T, 0, st>>>(g, phys_of_user, x, v, C, F, N);
+    auto kernel = x && v && C && F ? k_planes_to_state<true> : k_planes_to_state<false>;
+    kernel<<<blocks_for(N, PACK_T), PACK_T, 0, st>>>(g, phys_of_user, x, v, C, F, N);
     return cudaGetLastError();
 }
 

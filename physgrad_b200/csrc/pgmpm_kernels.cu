@@ -1973,11 +1973,12 @@ __global__ void __launch_bounds__(PACK_T, 3) k_pack(View V, const float* __restr
 
 // Walks the upload order: the caller's records are written contiguously and
 // the state planes are gathered (scattered partial-sector writes cost more).
+template <bool ALL>
 __global__ void __launch_bounds__(PACK_T) k_unpack(const float4* __restrict__ q, int64_t N,
                                                    const uint32_t* __restrict__ phys_of_user, float* __restrict__ x,
                                                    float* __restrict__ v, float* __restrict__ C,
                                                    float* __restrict__ F) {
-    planes_to_records(q, N, phys_of_user, x, v, C, F);
+    planes_to_records<ALL>(q, N, phys_of_user, x, v, C, F);
 }
 
 __global__ void k_grid_download(View V, SceneDev sc, float* __restrict__ mass, float* __restrict__ vel) {
@@ -2300,7 +2301,8 @@ cudaError_t launch_pack(const View& V, const float* x, const float* v, const flo
 cudaError_t launch_unpack(const View& V, const uint32_t* phys_of_user, float* x, float* v, float* C, float* F,
                           cudaStream_t st) {
     if (V.N == 0) return cudaSuccess;
-    k_unpack<<<grid_for(V.N, PACK_T), PACK_T, 0, st>>>(V.q, V.N, phys_of_user, x, v, C, F);
+    auto kernel = x && v && C && F ? k_unpack<true> : k_unpack<false>;
+    kernel<<<grid_for(V.N, PACK_T), PACK_T, 0, st>>>(V.q, V.N, phys_of_user, x, v, C, F);
     return cudaGetLastError();
 }
 
